@@ -250,6 +250,15 @@ static SsaArgs base_args(const Packed &p) {
     return a;
 }
 
+// Networks of 17 to 32 reactions (and at most 16 species) have a generated
+// kernel but no descriptor-driven speculative one: TableOps keeps every
+// running sum in registers and walks its factor lists, and spills beyond 16.
+// Their other kernel is the lockstep exact one.
+static bool spec_jit_only(const SsaArgs &a, const Packed &p, int grid, const DeviceCtx &ctx) {
+    return p.R > 16 && jit_supported(p) && p.max_order < 32768 &&
+           ssa_spec_slots(a, grid, ctx.smem_optin, 128) > 0;
+}
+
 Feasible feasible_kernels(const Packed &p, const DeviceCtx &ctx, int64_t n_traj, int64_t n_samples, bool times_ok,
                           double t_last, bool rates_per_traj) {
     SsaArgs a = base_args(p);
@@ -262,7 +271,8 @@ Feasible feasible_kernels(const Packed &p, const DeviceCtx &ctx, int64_t n_traj,
         1, std::min<int64_t>(ctx.sm_count, (n_traj + ssa_spec_block() - 1) / ssa_spec_block()));
     f.spec = !p.has_expr && times_ok && t_last < 0x1p60 && ssa_spec_supported(a, p.max_order) &&
              ssa_spec_slots(a, spec_grid, ctx.smem_optin, ssa_spec_block()) > 0;
-    f.jit = f.spec && jit_supported(p);
+    f.jit = (f.spec || (!p.has_expr && times_ok && t_last < 0x1p60 && spec_jit_only(a, p, spec_grid, ctx))) &&
+            jit_supported(p);
     f.warp = !p.has_expr && ssa_warp_supported(a, p.max_order) && ssa_warp_warps(a, ctx.smem_optin) > 0;
     f.fast = !p.has_expr && times_ok && ssa_fast_supported(a, p.max_order) && ssa_fast_smem(a, 128) <= ctx.smem_optin;
     f.generic = p.R <= 32 && ssa_thread_max_block(a, ctx.smem_optin) > 0;
@@ -339,8 +349,16 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
                       (want_warp || (!spec && !(p.R <= 32 && ssa_thread_max_block(a, ctx->smem_optin) > 0)));
     const bool fast = !warp && !spec && !p.has_expr && !want_generic && r.times_ok && ssa_fast_supported(a, p.max_order) &&
                       ssa_fast_smem(a, 128) <= ctx->smem_optin;
+    // Networks of 17 to 32 reactions run a generated kernel too (the lockstep
+    // exact kernel until it is compiled): 20 000 trajectories of 12 species
+    // and 24 reactions (2.4e7 events) take 21.1 ms in the lockstep kernel and
+    // 2.1 ms generated, of 16 species and 32 reactions 42.9 and 3.1 ms.
+    const bool jit_only = !spec && !warp && !want_generic && !want_fast && !want_desc &&
+                          !(pref && std::strcmp(pref, "spec") == 0) && r.times_ok && r.t_last < 0x1p60 &&
+                          !p.has_expr && spec_jit_only(a, p, spec_grid, *ctx);
     const bool strict = pref || force;  // a kernel asked for must run
-    if (strict && ((want_fast && !fast) || (want_warp && !warp) || ((want_desc || want_jit) && !spec))) {
+    if (strict && ((want_fast && !fast) || (want_warp && !warp) || (want_desc && !spec) ||
+                   (want_jit && !spec && !jit_only))) {
         set_error(std::string("kernel ") + (pref ? pref : std::to_string(k).c_str()) +
                   " does not cover this network or sample grid");
         return false;
@@ -350,7 +368,7 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
     // trajectory's step latency is close to a lone lane's (RB_SPEC_LANES=k
     // sets k lanes per warp; 32 turns the spreading off).
     int lanes = 0;
-    if (spec) {
+    if (spec || jit_only) {
         const int64_t sched = (int64_t)ctx->sm_count * 4;
         if (const char *e = std::getenv("RB_SPEC_LANES")) lanes = std::max(1, std::min(32, std::atoi(e)));
         else if (r.n_traj < sched * 32) lanes = (int)((r.n_traj + sched - 1) / sched);
@@ -400,15 +418,17 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
         if (mapping) *mapping = 5;
         return true;
     }
-    if (spec) {
+    if (spec || jit_only) {
         a.row_done = r.n_samples < 65536 ? r.row_done : nullptr;
-        block = lanes ? 128 : ssa_spec_block();
-        a.n_slots = lanes ? 128 : spec_slots;
-        a.lanes = lanes;
         a.phase_steps = shape.phase;
         a.sched = shape.sched > 0 ? 1 : 0;
         if (const char *ph = std::getenv("RB_SPEC_PHASE")) a.phase_steps = std::atoi(ph);
         if (const char *sc = std::getenv("RB_SPEC_SCHED")) a.sched = std::strcmp(sc, "rot") == 0 ? 1 : 0;
+    }
+    if (spec) {
+        block = lanes ? 128 : ssa_spec_block();
+        a.n_slots = lanes ? 128 : spec_slots;
+        a.lanes = lanes;
         smem = ssa_spec_smem(a, a.n_slots);
         per_sm = ssa_spec_occupancy(a, block, smem);
     } else if (fast) {
@@ -426,7 +446,7 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
         per_sm = ssa_thread_occupancy(a, block, smem);
     }
     if (per_sm < 1) per_sm = 1;
-    int64_t want = lanes ? (r.n_traj + 4 * lanes - 1) / (4 * lanes) : (r.n_traj + block - 1) / block;
+    int64_t want = spec && lanes ? (r.n_traj + 4 * lanes - 1) / (4 * lanes) : (r.n_traj + block - 1) / block;
     int64_t cap = (int64_t)ctx->sm_count * per_sm;
     int grid = (int)std::max<int64_t>(1, std::min(want, cap));
     // A network the generator covers runs on its own compiled kernel (RB_JIT=0
@@ -436,22 +456,32 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
     // already loaded or in the disk cache.
     const void *jk = nullptr;
     const int64_t run_no = ++dn.runs;
-    if (spec && jit_supported(p)) {
+    if ((spec && jit_supported(p)) || jit_only) {
         const char *jit = std::getenv("RB_JIT");
         // RB_SSA_KERNEL=spec (or a shape of kernel 3) asks for the
         // packed-descriptor kernel itself
         const bool off = (jit && std::strcmp(jit, "0") == 0) || want_desc;
-        const bool compile = jit ? !off : (want_jit || r.n_traj >= 4096 || run_no >= 2);
+        // (a 17- to 32-reaction network compiles for longer: only a large
+        // ensemble run a second time waits for it)
+        const bool compile = jit ? !off : (want_jit || (jit_only ? r.n_traj >= 4096 && run_no >= 2
+                                                                 : r.n_traj >= 4096 || run_no >= 2));
         if (!off) {
             // generated kernels may run larger blocks (fewer registers per lane)
-            int kb = shape.block > 0 && !std::getenv("RB_JIT_BLOCK") ? shape.block : jit_block();
+            int kb = shape.block > 0 && !std::getenv("RB_JIT_BLOCK") ? shape.block : jit_block_for(p);
             // spread launches run 128 lanes of a kernel built for 128 (all
             // registers to the few lanes that hold trajectories)
             const bool spread = lanes != 0;
             if (spread) kb = 128;
+            auto blocks_of = [&](int lanes_per_block) {
+                return (int)std::max<int64_t>(
+                    1, std::min<int64_t>(ctx->sm_count, (r.n_traj + lanes_per_block - 1) / lanes_per_block));
+            };
+            // many reactions with rate constants of their own per trajectory:
+            // blocks as large as shared memory holds slots for
+            if (jit_only && !spread)
+                while (kb > 128 && ssa_spec_slots(a, blocks_of(kb), ctx->smem_optin, kb) == 0) kb -= 64;
             const int jb = kb;
-            const int jgrid = spread ? grid
-                                     : (int)std::max<int64_t>(1, std::min<int64_t>(ctx->sm_count, (r.n_traj + jb - 1) / jb));
+            const int jgrid = !spread ? blocks_of(jb) : spec ? grid : blocks_of(4 * lanes);
             const int jslots = spread ? 128 : ssa_spec_slots(a, jgrid, ctx->smem_optin, jb);
             if (jslots > 0) {
                 if (dn.jit_k && dn.jit_block == kb && dn.jit_version == dn.version) {

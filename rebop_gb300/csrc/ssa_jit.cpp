@@ -366,7 +366,9 @@ void jit_compile_async(const Packed &p, int block) {
 }
 
 const void *jit_kernel(const Packed &p, int block, bool compile) {
-    std::lock_guard<std::mutex> lk(g_mu);
+    std::unique_lock<std::mutex> lk(g_mu, std::defer_lock);
+    if (compile) lk.lock();
+    else if (!lk.try_lock()) return nullptr;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) {
         cudaGetLastError();
@@ -394,6 +396,11 @@ const void *jit_kernel(const Packed &p, int block, bool compile) {
 int jit_block() {
     if (const char *e = std::getenv("RB_JIT_BLOCK")) return std::max(32, std::min(1024, std::atoi(e) / 32 * 32));
     return 384;
+}
+
+int jit_block_for(const Packed &p) {
+    if (std::getenv("RB_JIT_BLOCK")) return jit_block();
+    return p.R > 16 ? 256 : jit_block();
 }
 
 int launch_ssa_jit(const void *kern, const SsaArgs &a, int block, int grid, size_t smem, cudaStream_t st) {

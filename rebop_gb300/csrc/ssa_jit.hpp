@@ -21,7 +21,8 @@ std::string jit_net_source(const Packed &p, int block);
 bool jit_compile(const Packed &p, int block, size_t *image_bytes);
 // The compiled kernel for the current device (compiled on first use); null
 // with the error set on failure.  With `compile` false only a kernel already
-// loaded or in the disk cache is returned (null, no error, otherwise).  A
+// loaded or in the disk cache is returned (null, no error, otherwise; it does
+// not wait for a compilation that another thread has running).  A
 // kernel built for `block` lanes also runs blocks of fewer lanes.
 const void *jit_kernel(const Packed &p, int block, bool compile = true);
 // Compile the network's kernel into the disk cache on a background thread
@@ -32,5 +33,11 @@ int launch_ssa_jit(const void *kern, const SsaArgs &a, int block, int grid, size
 // warps per SM at up to 168 registers a lane; fastest measured on the dimer and
 // Vilar networks), or RB_JIT_BLOCK rounded to a multiple of 32.
 int jit_block();
+// The same for a network: beyond 16 reactions 256 lanes, whose 255 registers a
+// lane hold most of the running sums; 320 and 384 lanes get 168 and spill
+// (100 000 trajectories of 12 species and 24 reactions: 192 / 256 / 320 / 384
+// lanes 7.4 / 7.0 / 11.4 / 10.8 ms; 16 species and 32 reactions 3.0 / 3.1 /
+// 5.2 / 6.5 ms for 20 000).
+int jit_block_for(const Packed &p);
 
 }  // namespace rbg

@@ -1,0 +1,56 @@
+"""GPU parity of kernel variants at the edges of the ranges their dispatch gives them."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def rb():
+    import rebop_gb300
+
+    return rebop_gb300
+
+
+def _seeds(n, salt):
+    return np.random.default_rng(4321 + salt).integers(np.iinfo(np.uint64).max, size=n, dtype=np.uint64)
+
+
+def _random(rb, O, seed, S, R, macro=False):
+    import bench
+
+    reactions, x0 = bench.random_network(seed, S, R, x0_mean=60.0)
+    onet = O.OracleNet(S, macro=macro)
+    if macro:
+        lines = [f"r{k}: {' + '.join(f'{c} x{i}' for i, c in enumerate(e) if c)} => "
+                 f"{' + '.join(f'{a + b} x{i}' for i, (a, b) in enumerate(zip(e, d)) if a + b)} @ {k_!r}"
+                 for k, (k_, e, d) in enumerate(reactions)]
+        net = rb.Network.from_dsl("Net { " + ", ".join(f"x{i}" for i in range(S)) + " }\n" + "\n".join(lines))
+    else:
+        net = rb.Network(S)
+    for k, e, d in reactions:
+        if macro:
+            onet.add_macro(k, [(i, x) for i, x in enumerate(e) if x], d)
+        else:
+            net.add_reaction(rb.Rate.lma(k, e), d)
+            onet.add_lma(k, e, d)
+    return net, onet, x0
+
+
+@pytest.mark.parametrize("S,R,seed,n,sweep", [(3, 17, 81, 700, False), (12, 24, 82, 5000, False),
+                                              (16, 32, 83, 300, True), (16, 32, 84, 20_000, False)])
+def test_generated_kernel_of_17_to_32_reactions(rb, O, monkeypatch, S, R, seed, n, sweep):
+    monkeypatch.setenv("RB_JIT", "1")
+    net, onet, x0 = _random(rb, O, seed, S, R)
+    seeds = _seeds(n, seed)
+    rates = None
+    if sweep:  # per-trajectory rates, some outside the float-pair range
+        k = np.array([net.reaction_rate(r) for r in range(R)])
+        rates = k * 10.0 ** np.random.default_rng(seed).uniform(-1, 1, (n, R))
+        rates[::40, 5] = 1e-30
+    res = net.run_ensemble(x0, seeds, 2e-2, 9, rates=rates)
+    ref, ev, _, _ = onet.run_ensemble(x0, seeds, 2e-2, 9, rates=rates)
+    assert res.stats["mapping"] == 4 and ev.max() > 20
+    np.testing.assert_array_equal(res.counts, ref)
+    np.testing.assert_array_equal(res.events, ev)
