@@ -273,6 +273,10 @@ bool Batch::build(cudaStream_t st) {
         it.o_rdf = take(8 * RP);
         it.o_lfac = take(4 * RP * p.P);
         it.o_shape = take(4 * RP);
+        it.dep_bytes = 0;
+        std::vector<unsigned char> dep;
+        if (warp_dep_masks(p, dep, it.dep_bytes)) it.o_dep = take(dep.size());
+        else it.dep_bytes = 0;
     }
     // thread-unit items
     int32_t maxTS = 1;
@@ -387,6 +391,14 @@ bool Batch::build(cudaStream_t st) {
             x.lm_rdf = reinterpret_cast<const float2 *>(d + it.o_rdf);
             x.lm_fac = reinterpret_cast<const int32_t *>(d + it.o_lfac);
             x.lm_shape = (mm <= 2 && p.S < 32767) ? reinterpret_cast<const uint32_t *>(d + it.o_shape) : nullptr;
+            if (it.dep_bytes) {
+                std::vector<unsigned char> dep;
+                int bytes = 0;
+                warp_dep_masks(p, dep, bytes);
+                std::memcpy(h + it.o_dep, dep.data(), dep.size());
+                x.dep_tab = d + it.o_dep;
+                x.dep_bytes = bytes;
+            }
             // lane-major factor and shape tables
             const int C = (p.R + 31) / 32, RP = 32 * C;
             int32_t *lf = reinterpret_cast<int32_t *>(h + it.o_lfac);

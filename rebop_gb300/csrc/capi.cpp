@@ -716,19 +716,36 @@ int rbg_internal_jit_source(const rb_network *net, char *buf, size_t len) {
     return copy_name(rbg::jit_net_source(p, rbg::jit_block()), buf, len);
 }
 
-// The warp kernel's dependency table for the network ([R][32] entries into
-// out, which holds cap entries); RB_ERR_UNSUPPORTED beyond its reach.
+// The warp kernel's dependency masks for the network, listed: row j of out
+// ([R][32], cap entries in all) holds the number of reactions reaction j's
+// jump touches, then their lane-major positions; 0xFFFF for more than 31.
+// RB_ERR_UNSUPPORTED beyond the masks' reach.
 int rbg_internal_warp_dep_table(const rb_network *net, uint16_t *out, size_t cap) {
     if (!net || !out) return fail(RB_ERR_INVALID, "null argument");
-    std::vector<uint16_t> tab;
+    std::vector<unsigned char> tab;
+    int bytes = 0;
+    size_t R;
     bool ok;
     {
         std::lock_guard<std::mutex> lk(net->net.mu);
-        ok = rbg::warp_dep_table(net->net.pack(), tab);
+        const rbg::Packed p = net->net.pack();
+        R = (size_t)p.R;
+        ok = rbg::warp_dep_masks(p, tab, bytes);
     }
-    if (!ok) return fail(RB_ERR_UNSUPPORTED, "network beyond the dependency table's reach");
-    if (tab.size() > cap) return fail(RB_ERR_INVALID, "buffer too small");
-    std::memcpy(out, tab.data(), 2 * tab.size());
+    if (!ok) return fail(RB_ERR_UNSUPPORTED, "network beyond the dependency masks' reach");
+    if (R * 32 > cap) return fail(RB_ERR_INVALID, "buffer too small");
+    const size_t C = (R + 31) / 32, W = (C + 31) / 32;
+    for (size_t j = 0; j < R; j++) {
+        size_t n = 0;
+        std::fill(out + 32 * j, out + 32 * (j + 1), (uint16_t)0);
+        for (size_t i = 0; i < C; i++)
+            for (size_t l = 0; l < 32; l++) {
+                const size_t word = (j * W + i / 32) * 32 + l;
+                if (!(tab[word * bytes + (i % 32) / 8] >> (i % 8) & 1)) continue;
+                if (++n <= 31) out[32 * j + n] = (uint16_t)(i * 32 + l);
+            }
+        out[32 * j] = n <= 31 ? (uint16_t)n : (uint16_t)0xFFFF;
+    }
     return RB_OK;
 }
 

@@ -114,12 +114,13 @@ DeviceNet::~DeviceNet() {
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-bool warp_dep_table(const Packed &p, std::vector<uint16_t> &tab) {
+bool warp_dep_masks(const Packed &p, std::vector<unsigned char> &tab, int &word_bytes) {
     const int R = p.R, P = p.P, Q = p.Q;
-    const int C = (R + 31) / 32;
+    const int C = (R + 31) / 32, W = (C + 31) / 32;
     tab.clear();
+    word_bytes = C <= 8 ? 1 : C <= 16 ? 2 : 4;
     if (R < 1 || C > 256) return false;
-    tab.assign((size_t)R * 32, 0);
+    tab.assign((size_t)R * W * 32 * word_bytes, 0);
     // reactions reading each species
     std::vector<std::vector<int32_t>> readers((size_t)p.S);
     for (int r = 0; r < R; r++)
@@ -128,20 +129,15 @@ bool warp_dep_table(const Packed &p, std::vector<uint16_t> &tab) {
                 auto &v = readers[(size_t)p.fac_sp[(size_t)r * P + k]];
                 if (v.empty() || v.back() != r) v.push_back(r);
             }
-    std::vector<int32_t> mark((size_t)R, -1);
-    for (int j = 0; j < R; j++) {
-        int n = 0;
-        uint16_t *row = tab.data() + (size_t)j * 32;
+    for (int j = 0; j < R; j++)
         for (int k = 0; k < Q; k++) {
             if (p.jmp_d[(size_t)j * Q + k] == 0) continue;
-            for (int32_t r : readers[(size_t)p.jmp_sp[(size_t)j * Q + k]])
-                if (mark[(size_t)r] != j) {
-                    mark[(size_t)r] = j;
-                    if (++n <= 31) row[n] = (uint16_t)((r % C) * 32 + r / C);
-                }
+            for (int32_t r : readers[(size_t)p.jmp_sp[(size_t)j * Q + k]]) {
+                const int i = r % C;
+                const size_t word = ((size_t)j * W + i / 32) * 32 + r / C;
+                tab[word * word_bytes + (i % 32) / 8] |= (unsigned char)(1u << (i % 8));  // little-endian words
+            }
         }
-        row[0] = n <= 31 ? (uint16_t)n : (uint16_t)0xFFFF;
-    }
     return true;
 }
 
@@ -382,17 +378,16 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
         per_sm = std::max(1, ssa_warp_occupancy(a, warp_w, smem));
         const int64_t blocks = std::max<int64_t>(
             1, std::min<int64_t>((r.n_traj + warp_w - 1) / warp_w, (int64_t)ctx->sm_count * per_sm));
-        // dependency lists: only the propensities a reaction's jump touches
+        // dependency masks: only the propensities a reaction's jump touches
         // are re-evaluated after it fires (RB_WARP_DEPS=0: all, every step)
         if (dn.dep_version != dn.version) {
             if (dn.dep) cudaFree(dn.dep);
             dn.dep = nullptr;
-            std::vector<uint16_t> tab;
-            dn.dep_ok = warp_dep_table(p, tab);
-            if (dn.dep_ok &&
-                (!cuda_ok(cudaMalloc(&dn.dep, sizeof(uint16_t) * tab.size()), "cudaMalloc(dependency table)") ||
-                 !cuda_ok(cudaMemcpy(dn.dep, tab.data(), sizeof(uint16_t) * tab.size(), cudaMemcpyHostToDevice),
-                          "cudaMemcpy(dependency table)")))
+            std::vector<unsigned char> tab;
+            dn.dep_ok = warp_dep_masks(p, tab, dn.dep_bytes);
+            if (dn.dep_ok && (!cuda_ok(cudaMalloc(&dn.dep, tab.size()), "cudaMalloc(dependency masks)") ||
+                              !cuda_ok(cudaMemcpy(dn.dep, tab.data(), tab.size(), cudaMemcpyHostToDevice),
+                                       "cudaMemcpy(dependency masks)")))
                 return false;
             dn.dep_version = dn.version;
         }
@@ -409,7 +404,10 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
         }
         a.warp_cnt0 = dn.warp_cnt0;
         const char *wd = std::getenv("RB_WARP_DEPS");
-        if (dn.dep_ok && !(wd && std::strcmp(wd, "0") == 0)) a.dep_tab = dn.dep;
+        if (dn.dep_ok && !(wd && std::strcmp(wd, "0") == 0)) {
+            a.dep_tab = dn.dep;
+            a.dep_bytes = dn.dep_bytes;
+        }
         if (const char *xc = std::getenv("RB_WARP_EXACT_CHOICE")) a.exact_choice = std::strcmp(xc, "0") != 0;
         if (timed && !cuda_ok(cudaEventRecord(dn.ev_start, stream), "cudaEventRecord")) return false;
         const int err = launch_ssa_warp(a, warp_w, (int)blocks, smem, stream);

@@ -58,7 +58,8 @@ struct DeviceNet {
     double out_gbs = 0;                 // sample bytes / kernel time of the last host-pointer run
     int64_t *warp_cnt0 = nullptr;       // warp kernel interval-start counts
     size_t warp_cnt0_n = 0;             //   (entries)
-    uint16_t *dep = nullptr;            // warp kernel dependency table [R][32]
+    void *dep = nullptr;                // warp kernel dependency masks (SsaArgs::dep_tab)
+    int dep_bytes = 0;                  //   their word size
     uint64_t dep_version = 0;           //   for this descriptor version (0: none built)
     bool dep_ok = false;                //   false: the network is beyond the lists' reach
     const void *jit_k = nullptr;        // generated kernel last used, for
@@ -67,12 +68,10 @@ struct DeviceNet {
     ~DeviceNet();
 };
 
-// Dependency table of the warp kernel for a packed network ([R][32], see
-// SsaArgs::dep_tab): row j lists the lane-major positions (reaction l*C + i
-// at i*32 + l, C = ceil(R / 32)) of the reactions whose propensity reads a
-// species reaction j changes.  False when the kernel's update groups cannot
-// cover the network (more than 8192 reactions).
-bool warp_dep_table(const Packed &p, std::vector<uint16_t> &tab);
+// Dependency masks of the warp kernel for a packed network (layout and word
+// size: SsaArgs::dep_tab).  False for more than 8192 reactions, whose masks
+// would outgrow the caches that serve one row per event.
+bool warp_dep_masks(const Packed &p, std::vector<unsigned char> &tab, int &word_bytes);
 
 // Make net.dev current for the active device and descriptor version.
 // Caller holds net.mu.  Returns false (error set) on failure.

@@ -95,13 +95,15 @@ struct SsaArgs {
     // slots (every trajectory gets the same number of steps).
     int32_t sched;
 
-    // Warp-per-trajectory kernel, one network: row j of dep_tab ([R][32])
-    // holds the number n of reactions whose propensity reads a species that
-    // reaction j changes, then their lane-major positions (see batch below)
-    // in entries 1 .. n; n = 0xFFFF when there are more than 31.  After j
-    // fires only those are re-evaluated (one coalesced load per step).  Null:
-    // every propensity is re-evaluated at every step.
-    const uint16_t *dep_tab;
+    // Warp-per-trajectory kernel: dep_tab holds, per reaction j and lane l,
+    // ceil(C / 32) words (C = ceil(R / 32) reactions a lane, words of
+    // dep_bytes bytes: 1 for C <= 8, 2 for C <= 16, else 4) whose bit i is set
+    // when lane l's reaction l*C + i reads a species that j changes:
+    // word w of (j, l) at index (j * ceil(C / 32) + w) * 32 + l, one coalesced
+    // load per step.  After j fires only those are re-evaluated.  Null: every
+    // propensity is re-evaluated at every step.
+    const void *dep_tab;
+    int32_t dep_bytes;
     // Warp-per-trajectory kernel: [blocks x warps per block][S] counts at the
     // start of each warp's current sample interval (read only by an exact
     // re-run of the interval, so they stay out of shared memory).

@@ -5,27 +5,39 @@
 // Each step of rebop's direct method (gillespie.rs:315-344) recomputes every
 // propensity and folds them left to right into cumulative sums
 // (make_cumrates, gillespie.rs:357-364).  Here the 32 lanes of a warp own
-// contiguous chunks of the reaction list: each lane evaluates its chunk's
-// propensities in float pairs and sums them, a shuffle scan of the lane sums
-// gives every chunk's prefix and the total, lane 0 holds the random stream,
-// the triple-float clock and its error bound (as in ssa_spec_body.cuh), and
-// the lane whose prefix range holds total * U walks its chunk to the chosen
-// reaction.
+// contiguous chunks of the reaction list and keep every propensity as a 64-bit
+// fixed-point number (units of 2^-E, E chosen per trajectory so that the total
+// fills 52 to 60 bits).  Integer sums are exact and associative, so
+//   * after a reaction fires each lane re-evaluates only those of its own
+//     reactions that read a changed species (a bit mask per reaction and
+//     lane, SsaArgs::dep_tab) and adds the differences to its chunk sum: no
+//     re-summation, no drift, nothing handed between lanes;
+//   * one shuffle scan of the chunk sums (two adds a step) gives every
+//     chunk's prefix and the total, a second one over the chunk that holds
+//     total * U the chosen reaction.
+// The clock is a 64-bit fixed-point number too, counted from the interval's
+// start in units of 2^-58 of the interval.  The random words are generated
+// ahead, 32 at a time, one kept per lane: the lanes then turn all 32 into
+// Exp1 candidates at once, and a step picks up the two words it consumes with
+// shuffles.  The clock arithmetic runs on every lane alike, so no decision has
+// to be handed around.
 //
 // The reference's sums are a sequential binary64 fold, within (R + M + 2)
-// 2^-53 of the exact sums; the float pairs are within a few 2^-44 of them.
-// A decision whose operands lie farther apart than both bounds together is
-// the reference's decision.  A close choice is redone for that step alone
-// with the exact fold below; anything else -- a close clock comparison, a
-// count outside [0, 2^23), a rate outside 2^-60 .. 2^60 -- re-runs the sample
-// interval from its saved start with the exact step: lanes compute the
-// binary64 propensities in the reference's multiply order and fold them in
-// order lane after lane, lane 0 draws in native binary64, so counts, event
-// numbers and the random stream equal rebop's bit for bit.
+// 2^-53 of the exact sums; a fixed-point propensity is within (M + 1) 2^-44 of
+// its own value plus 2 units of the exact one.  A decision whose operands lie
+// farther apart than both bounds together is the reference's decision.  A
+// close choice is redone for that step alone with the exact fold below;
+// anything else -- a close clock comparison, a count outside [0, 2^23), a rate
+// outside 2^-60 .. 2^60 -- re-runs the sample interval from its saved start
+// with the exact step: lanes compute the binary64 propensities in the
+// reference's multiply order and fold them in order lane after lane, lane 0
+// draws in native binary64, so counts, event numbers and the random stream
+// equal rebop's bit for bit.
 //
-// After a reaction fires only the propensities reading a species it changed
-// are re-evaluated (SsaArgs::dep_tab); a lane's chunk is summed in groups, so
-// only the groups holding them are re-summed.
+// Bound: instruction issue and, at 16 warps per SM, the dependent chain of a
+// step: 618 warp instructions per event at 60 % issue on 200 species and 1000
+// reactions (1 216 at 71 % with float-pair sums), 10 000 trajectories of 6.0e4
+// events each in 569 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -49,19 +61,16 @@ struct WarpLayout {
 // i*32 + l -- so one step of the walk touches 32 consecutive words.
 __host__ __device__ inline int warp_chunk(int R) { return (R + 31) / 32; }
 
-// A lane's chunk is summed in groups of warp_group(C) reactions (at most 32
-// groups), so that re-evaluating a few propensities re-sums only their groups.
-__host__ __device__ inline int warp_group(int C) { return C > 256 ? (C + 31) / 32 : 8; }
-__host__ __device__ inline int warp_ngroups(int C) { return (C + warp_group(C) - 1) / warp_group(C); }
-
 // Every reaction of order <= 2 over fewer than 32767 species: propensities
 // come from two-slot shapes (shape_word) and the factor list is not needed.
 __host__ __device__ inline bool warp_shape2(const SsaArgs &a) { return a.max_mults <= 2 && a.S < 32767; }
 
 // Shared memory: block tables (Exp1 tables, float-pair rates when shared,
-// reactant factors in both layouts, jumps), then per warp: counts,
-// float-pair propensities (and float-pair rates when per trajectory).  The
-// counts at the interval start go to global memory (SsaArgs::warp_cnt0).
+// shapes or factors, jumps), then per warp: the generator at the word buffer's
+// start and at the interval's, counts, fixed-point propensities (and
+// float-pair rates when per trajectory).  The counts at the interval start go
+// to global memory (SsaArgs::warp_cnt0).
+constexpr size_t kWarpState = 96;  // generator states: buffer start, before its last word, interval start
 __host__ __device__ inline WarpLayout warp_layout(const SsaArgs &a) {
     WarpLayout l;
     const size_t RP = 32 * (size_t)warp_chunk(a.R);     // lane-major positions
@@ -70,35 +79,89 @@ __host__ __device__ inline WarpLayout warp_layout(const SsaArgs &a) {
         b += 8 * RP;                                        // shared float-pair rates (lane-major)
         if (!warp_shape2(a)) b += 4 * RP * a.P;             // factors (lane-major), when shapes do not cover
         b += 4 * RP;                                        // two-slot reaction shapes (lane-major)
-        b += 2 * (size_t)a.R * a.Q + 2 * (size_t)a.R * a.Q; // jumps: species, deltas (16 bit each)
-        b += 16;                                            // alignment of the jump deltas
+        b += 4 * (size_t)a.R * a.Q;                         // jumps: species, delta (16 bit each)
     }
     l.block_bytes = (b + 15) & ~(size_t)15;
-    size_t w = 8 * (size_t)a.S;                         // counts
+    size_t w = kWarpState + 8 * (size_t)a.S;            // generator states, counts
     w += 4 * ((size_t)a.S + 1);                         // counts as floats, plus the constant 1
     w += 8 * RP + 8;                                    // propensities (lane-major), alignment
     if (a.rate_stride) w += 8 * RP;                     // per-trajectory float-pair rates
-    if (!a.batch) w += 8 * 32 * (size_t)warp_ngroups(warp_chunk(a.R)) + 4 * 32;  // group sums, dirty masks
     const size_t wt = 8 * 32 * (2 * (size_t)a.tbatch_S + 4);  // a thread unit's counts, their copy, generator
     if (a.batch && wt > w) w = wt;
     l.warp_bytes = (w + 15) & ~(size_t)15;
     return l;
 }
 
-// Physical slot of the float-pair propensity at lane-major position pos
+// Physical slot of the propensity at lane-major position pos
 // (reaction l*C + i at i*32 + l): the lane bits are XORed with the row, so a
 // row read by the 32 lanes (the chunk sums) and a column read by the 32 lanes
 // (the walk through one lane's chunk to the chosen reaction) both touch 32
 // distinct banks.  Without it every lane of the walk hit the same bank.
 __device__ __forceinline__ int pz(int pos) { return pos ^ ((pos >> 5) & 31); }
 
-__device__ __forceinline__ DF shfl_df(DF v, int src) {
-    return DF{__shfl_sync(0xffffffffu, v.h, src), __shfl_sync(0xffffffffu, v.l, src)};
+__device__ __forceinline__ int64_t shfl_i64(int64_t v, int src) {
+    return (int64_t)__shfl_sync(0xffffffffu, (long long)v, src);
 }
 
-__device__ __forceinline__ DF shfl_up_df(DF v, int d) {
-    return DF{__shfl_up_sync(0xffffffffu, v.h, d), __shfl_up_sync(0xffffffffu, v.l, d)};
+// Inclusive sum over the lanes of a warp, over the nearest 2 * last lanes
+// (16: all 32): the shuffle's own range predicate guards the two adds.
+template <int D>
+__device__ __forceinline__ void scan_step(int64_t &v) {
+    asm volatile(
+        "{\n .reg .u32 lo, hi, rl, rh;\n .reg .pred p;\n mov.b64 {lo, hi}, %0;\n"
+        " shfl.sync.up.b32 rl|p, lo, %1, 0, 0xffffffff;\n shfl.sync.up.b32 rh, hi, %1, 0, 0xffffffff;\n"
+        " @p add.cc.u32 lo, lo, rl;\n @p addc.u32 hi, hi, rh;\n mov.b64 %0, {lo, hi};\n}\n"
+        : "+l"(v)
+        : "n"(D));
 }
+__device__ __forceinline__ int64_t scan_i64(int64_t v, int width) {
+    scan_step<1>(v);
+    if (width > 2) scan_step<2>(v);
+    if (width > 4) scan_step<4>(v);
+    if (width > 8) scan_step<8>(v);
+    if (width > 16) scan_step<16>(v);
+    return v;
+}
+
+// The warp kernel's fixed-point numbers have 22 fraction bits below the part a
+// 32-bit conversion reaches: v = floor(a) 2^22 + the rest.  64-bit conversions
+// from and to float run on the FP64 pipe here and kept it 67 % busy; the
+// 32-bit ones do not.
+constexpr int kFxLow = 22;
+constexpr int kFxLim = 52;  // single values stay below 2^52: a below 2^30
+
+// round((h + l) 2^22) within one unit (and 2^-47 of the value) for a float pair
+// with 0 <= h < 2^31, |l| <= 2^-20 h; l22 = 2^22 l.
+__device__ __forceinline__ int64_t fx_from_df(float h, float l22) {
+    const int a = __float2int_rz(h);
+    const int b = __float2int_rn(__fmaf_rn(__fsub_rn(h, (float)a), 0x1p22f, l22));
+    return (int64_t)a * (1 << kFxLow) + b;
+}
+
+// Float pair of 0 <= v < 2^57 within 2^-45 (v >= 2^47).
+__device__ __forceinline__ DF df_from_fx(int64_t v) {
+    const int hi = (int)(v >> 27);
+    const float fh = __int2float_rz(hi);
+    const int rest = hi - __float2int_rz(fh);  // below 2^6
+    const int lo = (rest << 25) + (int)((uint32_t)v >> 2 & 0x1FFFFFFu);
+    return DF{__fmul_rn(fh, 0x1p27f), __fmul_rn((float)lo, 4.0f)};
+}
+
+// u 2^-53 for 0 < u < 2^53 as a float pair, within 2^-47 of u itself however
+// small it is.
+__device__ __forceinline__ DF df_u53_rel(uint64_t u) {
+    const int z = __clzll((long long)u);
+    const uint64_t v = u << z;
+    const float s = __uint_as_float((uint32_t)(127 - 13 - z) << 23);
+    return DF{__fmul_rn((float)(uint32_t)(v >> 40), s),
+              __fmul_rn((float)((uint32_t)(v >> 16) & 0xFFFFFFu), __fmul_rn(s, 0x1p-24f))};
+}
+
+// 2^e for -126 <= e <= 126.
+__device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
+// floor(log2(v)) of a positive normal float / double.
+__device__ __forceinline__ int ilog2f(float v) { return (int)(__float_as_uint(v) >> 23) - 127; }
+__device__ __forceinline__ int ilog2d(double v) { return (int)((uint64_t)__double_as_longlong(v) >> 52) - 1023; }
 
 __device__ __forceinline__ double shfl_d(double v, int src) {
     return __longlong_as_double(__shfl_sync(0xffffffffu, __double_as_longlong(v), src));
@@ -233,6 +296,21 @@ __host__ __device__ inline uint32_t shape_word(const int32_t *fac_sp, const int3
         }
     }
     return sl[0] | of[0] << 15 | sl[1] << 16 | of[1] << 31;
+}
+
+// Exp1 draw as a float pair within gamma of itself, consuming the stream as
+// the reference does (exp1_df with the candidate's fraction normalised first).
+__device__ __forceinline__ DF exp1_df_rel(Xoshiro &g, const ExactTables &ex, const float2 *xdf) {
+    for (;;) {
+        const uint64_t b = xo_next(g);
+        const int i = (int)(b & 0xff);
+        const uint64_t k = b >> 12;
+        const float2 X = xdf[i];
+        const DF x = df_mul(df_u53_rel(2 * k + 1), DF{X.x, X.y});
+        if (k < ex.zxk[i].y) return x;
+        if (i == 0) return df_from_double(__dsub_rn(kZigR, log(xo_uniform(g))));
+        if (wedge_df(ex, i, k, x.h, xo_next(g) >> 11)) return x;
+    }
 }
 
 // One thread unit of a persistent batch: lane l runs trajectory first + l of
@@ -401,11 +479,9 @@ __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWar
     const bool shape2 = warp_shape2(a);
     int32_t *facl_sh = reinterpret_cast<int32_t *>(rdf_sh + RP0);  // absent (size 0) when shape2
     uint32_t *shape_sh = reinterpret_cast<uint32_t *>(facl_sh + (shape2 ? 0 : (size_t)RP0 * a.P));
-    // jumps of the one network: species as 16-bit indices (S < 65536), deltas
-    // as 16-bit values when every one fits (else read from the descriptor)
-    uint16_t *jsp_sh = reinterpret_cast<uint16_t *>(shape_sh + RP0);
-    int16_t *jd_sh = reinterpret_cast<int16_t *>(
-        (reinterpret_cast<uintptr_t>(jsp_sh + (size_t)a.R * a.Q) + 15) & ~(uintptr_t)15);
+    // jumps of the one network: species as 16-bit indices (S < 65536) below
+    // deltas of 16 bits when every one fits (else read from the descriptor)
+    uint32_t *jump_sh = shape_sh + RP0;
     for (int k = tid; k < 256; k += blockDim.x) {
         zxk[k] = make_ulonglong2((uint64_t)__double_as_longlong(a.zig[k]),
                                  (uint64_t)__double_as_longlong(a.zig[kZigOffK + k]));
@@ -416,8 +492,7 @@ __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWar
     if (!BATCH) {
         for (int k = tid; k < a.R * a.Q; k += blockDim.x) {
             const int64_t dlt = a.jmp_d[k];
-            jsp_sh[k] = (uint16_t)a.jmp_sp[k];
-            jd_sh[k] = (int16_t)dlt;
+            jump_sh[k] = (uint32_t)a.jmp_sp[k] | ((uint32_t)(uint16_t)dlt << 16);
             jd_wide |= dlt != (int64_t)(int16_t)dlt;
         }
         for (int q = tid; q < RP0; q += blockDim.x) {
@@ -445,13 +520,12 @@ __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWar
 
     // ---- this warp's region (sized for the largest network)
     unsigned char *wbase = g_spec_smem + L.block_bytes + (size_t)warp * L.warp_bytes;
-    int64_t *cnt = reinterpret_cast<int64_t *>(wbase);
+    uint64_t *gst = reinterpret_cast<uint64_t *>(wbase);  // [12]: buffer start, before its last word, interval start
+    int64_t *cnt = reinterpret_cast<int64_t *>(wbase + kWarpState);
     int64_t *cnt0 = a.warp_cnt0 + ((size_t)blockIdx.x * nw + warp) * (size_t)a.S;  // global
     float *cntf = reinterpret_cast<float *>(cnt + a.S);  // [S + 1]
-    float2 *prop = reinterpret_cast<float2 *>((reinterpret_cast<uintptr_t>(cntf + a.S + 1) + 7) & ~(uintptr_t)7);
-    float2 *rdf_w = prop + RP0;  // per-trajectory float-pair rates (single-network mode)
-    float2 *gsum = rdf_w + (a.rate_stride ? RP0 : 0);  // group sums [NG][32] (one network only)
-    uint32_t *dmask = reinterpret_cast<uint32_t *>(gsum + 32 * (size_t)warp_ngroups(C0));  // dirty groups per lane
+    int64_t *prop = reinterpret_cast<int64_t *>((reinterpret_cast<uintptr_t>(cntf + a.S + 1) + 7) & ~(uintptr_t)7);
+    float2 *rdf_w = reinterpret_cast<float2 *>(prop + RP0);  // per-trajectory float-pair rates (single-network mode)
     // exact steps use the propensity array as their scratch (32 * C doubles)
     double *scr = reinterpret_cast<double *>(prop);
     const int64_t t_start = global_ns();
@@ -509,107 +583,77 @@ __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWar
         const int32_t *facl = BATCH ? it.lm_fac : facl_sh;
         const uint32_t *shape = BATCH ? it.lm_shape : shape_sh;
         const bool use_shape = BATCH ? it.lm_shape != nullptr : (it.max_mults <= 2 && it.S < 32767);
-        // reaction j's k-th jump entry: species, delta
-        auto jump_sp = [&](int e) -> int { return BATCH ? it.jmp_sp[e] : (int)jsp_sh[e]; };
-        auto jump_d = [&](int e) -> int64_t { return BATCH || jd_wide ? it.jmp_d[e] : (int64_t)jd_sh[e]; };
         // lane l owns reactions [l * C, min(R, (l + 1) * C)); local index i sits at i*32 + l
         const int r_lo = min(R, lane * C), r_hi = min(R, r_lo + C);
         const int n_own = r_hi - r_lo;
         const int mm = use_shape ? 2 : it.max_mults;  // multiplies per propensity
-        const int GS = warp_group(C), NG = warp_ngroups(C);
-        // dependency table (one network only: a batch's small networks gain
-        // nothing from it); a reaction with more than 31 dependents
-        // re-evaluates everything after it fires
-        const bool deps = !BATCH && a.dep_tab != nullptr;
-        // adds on the way to a chunk sum: a batch sums its chunk in order (C),
-        // one network sums groups and then their sums (at most GS + NG)
-        const int depth = BATCH ? C : GS + NG;
-        const float c_tot = (float)(mm + 1 + depth + 5) * kGamma + (float)(R + mm + 4) * 0x1p-53f;
-        const float c_q = c_tot + 6.0f * kGamma;
-        const float c_sel = 2.0f * (c_tot + (float)(C + 4) * kGamma);
-        // float-pair propensity of the reaction at lane-major position pos;
-        // bad is set when a count it reads lies outside [0, 2^23)
-        auto eval_prop = [&](int pos, bool &bad) -> DF {
+        // dependency masks; without them every propensity is re-evaluated
+        const int dep_bytes = it.dep_bytes, n_words = (C + 31) >> 5;
+        const void *dep_tab = it.dep_tab;
+        // Fixed point: single propensities and the 32 chunk sums stay below
+        // 2^52, so nothing overflows (up to 256 reactions a lane); the total is
+        // scaled to 2^50 .. 2^51, and scaled anew when it falls below 2^47 or a
+        // chunk sum reaches 2^52.
+        // Relative error bound of a propensity or sum against the reference's
+        // binary64 one, apart from one unit per propensity:
+        const float c_p = (float)(mm + 2) * kGamma + (float)(R + mm + 4) * 0x1p-53f;
+        // Exp1 / total: the total's bound (its units at the smallest total),
+        // the Exp1 pair, the total's pair and the division
+        const float c_q = (c_p + (float)(R + 2) * 0x1p-47f + 9.0f * kGamma) * 1.001f;
+        const int sh_q = -ilog2f(c_q) - 1;         // 2^-sh_q >= c_q
+        const int sh_p = -ilog2f(2.0f * c_p) - 1;  // choice: both operands' bounds
+        // fixed-point propensity of the reaction at lane-major position pos, sc
+        // times its value in units of 2^-22; mx collects the largest count it read (as float
+        // bits: a count outside [0, 2^23) has bits >= 0x4B000000), mh the
+        // largest sc * propensity
+        auto eval_prop = [&](int pos, float sc, uint32_t &mx, float &mh) -> int64_t {
             const float2 k = rdf[pos];
-            if (use_shape) {
-                const uint32_t w = shape[pos];
-                const float n1 = cntf[w & 0x7FFFu], n2 = cntf[(w >> 16) & 0x7FFFu];
-                bad |= !(n1 >= 0.0f && n1 < 8388608.0f && n2 >= 0.0f && n2 < 8388608.0f);
-                const float f1 = fmaxf(__fsub_rn(n1, (float)((w >> 15) & 1u)), 0.0f);
-                const float f2 = fmaxf(__fsub_rn(n2, (float)(w >> 31)), 0.0f);
-                return df_mul_fu(df_mul_fu(DF{k.x, k.y}, f1), f2);
-            }
-            const int i2 = pos >> 5, l = pos & 31;
             DF acc{k.x, k.y};
-            for (int p = 0; p < P; ++p) {
-                const int f = facl[(i2 * P + p) * 32 + l];
-                const int o = f >> 16;
-                if (o == 0) continue;
-                const int64_t n = cnt[f & 0xFFFF];
-                bad |= (uint64_t)n >= (1ull << 23);
-                for (int j = 0; j < o; ++j) {
-                    const int64_t x = n - j > 0 ? n - j : 0;
-                    acc = df_mul_fu(acc, f23((uint32_t)x & 0x7FFFFFu));
+            if (use_shape) {
+                const uint32_t w = shape[pos];  // the first slot's offset is 0
+                const float n1 = cntf[w & 0x7FFFu], n2 = cntf[(w >> 16) & 0x7FFFu];
+                mx = max(mx, max(__float_as_uint(n1), __float_as_uint(n2)));
+                acc = df_mul_fu(df_mul_fu(acc, n1), fmaxf(__fsub_rn(n2, (float)(w >> 31)), 0.0f));
+            } else {
+                const int i2 = pos >> 5, l = pos & 31;
+                for (int p = 0; p < P; ++p) {
+                    const int f = facl[(i2 * P + p) * 32 + l];
+                    const int o = f >> 16;
+                    if (o == 0) continue;
+                    const float n = cntf[f & 0xFFFF];
+                    mx = max(mx, __float_as_uint(n));
+                    for (int j = 0; j < o; ++j) acc = df_mul_fu(acc, fmaxf(__fsub_rn(n, (float)j), 0.0f));
+                    acc = fast2sum(acc.h, acc.l);
                 }
             }
-            return acc;
+            const float hs = __fmul_rn(acc.h, sc);
+            mh = fmaxf(mh, hs);
+            return fx_from_df(hs, __fmul_rn(acc.l, __fmul_rn(sc, 0x1p22f)));
         };
-        // sum of this lane's group g (its propensities already in prop), as
-        // a pairwise tree for groups of 8
-        auto group_sum = [&](int g) -> DF {
-            const int b = g * GS, e = min(n_own, b + GS);
-            if (GS == 8) {
-                DF v[8];
-#pragma unroll
-                for (int t = 0; t < 8; ++t) {
-                    const float2 q = b + t < e ? prop[pz((b + t) * 32 + lane)] : make_float2(0.f, 0.f);
-                    v[t] = DF{q.x, q.y};
-                }
-                return df_add(df_add(df_add(v[0], v[1]), df_add(v[2], v[3])),
-                              df_add(df_add(v[4], v[5]), df_add(v[6], v[7])));
-            }
-            DF s{0.f, 0.f};
-            for (int i2 = b; i2 < e; ++i2) {
-                const float2 q = prop[pz(i2 * 32 + lane)];
-                s = df_add(s, DF{q.x, q.y});
-            }
-            return s;
-        };
-        // this lane's chunk sum from its group sums (pairwise up to 4 groups)
-        auto chunk_sum = [&]() -> DF {
-            if (NG <= 4) {
-                DF v[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    const float2 q = t < NG ? gsum[t * 32 + lane] : make_float2(0.f, 0.f);
-                    v[t] = DF{q.x, q.y};
-                }
-                return df_add(df_add(v[0], v[1]), df_add(v[2], v[3]));
-            }
-            DF s{0.f, 0.f};
-            for (int g = 0; g < NG; ++g) {
-                const float2 q = gsum[g * 32 + lane];
-                s = df_add(s, DF{q.x, q.y});
-            }
-            return s;
-        };
-        bool need_full = true;  // every propensity to be evaluated
+        bool need_full = true;  // every propensity to be evaluated, the scale chosen anew
         bool amb_next = false;  // a re-evaluated propensity read a count out of range
-        DF ls{0.f, 0.f};        // this lane's chunk sum
+        bool absorbed = false;  // every propensity is 0
+        float sc = 1.0f;        // scale of the fixed point
+        int64_t ls = 0;         // this lane's chunk sum
 
-        // ---- start (or resume) the trajectory
-        Xoshiro g{0, 0, 0, 0};
+        // ---- start (or resume) the trajectory.  g (the same on every lane) is
+        // the generator past the word buffer, word p of which comes next
+        // (p = 32: empty); x and acc_mask are the words' Exp1 candidates and
+        // which of them the ziggurat's first test accepts.
+        Xoshiro g;
+        int p = 32;
+        uint64_t word = 0;
+        DF x{0.f, 0.f};
+        uint32_t acc_mask = 0;
         double t;
         if (it.in_species) {
             for (int s = lane; s < S; s += 32) cnt[s] = it.in_species[traj * S + s];
             t = it.in_t[traj];
-            if (lane == 0)
-                g = Xoshiro{it.in_rng[traj * 4], it.in_rng[traj * 4 + 1], it.in_rng[traj * 4 + 2],
-                            it.in_rng[traj * 4 + 3]};
+            g = Xoshiro{it.in_rng[traj * 4], it.in_rng[traj * 4 + 1], it.in_rng[traj * 4 + 2], it.in_rng[traj * 4 + 3]};
         } else {
             for (int s = lane; s < S; s += 32) cnt[s] = it.x0[traj * it.x0_stride + s];
             t = 0.0;
-            if (lane == 0) xo_seed(g, it.seeds[traj]);
+            xo_seed(g, it.seeds[traj]);
         }
         const double *rates = it.rate + traj * it.rate_stride;
         bool exact_traj = !spec_rate_ok((uint64_t)__double_as_longlong(t)) || !(t < 0x1p60);
@@ -620,22 +664,46 @@ __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWar
                 const DF d = r < R ? df_from_double(rates[r]) : DF{0.f, 0.f};
                 rdf_w[q] = make_float2(d.h, d.l);
             }
-        exact_traj = __any_sync(0xffffffffu, exact_traj);
+        exact_traj = __any_sync(0xffffffffu, exact_traj) || mm > 1024;  // (choice margins stay below 2^32 units)
         for (int s = lane; s <= S; s += 32) cntf[s] = s < S ? (float)cnt[s] : 1.0f;
         __syncwarp();
         unsigned long long ev = 0;
 
+        // the generator before word q of the buffer that starts at state st
+        auto state_at = [&](const uint64_t *st, int q) {
+            Xoshiro h{st[0], st[1], st[2], st[3]};
+            for (int k = 0; k < q; ++k) xo_next(h);
+            return h;
+        };
         for (long long i = 0; i < it.n_samples && !abort_run; ++i) {
             const double T = it.sample_t[i];
             // ---- interval start: save what an exact re-run needs
             for (int s = lane; s < S; s += 32) cnt0[s] = cnt[s];
-            const Xoshiro g0 = g;
+            const int p0 = p;
+            __syncwarp();
+            if (lane == 0) {
+                const bool empty = p == 32;  // then the generator itself is the state
+                gst[8] = empty ? g.s0 : gst[0];
+                gst[9] = empty ? g.s1 : gst[1];
+                gst[10] = empty ? g.s2 : gst[2];
+                gst[11] = empty ? g.s3 : gst[3];
+            }
             const double t0 = t;
             const unsigned long long ev0 = ev;
-            const TF Tc = tf_from_double(T);
-            TF tc = tf_from_double(t0);
-            float err_t = 0.0f;
             bool replay = exact_traj || !(T < 0x1p60) || (T != 0.0 && !(T >= 0x1p-60));
+            // clock: units of 2^-et from t0 on; the interval (the sample time
+            // itself when it is empty or lies behind t0) fills 2^50 .. 2^51
+            const double len = __dsub_rn(T, t0);
+            const double base = len > 0.0 ? len : (T > 0.0 ? T : 1.0);
+            replay |= !(base >= 0x1p-60) || !(fabs(len) <= base * 0x1p2);
+            const int et = replay ? 0 : 50 - ilog2d(base);
+            const double ets = __longlong_as_double((long long)(1023 + et) << 52);
+            const float etf = pow2f(et);
+            const int64_t D = replay ? 0 : __double2ll_rn(__dmul_rn(len, ets));
+            // what a step adds to the clock's error bound beside the quotient's:
+            // the reference's rounding (2^-52 T), the conversions' units
+            const int64_t err_step = replay ? 0 : __double2ll_ru(__dmul_ru(__dmul_ru(T, 0x1p-52), ets)) + 4;
+            int64_t clk = 0, err = 2 * err_step;
             __syncwarp();
             unsigned int steps = 0;
             while (!replay) {
@@ -646,162 +714,208 @@ __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWar
                         break;
                     }
                 }
-                // ---- float-pair propensities of this lane's chunk and their sum
-                bool amb = amb_next;
-                amb_next = false;
-                if (BATCH) {
-                    ls = DF{0.f, 0.f};
+                if (need_full || amb_next) {
+                    // ---- every propensity of this lane's chunk, after the
+                    // scale: 2^28 <= total * sc < 2^29
+                    uint32_t mx = amb_next ? 0x7F800000u : 0u;
+                    float mh = 0.0f, tf = 0.0f;
+                    for (int i2 = 0; i2 < n_own && !amb_next; ++i2) {
+                        float h = 0.0f;
+                        eval_prop(i2 * 32 + lane, 1.0f, mx, h);
+                        tf = __fadd_rn(tf, h);
+                    }
+#pragma unroll
+                    for (int d = 16; d > 0; d >>= 1) tf = __fadd_rn(tf, __shfl_xor_sync(0xffffffffu, tf, d));
+                    // an undecided step: a count out of range, a total beyond
+                    // 2^90 or below 2^-90 (where a positive one is possible)
+                    if (__any_sync(0xffffffffu, mx >= 0x4B000000u) || !(tf <= 0x1p90f) || (tf > 0.0f && tf < 0x1p-60f)) {
+                        replay = true;
+                        break;
+                    }
+                    absorbed = tf == 0.0f;
+                    sc = absorbed ? 1.0f : pow2f(28 - ilog2f(tf));
+                    ls = 0;
                     for (int i2 = 0; i2 < n_own; ++i2) {
-                        const DF acc = eval_prop(i2 * 32 + lane, amb);
-                        prop[pz(i2 * 32 + lane)] = make_float2(acc.h, acc.l);
-                        ls = df_add(ls, acc);
+                        const int64_t v = eval_prop(i2 * 32 + lane, sc, mx, mh);
+                        prop[pz(i2 * 32 + lane)] = v;
+                        ls += v;
                     }
-                } else if (need_full) {
-                    for (int g = 0; g < NG; ++g) {
-                        const int e = min(n_own, (g + 1) * GS);
-                        for (int i2 = g * GS; i2 < e; ++i2) {
-                            const DF acc = eval_prop(i2 * 32 + lane, amb);
-                            prop[pz(i2 * 32 + lane)] = make_float2(acc.h, acc.l);
-                        }
-                        const DF gs = group_sum(g);
-                        gsum[g * 32 + lane] = make_float2(gs.h, gs.l);
-                    }
-                    ls = chunk_sum();
-                    dmask[lane] = 0u;
-                    need_full = !deps;
+                    need_full = false;
                     __syncwarp();
                 }
-                // inclusive scan of the chunk sums
-                DF incl = ls;
-#pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const DF o = shfl_up_df(incl, d);
-                    if (lane >= d) incl = df_add(o, incl);
+                // ---- chunk prefixes and the total
+                const int64_t incl = scan_i64(ls, 32);
+                const int64_t tot = shfl_i64(incl, 31);
+                if (tot < (1ll << 47)) {
+                    if (absorbed) break;  // no reaction can fire: the sample records, no draw is made
+                    need_full = true;     // too few bits left (a new scale's total has 50)
+                    continue;
                 }
-                const DF tot = shfl_df(incl, 31);
-                amb = __any_sync(0xffffffffu, amb) || tot.h > 0x1p90f || (tot.h > 0.0f && tot.h < 0x1p-90f);
-
-                // ---- lane 0: Exp1 draw, clock, decision; then the uniform
-                int state = 0;  // 0 record, 1 fire, 2 undecided
-                DF ch{0.f, 0.f};
-                uint64_t u53 = 0;  // the choice uniform's top 53 bits (lane 0)
-                if (lane == 0 && !amb && tot.h > 0.0f) {
-                    float xerr;
-                    Xoshiro gt = g;
-                    const DF x = exp1_df(gt, ex, xdf, xerr);
-                    const float rr = rcp_approx(tot.h);
-                    const DF q = df_div(x, tot, rr);
-                    const TF tn = tf_add(tc, q);
-                    float err_tn = __fadd_ru(err_t, __fmul_ru(c_q, q.h));
-                    err_tn = __fadd_ru(err_tn, __fmul_ru(__fmul_ru(xerr, rr), 1.001f));
-                    err_tn = __fadd_ru(err_tn, __fmul_ru(0x1p-52f, tn.h));
-                    err_tn = __fadd_ru(err_tn, __fmul_ru(0x1p-23f, fabsf(tn.l)));
-                    const float d = __fadd_rn(__fsub_rn(Tc.h, tn.h),
-                                              __fadd_rn(__fsub_rn(Tc.m, tn.m), __fsub_rn(Tc.l, tn.l)));
-                    const float mt = __fadd_ru(err_tn, __fmul_ru(0x1p-44f, fmaxf(Tc.h, tn.h)));
-                    const float dd = __fmul_rn(d, 1.0f - 0x1p-22f);
-                    if (!(err_tn < 1.0e30f) || q.h < 0x1p-100f) {
-                        state = 2;
-                    } else if (dd > mt) {
-                        state = 1;
-                        u53 = xo_next(gt) >> 11;
-                        ch = df_mul(tot, df_u53(u53));
-                        g = gt;
-                        tc = tn;
-                        err_t = err_tn;
-                    } else if (dd < -mt) {
-                        state = 0;
-                        g = gt;  // the sample records; the Exp1 draw was made
-                    } else {
-                        state = 2;
+                // ---- draws: refill the buffer when fewer than two words are left
+                if (p > 30) {
+                    __syncwarp();
+                    int first = 0;
+                    uint64_t w0 = 0;
+                    if (p == 31) {  // the last word is still to come
+                        first = 1;
+                        w0 = (uint64_t)shfl_i64((int64_t)word, 31);
+                        if (lane < 4) gst[lane] = gst[4 + lane];
+                    } else if (lane == 0) {
+                        gst[0] = g.s0;
+                        gst[1] = g.s1;
+                        gst[2] = g.s2;
+                        gst[3] = g.s3;
                     }
+                    word = w0;
+                    for (int k = first; k < 31; ++k) {
+                        const uint64_t w = xo_next(g);
+                        if (lane == k) word = w;
+                    }
+                    __syncwarp();
+                    if (lane == 0) {
+                        gst[4] = g.s0;
+                        gst[5] = g.s1;
+                        gst[6] = g.s2;
+                        gst[7] = g.s3;
+                    }
+                    const uint64_t w = xo_next(g);
+                    if (lane == 31) word = w;
+                    p = 0;
+                    const int layer = (int)(word & 0xff);
+                    const float2 X = xdf[layer];
+                    x = df_mul(df_u53_rel(2 * (word >> 12) + 1), DF{X.x, X.y});
+                    acc_mask = __ballot_sync(0xffffffffu, (word >> 12) < zxk[layer].y);
+                    __syncwarp();
                 }
-                if (amb) state = 2;
-                state = __shfl_sync(0xffffffffu, state, 0);
-                if (state == 2) {
-                    replay = true;
+                DF xe{__shfl_sync(0xffffffffu, x.h, p), __shfl_sync(0xffffffffu, x.l, p)};
+                uint64_t bu = (uint64_t)shfl_i64((int64_t)word, p + 1);
+                int used = p + 1;  // words consumed by the Exp1 draw, counted from the buffer's start
+                const bool slow = !((acc_mask >> p) & 1u);
+                Xoshiro gs{0, 0, 0, 0};
+                if (slow) {
+                    // wedge or tail (1.2 % of draws): the generator itself from
+                    // here on, the buffer is given up
+                    gs = state_at(gst, p);
+                    xe = exp1_df_rel(gs, ex, xdf);
+                }
+                // ---- Exp1 / total in clock units, the decision
+                const DF td = df_from_fx(tot);
+                const DF q = df_div(xe, td, rcp_approx(td.h));  // / (sc 2^22)
+                const float qh = fminf(__fmul_rn(__fmul_rn(q.h, sc), etf), 0x1p30f);
+                const float ql = fmaxf(fminf(__fmul_rn(__fmul_rn(q.l, __fmul_rn(sc, 0x1p22f)), etf), 0x1p30f), -0x1p30f);
+                const int64_t qc = fx_from_df(qh, ql);
+                const int64_t clk_n = clk + qc;
+                const int64_t err_n = err + err_step + (qc >> sh_q);
+                const int64_t d = D - clk_n;
+                if (d <= err_n || q.h < 0x1p-100f) {  // not a clear fire
+                    if (d + err_n >= 0 || q.h < 0x1p-100f) {
+                        replay = true;
+                        break;
+                    }
+                    // the sample records; the Exp1 draw was made
+                    if (slow) {
+                        g = gs;
+                        p = 32;
+                    } else {
+                        p = used;
+                    }
                     break;
                 }
-                if (state == 0) break;  // record
+                clk = clk_n;
+                err = err_n;
+                if (slow) {
+                    bu = xo_next(gs);
+                    g = gs;
+                    p = 32;
+                } else {
+                    p = used + 1;
+                }
                 // ---- the choice: #{r : cum_r < total * U}
-                ch = shfl_df(ch, 0);
-                DF excl = shfl_up_df(incl, 1);  // this chunk's exclusive prefix
-                if (lane == 0) excl = DF{0.f, 0.f};
-                const float msel = c_sel * tot.h;
-                const float di = __fadd_rn(__fsub_rn(incl.h, ch.h), __fsub_rn(incl.l, ch.l));
-                const unsigned int below = __ballot_sync(0xffffffffu, di < 0.0f);
-                bool close = fabsf(di) <= msel;
-                const int k = __popc(below);  // chunks entirely below the choice
+                const int64_t ch = (int64_t)__umul64hi((uint64_t)tot, bu & ~0x7FFull);
+                const int64_t di = incl - ch;
+                const int k = __popc(__ballot_sync(0xffffffffu, di < 0));  // chunks entirely below the choice
+                const int64_t before = shfl_i64(incl - ls, k & 31);        // running sum before chunk k
+                bool near = (uint32_t)((int)(di >> 32) + 1) <= 1u;         // |di| < 2^32
                 // walk chunk k with the whole warp: lane j takes its reaction k*C + j
-                int idx = R;
-                if (k < 32) {
-                    DF carry = shfl_df(excl, k);
-                    int count = 0;
+                int count = 0;
+                int64_t carry = before - ch, dr = di;
+                for (int seg = 0; seg < C; seg += 32) {
+                    const int j = seg + lane;
+                    const bool valid = j < C && k * C + j < R;
+                    dr = carry + scan_i64(valid ? prop[pz(j * 32 + k)] : 0, C);
+                    count += __popc(__ballot_sync(0xffffffffu, valid && dr < 0));
+                    near |= (uint32_t)((int)(dr >> 32) + 1) <= 1u;
+                    if (C > 32) carry = shfl_i64(dr, 31);
+                }
+                int idx = k * C + count;
+                if (__any_sync(0xffffffffu, near) || a.exact_choice) {
+                    // some sum lies within 2^32 units of the choice: within the
+                    // margin the choice alone is redone exactly (the clock is
+                    // decided; the fixed-point propensities are overwritten)
+                    const int64_t m = (tot >> sh_p) + 4 * (int64_t)R + 16;
+                    bool close = di <= m && di >= -m;
                     for (int seg = 0; seg < C; seg += 32) {
                         const int j = seg + lane;
-                        const bool valid = j < C && k * C + j < R;
-                        DF v{0.f, 0.f};
-                        if (valid) {
-                            const float2 pa = prop[pz(j * 32 + k)];
-                            v = DF{pa.x, pa.y};
-                        }
-#pragma unroll
-                        for (int d2 = 1; d2 < 32; d2 <<= 1) {
-                            const DF o = shfl_up_df(v, d2);
-                            if (lane >= d2) v = df_add(o, v);
-                        }
-                        const DF cum = df_add(carry, v);
-                        const float dr = __fadd_rn(__fsub_rn(cum.h, ch.h), __fsub_rn(cum.l, ch.l));
-                        count += __popc(__ballot_sync(0xffffffffu, valid && dr < 0.0f));
-                        close |= valid && fabsf(dr) <= msel;
-                        carry = shfl_df(cum, 31);
+                        if (seg == 0) carry = before - ch;
+                        dr = carry + scan_i64(j < C && k * C + j < R ? prop[pz(j * 32 + k)] : 0, 32);
+                        close |= dr <= m && dr >= -m;
+                        carry = shfl_i64(dr, 31);
                     }
-                    idx = k * C + count;
-                }
-                if (__any_sync(0xffffffffu, close) || a.exact_choice) {
-                    // the clock is decided: only the choice is redone, exactly
-                    // (the float-pair propensities are overwritten)
-                    idx = warp_exact_choice<MACRO>(it, cnt, rates, scr, __shfl_sync(0xffffffffu, u53, 0));
-                    need_full = true;
+                    if (__any_sync(0xffffffffu, close) || a.exact_choice) {
+                        __syncwarp();
+                        idx = warp_exact_choice<MACRO>(it, cnt, rates, scr, bu >> 11);
+                        need_full = true;
+                    }
                 }
                 // ---- jump
                 ++ev;
                 if (idx < R)
-                    for (int q = lane; q < Q; q += 32) {
-                        const int64_t dlt = jump_d(idx * Q + q);
+                    for (int q2 = lane; q2 < Q; q2 += 32) {
+                        int sp;
+                        int64_t dlt;
+                        if (BATCH || jd_wide) {
+                            sp = it.jmp_sp[idx * Q + q2];
+                            dlt = it.jmp_d[idx * Q + q2];
+                        } else {
+                            const uint32_t e = jump_sh[idx * Q + q2];
+                            sp = (int)(e & 0xFFFFu);
+                            dlt = (int64_t)((int32_t)e >> 16);
+                        }
                         if (dlt != 0) {
-                            const int sp = jump_sp(idx * Q + q);
                             cnt[sp] += dlt;
                             cntf[sp] = __fadd_rn(cntf[sp], (float)dlt);
                         }
                     }
                 __syncwarp();
-                // ---- re-evaluate the propensities the jump touched, re-sum
-                // their groups and the chunks holding them
-                if (deps && idx < R && !need_full) {
-                    const int v = a.dep_tab[(size_t)idx * 32 + lane];
-                    const int nd = __shfl_sync(0xffffffffu, v, 0);
-                    if (nd > 31) {
+                // ---- re-evaluate this lane's propensities that read a changed
+                // species; their differences go to the chunk sum
+                if (idx < R && !need_full) {
+                    uint32_t mx = 0u;
+                    float mh = 0.0f;
+                    for (int w = 0; w < n_words; ++w) {
+                        const size_t e = ((size_t)idx * n_words + w) * 32 + lane;
+                        const int left = n_own - 32 * w;
+                        uint32_t m = left >= 32 ? 0xFFFFFFFFu : left > 0 ? (1u << left) - 1u : 0u;
+                        if (dep_tab)
+                            m = dep_bytes == 1   ? reinterpret_cast<const uint8_t *>(dep_tab)[e]
+                                : dep_bytes == 2 ? reinterpret_cast<const uint16_t *>(dep_tab)[e]
+                                                 : reinterpret_cast<const uint32_t *>(dep_tab)[e];
+                        while (m) {
+                            const int pos = (32 * w + __ffs((int)m) - 1) * 32 + lane;
+                            m &= m - 1u;
+                            const int64_t v = eval_prop(pos, sc, mx, mh);
+                            const int ps = pz(pos);
+                            ls += v - prop[ps];
+                            prop[ps] = v;
+                        }
+                    }
+                    __syncwarp();
+                    // a count out of range makes the next step undecided, a
+                    // sum that outgrew the fixed point asks for a new scale
+                    const bool out = mx >= 0x4B000000u;
+                    if (__any_sync(0xffffffffu, out || !(mh < 0x1p30f) || (uint64_t)ls >> kFxLim != 0)) {
+                        amb_next = __any_sync(0xffffffffu, out);
                         need_full = true;
-                    } else {
-                        if (lane >= 1 && lane <= nd) {
-                            const DF acc = eval_prop(v, amb_next);
-                            prop[pz(v)] = make_float2(acc.h, acc.l);
-                            atomicOr(&dmask[v & 31], 1u << ((v >> 5) / GS));
-                        }
-                        __syncwarp();
-                        uint32_t m = dmask[lane];
-                        if (m) {
-                            dmask[lane] = 0u;
-                            while (m) {
-                                const int g = __ffs((int)m) - 1;
-                                m &= m - 1u;
-                                const DF gs = group_sum(g);
-                                gsum[g * 32 + lane] = make_float2(gs.h, gs.l);
-                            }
-                            ls = chunk_sum();
-                        }
-                        __syncwarp();
                     }
                 }
             }
@@ -810,7 +924,8 @@ __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWar
                 // ---- exact re-run of the interval from its saved start
                 if (!exact_traj && lane == 0) atomicAdd(a.work + 3, 1ull);
                 for (int s = lane; s < S; s += 32) cnt[s] = cnt0[s];
-                g = g0;
+                g = state_at(gst + 8, p0 == 32 ? 0 : p0);
+                p = 32;
                 t = t0;
                 ev = ev0;
                 __syncwarp();
@@ -827,8 +942,8 @@ __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWar
                     ++ev;
                     if (idx < R)
                         for (int q = lane; q < Q; q += 32) {
-                            const int64_t dlt = jump_d(idx * Q + q);
-                            if (dlt != 0) cnt[jump_sp(idx * Q + q)] += dlt;
+                            const int64_t dlt = it.jmp_d[idx * Q + q];
+                            if (dlt != 0) cnt[it.jmp_sp[idx * Q + q]] += dlt;
                         }
                     __syncwarp();
                 }
@@ -836,6 +951,11 @@ __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWar
                 for (int s = lane; s < S; s += 32) cntf[s] = (float)cnt[s];
                 need_full = true;
                 amb_next = false;
+                // lane 0 drew: its generator is the trajectory's
+                g.s0 = (uint64_t)shfl_i64((int64_t)g.s0, 0);
+                g.s1 = (uint64_t)shfl_i64((int64_t)g.s1, 0);
+                g.s2 = (uint64_t)shfl_i64((int64_t)g.s2, 0);
+                g.s3 = (uint64_t)shfl_i64((int64_t)g.s3, 0);
                 __syncwarp();
             }
             // ---- record sample i at t = T
@@ -850,6 +970,7 @@ __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWar
         }
         if (it.fin_species)
             for (int s = lane; s < S; s += 32) it.fin_species[traj * S + s] = cnt[s];
+        if (it.fin_rng && p < 32) g = state_at(gst, p);
         if (lane == 0) {
             if (it.fin_t) it.fin_t[traj] = t;
             if (it.fin_rng) {
