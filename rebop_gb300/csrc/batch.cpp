@@ -253,6 +253,8 @@ bool Batch::build(cudaStream_t st) {
     }
     // warp batch items
     int32_t maxS = 1, maxR = 1, maxP = 1, maxQ = 1;
+    int64_t n_warp = 0;  // trajectories, and the mean length of their dependency lists
+    double deps = 0.0;
     for (int i : warp_items) {
         Item &it = items[i];
         const Packed &p = it.packed;
@@ -260,7 +262,6 @@ bool Batch::build(cudaStream_t st) {
         maxR = std::max(maxR, p.R);
         maxP = std::max(maxP, p.P);
         maxQ = std::max(maxQ, p.Q);
-        const size_t RP = 32 * (size_t)((p.R + 31) / 32);
         it.o_x0 = take(8 * (size_t)(it.in.x0_per_traj ? it.in.n_traj : 1) * p.S);
         it.o_seeds = take(8 * (size_t)it.in.n_traj);
         it.o_times = take(8 * (size_t)(it.in.nb_steps + 1));
@@ -270,13 +271,12 @@ bool Batch::build(cudaStream_t st) {
         it.o_ford = take(4 * (size_t)p.R * p.P);
         it.o_jsp = take(4 * (size_t)p.R * p.Q);
         it.o_jd = take(8 * (size_t)p.R * p.Q);
-        it.o_rdf = take(8 * RP);
-        it.o_lfac = take(4 * RP * p.P);
-        it.o_shape = take(4 * RP);
-        it.dep_bytes = 0;
-        std::vector<unsigned char> dep;
-        if (warp_dep_masks(p, dep, it.dep_bytes)) it.o_dep = take(dep.size());
-        else it.dep_bytes = 0;
+        it.o_rdf = take(8 * (size_t)std::max(p.R, 1));
+        it.o_shape = take(4 * (size_t)std::max(p.R * p.P, 1));
+        it.o_jump = take(4 * (size_t)std::max(p.R * p.Q, 1));
+        if (warp_dep_lists(p, it.dep_head, it.dep_list)) it.o_dep = take(4 * it.dep_head.size() + 2 * it.dep_list.size());
+        n_warp += it.in.n_traj;
+        deps += warp_mean_deps(p, it.dep_head) * (double)it.in.n_traj;
     }
     // thread-unit items
     int32_t maxTS = 1;
@@ -314,7 +314,7 @@ bool Batch::build(cudaStream_t st) {
         it.o_out = take(8 * (size_t)(it.in.nb_steps + 1) * it.save.size() * it.in.n_traj);
         it.o_events = take(8 * (size_t)std::max<int64_t>(it.in.n_traj, 1));
     }
-    o_work = take(8 * 4);
+    o_work = take(8 * 5);
     total_bytes = off;
     if (!cuda_ok(cudaMallocHost(&host, total_bytes), "cudaMallocHost(batch staging)") ||
         !cuda_ok(cudaMalloc(&dev, total_bytes), "cudaMalloc(batch arena)"))
@@ -339,6 +339,7 @@ bool Batch::build(cudaStream_t st) {
         la.Q = maxQ;
         la.batch = reinterpret_cast<const SsaArgs *>(d + o_items);
         la.tbatch_S = maxTS;
+        la.group = ssa_warp_group(la, n_warp, n_warp ? deps / (double)n_warp : 0.0, ctx->smem_optin, ctx->sm_count);
         warp_warps = ssa_warp_warps(la, ctx->smem_optin);
         if (warp_warps < 1) {
             set_error("the largest network of the batch does not fit the warp kernel");
@@ -389,27 +390,33 @@ bool Batch::build(cudaStream_t st) {
             x.events = reinterpret_cast<uint64_t *>(d + it.o_events);
             x.max_mults = mm;
             x.lm_rdf = reinterpret_cast<const float2 *>(d + it.o_rdf);
-            x.lm_fac = reinterpret_cast<const int32_t *>(d + it.o_lfac);
-            x.lm_shape = (mm <= 2 && p.S < 32767) ? reinterpret_cast<const uint32_t *>(d + it.o_shape) : nullptr;
-            if (it.dep_bytes) {
-                std::vector<unsigned char> dep;
-                int bytes = 0;
-                warp_dep_masks(p, dep, bytes);
-                std::memcpy(h + it.o_dep, dep.data(), dep.size());
-                x.dep_tab = d + it.o_dep;
-                x.dep_bytes = bytes;
+            x.lm_shape = reinterpret_cast<const uint32_t *>(d + it.o_shape);
+            if (!it.dep_head.empty()) {
+                const size_t hb = 4 * it.dep_head.size();
+                std::memcpy(h + it.o_dep, it.dep_head.data(), hb);
+                std::memcpy(h + it.o_dep + hb, it.dep_list.data(), 2 * it.dep_list.size());
+                x.dep_head = reinterpret_cast<const uint32_t *>(d + it.o_dep);
+                x.dep_list = reinterpret_cast<const uint16_t *>(d + it.o_dep + hb);
+                it.dep_head = std::vector<uint32_t>();
+                it.dep_list = std::vector<uint16_t>();
             }
-            // lane-major factor and shape tables
-            const int C = (p.R + 31) / 32, RP = 32 * C;
-            int32_t *lf = reinterpret_cast<int32_t *>(h + it.o_lfac);
+            // jumps with 16-bit species and deltas, when every one fits
+            uint32_t *jp = reinterpret_cast<uint32_t *>(h + it.o_jump);
+            bool narrow = true;
+            for (size_t e = 0; e < p.jmp_d.size(); e++) {
+                narrow = narrow && p.jmp_d[e] == (int64_t)(int16_t)p.jmp_d[e];
+                jp[e] = (uint32_t)p.jmp_sp[e] | ((uint32_t)(uint16_t)p.jmp_d[e] << 16);
+            }
+            x.lm_jump = narrow ? reinterpret_cast<const uint32_t *>(d + it.o_jump) : nullptr;
+            // two-slot shapes, or the factors (as the kernel tells them apart)
             uint32_t *sh = reinterpret_cast<uint32_t *>(h + it.o_shape);
-            for (int q = 0; q < RP; q++) {
-                const int i2 = q >> 5, l = q & 31, r = l * C + i2;
-                for (int f = 0; f < p.P; f++)
-                    lf[(i2 * p.P + f) * 32 + l] =
-                        r < p.R ? (p.fac_sp[(size_t)r * p.P + f] | (p.fac_ord[(size_t)r * p.P + f] << 16)) : 0;
-                sh[q] = r < p.R ? warp_shape_word(p.fac_sp.data(), p.fac_ord.data(), p.P, p.S, r)
-                                : ((uint32_t)p.S << 16 | (uint32_t)p.S);
+            const bool shape2 = mm <= 2 && p.S < 32767;
+            for (int32_t r = 0; r < p.R; r++) {
+                if (shape2) sh[r] = warp_shape_word(p.fac_sp.data(), p.fac_ord.data(), p.P, p.S, r);
+                else
+                    for (int f = 0; f < p.P; f++)
+                        sh[(size_t)r * p.P + f] =
+                            (uint32_t)(p.fac_sp[(size_t)r * p.P + f] | (p.fac_ord[(size_t)r * p.P + f] << 16));
             }
         }
         start[warp_items.size()] = acc;
@@ -468,6 +475,7 @@ bool Batch::build(cudaStream_t st) {
         warp_args.P = maxP;
         warp_args.Q = maxQ;
         warp_args.macro_mode = macro_mode;
+        warp_args.group = la.group;
         warp_args.n_traj = acc + units;
         warp_args.n_warp_tickets = acc;
         warp_args.batch = reinterpret_cast<const SsaArgs *>(d + o_items);
@@ -480,12 +488,16 @@ bool Batch::build(cudaStream_t st) {
         warp_args.work = reinterpret_cast<unsigned long long *>(d + o_work);
         warp_args.zig = ctx->zig;
         warp_args.budget_ns = kernel_budget_ns();
-        const int per_sm = std::max(1, ssa_warp_occupancy(warp_args, warp_warps, ssa_warp_smem(warp_args, warp_warps)));
-        warp_grid = (int)std::max<int64_t>(
-            1, std::min<int64_t>((acc + units + warp_warps - 1) / warp_warps, (int64_t)ctx->sm_count * per_sm));
+        // one block per SM, no more warps in it than spread the work over all
+        // SMs: a warp runs a thread unit or 32 / group trajectories of the
+        // larger networks side by side
+        const int side = 32 / la.group;
+        const int64_t want = (acc + side - 1) / side + units;
+        warp_warps = (int)std::max<int64_t>(1, std::min<int64_t>(warp_warps, (want + ctx->sm_count - 1) / ctx->sm_count));
+        warp_grid = (int)std::max<int64_t>(1, std::min<int64_t>((want + warp_warps - 1) / warp_warps, ctx->sm_count));
         if (warp_cnt0) cudaFree(warp_cnt0);
         warp_cnt0 = nullptr;
-        if (!cuda_ok(cudaMalloc(&warp_cnt0, 8 * (size_t)warp_grid * warp_warps * std::max(maxS, 1)),
+        if (!cuda_ok(cudaMalloc(&warp_cnt0, 8 * (size_t)warp_grid * warp_warps * side * std::max(maxS, 1)),
                      "cudaMalloc(interval-start counts)"))
             return false;
         warp_args.warp_cnt0 = warp_cnt0;
@@ -509,7 +521,7 @@ bool Batch::build(cudaStream_t st) {
     // ---------------- capture: inputs in, kernels on two branches, results out
     if (!cuda_ok(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed), "cudaStreamBeginCapture")) return false;
     bool ok = cuda_ok(cudaMemcpyAsync(dev, host, in_bytes, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync(in)");
-    ok = ok && cuda_ok(cudaMemsetAsync(d + o_work, 0, 32, st), "cudaMemsetAsync");
+    ok = ok && cuda_ok(cudaMemsetAsync(d + o_work, 0, 40, st), "cudaMemsetAsync");
     // external record nodes: the events record as plain timed events on replay
     ok = ok && cuda_ok(cudaEventRecordWithFlags(e_in, st, cudaEventRecordExternal), "cudaEventRecordWithFlags");
     ok = ok && cuda_ok(cudaEventRecord(fork, st), "cudaEventRecord") &&
@@ -601,12 +613,8 @@ void Batch::stage_inputs() {
         std::memcpy(h + it.o_seeds, it.in.seeds, 8 * (size_t)n);
         const double *rt = it.in.rates ? it.in.rates : p.rate.data();
         std::memcpy(h + it.o_rates, rt, 8 * (size_t)p.R);
-        const int C = (p.R + 31) / 32, RP = 32 * C;
         float *rdf = reinterpret_cast<float *>(h + it.o_rdf);
-        for (int q = 0; q < RP; q++) {
-            const int r = (q & 31) * C + (q >> 5);
-            float_pair(r < p.R ? rt[r] : 0.0, rdf + 2 * q);
-        }
+        for (int32_t r = 0; r < p.R; r++) float_pair(rt[r], rdf + 2 * r);
     }
     for (int i : thread_items) {
         const Item &it = items[i];

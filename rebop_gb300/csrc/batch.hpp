@@ -47,8 +47,9 @@ struct Batch {
         // not contiguous in the staging buffer (merged classes)
         std::vector<int64_t> own_out;
         size_t o_x0 = 0, o_seeds = 0, o_times = 0, o_save = 0, o_rates = 0, o_fsp = 0, o_ford = 0, o_jsp = 0,
-               o_jd = 0, o_rdf = 0, o_lfac = 0, o_shape = 0, o_dep = 0, o_fpk = 0, o_out = 0, o_events = 0;
-        int dep_bytes = 0;  // dependency mask words (0: none)
+               o_jd = 0, o_rdf = 0, o_shape = 0, o_jump = 0, o_dep = 0, o_fpk = 0, o_out = 0, o_events = 0;
+        std::vector<uint32_t> dep_head;  // warp items: dependency lists (SsaArgs)
+        std::vector<uint16_t> dep_list;
     };
     // A launch of the thread-per-trajectory kernels: items of one structure
     // and sample grid merged (Merged), or one item alone (Single).

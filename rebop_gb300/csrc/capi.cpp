@@ -716,35 +716,30 @@ int rbg_internal_jit_source(const rb_network *net, char *buf, size_t len) {
     return copy_name(rbg::jit_net_source(p, rbg::jit_block()), buf, len);
 }
 
-// The warp kernel's dependency masks for the network, listed: row j of out
-// ([R][32], cap entries in all) holds the number of reactions reaction j's
-// jump touches, then their lane-major positions; 0xFFFF for more than 31.
-// RB_ERR_UNSUPPORTED beyond the masks' reach.
+// The warp kernel's dependency lists for the network: row j of out ([R][32],
+// cap entries in all) holds the number of reactions reaction j's jump touches,
+// then their positions (reaction l*C + i at i*32 + l, C = ceil(R / 32));
+// 0xFFFF for more than 31.  RB_ERR_UNSUPPORTED beyond the lists' reach.
 int rbg_internal_warp_dep_table(const rb_network *net, uint16_t *out, size_t cap) {
     if (!net || !out) return fail(RB_ERR_INVALID, "null argument");
-    std::vector<unsigned char> tab;
-    int bytes = 0;
-    size_t R;
+    std::vector<uint32_t> head;
+    std::vector<uint16_t> list;
     bool ok;
     {
         std::lock_guard<std::mutex> lk(net->net.mu);
-        const rbg::Packed p = net->net.pack();
-        R = (size_t)p.R;
-        ok = rbg::warp_dep_masks(p, tab, bytes);
+        ok = rbg::warp_dep_lists(net->net.pack(), head, list);
     }
-    if (!ok) return fail(RB_ERR_UNSUPPORTED, "network beyond the dependency masks' reach");
+    if (!ok) return fail(RB_ERR_UNSUPPORTED, "network beyond the dependency lists' reach");
+    const size_t R = head.size(), C = (R + 31) / 32;
     if (R * 32 > cap) return fail(RB_ERR_INVALID, "buffer too small");
-    const size_t C = (R + 31) / 32, W = (C + 31) / 32;
+    std::memset(out, 0, 2 * 32 * R);
     for (size_t j = 0; j < R; j++) {
-        size_t n = 0;
-        std::fill(out + 32 * j, out + 32 * (j + 1), (uint16_t)0);
-        for (size_t i = 0; i < C; i++)
-            for (size_t l = 0; l < 32; l++) {
-                const size_t word = (j * W + i / 32) * 32 + l;
-                if (!(tab[word * bytes + (i % 32) / 8] >> (i % 8) & 1)) continue;
-                if (++n <= 31) out[32 * j + n] = (uint16_t)(i * 32 + l);
-            }
+        const size_t n = head[j] & rbg::kDepAll;
         out[32 * j] = n <= 31 ? (uint16_t)n : (uint16_t)0xFFFF;
+        for (size_t k = 0; n <= 31 && k < n; k++) {
+            const size_t r = list[8 * (size_t)(head[j] >> 12) + k];
+            out[32 * j + 1 + k] = (uint16_t)((r % C) * 32 + r / C);
+        }
     }
     return RB_OK;
 }

@@ -114,13 +114,11 @@ DeviceNet::~DeviceNet() {
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-bool warp_dep_masks(const Packed &p, std::vector<unsigned char> &tab, int &word_bytes) {
+bool warp_dep_lists(const Packed &p, std::vector<uint32_t> &head, std::vector<uint16_t> &list) {
     const int R = p.R, P = p.P, Q = p.Q;
-    const int C = (R + 31) / 32, W = (C + 31) / 32;
-    tab.clear();
-    word_bytes = C <= 8 ? 1 : C <= 16 ? 2 : 4;
-    if (R < 1 || C > 256) return false;
-    tab.assign((size_t)R * W * 32 * word_bytes, 0);
+    head.clear();
+    list.clear();
+    if (R < 1 || R > 8160) return false;
     // reactions reading each species
     std::vector<std::vector<int32_t>> readers((size_t)p.S);
     for (int r = 0; r < R; r++)
@@ -129,16 +127,35 @@ bool warp_dep_masks(const Packed &p, std::vector<unsigned char> &tab, int &word_
                 auto &v = readers[(size_t)p.fac_sp[(size_t)r * P + k]];
                 if (v.empty() || v.back() != r) v.push_back(r);
             }
-    for (int j = 0; j < R; j++)
+    std::vector<int32_t> mark((size_t)R, -1);
+    std::vector<uint16_t> row;
+    for (int j = 0; j < R; j++) {
+        row.clear();
         for (int k = 0; k < Q; k++) {
             if (p.jmp_d[(size_t)j * Q + k] == 0) continue;
-            for (int32_t r : readers[(size_t)p.jmp_sp[(size_t)j * Q + k]]) {
-                const int i = r % C;
-                const size_t word = ((size_t)j * W + i / 32) * 32 + r / C;
-                tab[word * word_bytes + (i % 32) / 8] |= (unsigned char)(1u << (i % 8));  // little-endian words
-            }
+            for (int32_t r : readers[(size_t)p.jmp_sp[(size_t)j * Q + k]])
+                if (mark[(size_t)r] != j) {
+                    mark[(size_t)r] = j;
+                    row.push_back((uint16_t)r);
+                }
         }
+        const size_t n = row.size(), start = (list.size() + 7) / 8;
+        if ((n > 31 && 4 * n > 3 * (size_t)R) || n >= kDepAll || 8 * start + n > (1u << 23)) {
+            head.push_back(kDepAll);
+            continue;
+        }
+        head.push_back((uint32_t)start << 12 | (uint32_t)n);
+        list.resize(8 * start);
+        list.insert(list.end(), row.begin(), row.end());
+    }
+    list.resize((list.size() + 15) / 8 * 8);
     return true;
+}
+
+double warp_mean_deps(const Packed &p, const std::vector<uint32_t> &head) {
+    double n = 0;
+    for (uint32_t h : head) n += (h & kDepAll) == kDepAll ? (double)p.R : (double)(h & kDepAll);
+    return head.empty() ? (double)p.R : n / (double)head.size();
 }
 
 bool ensure_device(const Network &net) {
@@ -373,25 +390,36 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
     int block, per_sm;
     size_t smem;
     if (warp) {
-        block = 32 * warp_w;
-        smem = ssa_warp_smem(a, warp_w);
-        per_sm = std::max(1, ssa_warp_occupancy(a, warp_w, smem));
-        const int64_t blocks = std::max<int64_t>(
-            1, std::min<int64_t>((r.n_traj + warp_w - 1) / warp_w, (int64_t)ctx->sm_count * per_sm));
-        // dependency masks: only the propensities a reaction's jump touches
+        // dependency lists: only the propensities a reaction's jump touches
         // are re-evaluated after it fires (RB_WARP_DEPS=0: all, every step)
         if (dn.dep_version != dn.version) {
             if (dn.dep) cudaFree(dn.dep);
             dn.dep = nullptr;
-            std::vector<unsigned char> tab;
-            dn.dep_ok = warp_dep_masks(p, tab, dn.dep_bytes);
-            if (dn.dep_ok && (!cuda_ok(cudaMalloc(&dn.dep, tab.size()), "cudaMalloc(dependency masks)") ||
-                              !cuda_ok(cudaMemcpy(dn.dep, tab.data(), tab.size(), cudaMemcpyHostToDevice),
-                                       "cudaMemcpy(dependency masks)")))
+            std::vector<uint32_t> head;
+            std::vector<uint16_t> list;
+            dn.dep_ok = warp_dep_lists(p, head, list);
+            dn.dep_mean = warp_mean_deps(p, head);
+            if (dn.dep_ok &&
+                (!cuda_ok(cudaMalloc(&dn.dep, 4 * head.size() + 2 * list.size()), "cudaMalloc(dependency lists)") ||
+                 !cuda_ok(cudaMemcpy(dn.dep, head.data(), 4 * head.size(), cudaMemcpyHostToDevice),
+                          "cudaMemcpy(dependency lists)") ||
+                 !cuda_ok(cudaMemcpy(static_cast<unsigned char *>(dn.dep) + 4 * head.size(), list.data(),
+                                     2 * list.size(), cudaMemcpyHostToDevice),
+                          "cudaMemcpy(dependency lists)")))
                 return false;
             dn.dep_version = dn.version;
         }
-        const size_t n_cnt0 = (size_t)blocks * warp_w * std::max(p.S, 1);
+        // one block per SM, no more warps in it than spread the trajectories
+        // over all SMs
+        a.group = ssa_warp_group(a, r.n_traj, dn.dep_mean, ctx->smem_optin, ctx->sm_count);
+        const int side = 32 / a.group;  // trajectories side by side in a warp
+        const int warps = (int)std::max<int64_t>(
+            1, std::min<int64_t>(ssa_warp_warps(a, ctx->smem_optin), ((r.n_traj + side - 1) / side + ctx->sm_count - 1) / ctx->sm_count));
+        block = 32 * warps;
+        smem = ssa_warp_smem(a, warps);
+        const int per_block = warps * side;
+        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((r.n_traj + per_block - 1) / per_block, ctx->sm_count));
+        const size_t n_cnt0 = (size_t)blocks * per_block * std::max(p.S, 1);
         if (dn.warp_cnt0_n < n_cnt0) {
             if (dn.warp_cnt0) {
                 cudaStreamSynchronize(stream);
@@ -405,12 +433,12 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
         a.warp_cnt0 = dn.warp_cnt0;
         const char *wd = std::getenv("RB_WARP_DEPS");
         if (dn.dep_ok && !(wd && std::strcmp(wd, "0") == 0)) {
-            a.dep_tab = dn.dep;
-            a.dep_bytes = dn.dep_bytes;
+            a.dep_head = static_cast<const uint32_t *>(dn.dep);
+            a.dep_list = reinterpret_cast<const uint16_t *>(a.dep_head + p.R);
         }
         if (const char *xc = std::getenv("RB_WARP_EXACT_CHOICE")) a.exact_choice = std::strcmp(xc, "0") != 0;
         if (timed && !cuda_ok(cudaEventRecord(dn.ev_start, stream), "cudaEventRecord")) return false;
-        const int err = launch_ssa_warp(a, warp_w, (int)blocks, smem, stream);
+        const int err = launch_ssa_warp(a, warps, (int)blocks, smem, stream);
         if (err != 0) return cuda_ok((cudaError_t)err, "SSA kernel launch");
         if (timed && !cuda_ok(cudaEventRecord(dn.ev_stop, stream), "cudaEventRecord")) return false;
         if (mapping) *mapping = 5;

@@ -58,8 +58,8 @@ struct DeviceNet {
     double out_gbs = 0;                 // sample bytes / kernel time of the last host-pointer run
     int64_t *warp_cnt0 = nullptr;       // warp kernel interval-start counts
     size_t warp_cnt0_n = 0;             //   (entries)
-    void *dep = nullptr;                // warp kernel dependency masks (SsaArgs::dep_tab)
-    int dep_bytes = 0;                  //   their word size
+    void *dep = nullptr;                // warp kernel dependency list heads, then lists
+    double dep_mean = 0;                //   their mean length
     uint64_t dep_version = 0;           //   for this descriptor version (0: none built)
     bool dep_ok = false;                //   false: the network is beyond the lists' reach
     const void *jit_k = nullptr;        // generated kernel last used, for
@@ -68,10 +68,14 @@ struct DeviceNet {
     ~DeviceNet();
 };
 
-// Dependency masks of the warp kernel for a packed network (layout and word
-// size: SsaArgs::dep_tab).  False for more than 8192 reactions, whose masks
-// would outgrow the caches that serve one row per event.
-bool warp_dep_masks(const Packed &p, std::vector<unsigned char> &tab, int &word_bytes);
+// Dependency lists of the warp kernel for a packed network (SsaArgs::dep_head,
+// dep_list).  A list longer than 31 and than three quarters of the reactions,
+// or that would take the lists past 2^23 entries, is left out (kDepAll).
+// False for networks of more than 8160 reactions: 32 lanes' chunk sums cover
+// no more (SsaArgs has no lists then).
+bool warp_dep_lists(const Packed &p, std::vector<uint32_t> &head, std::vector<uint16_t> &list);
+// Mean number of propensities re-evaluated after a firing.
+double warp_mean_deps(const Packed &p, const std::vector<uint32_t> &head);
 
 // Make net.dev current for the active device and descriptor version.
 // Caller holds net.mu.  Returns false (error set) on failure.

@@ -19,6 +19,7 @@ constexpr int kZigOffK = 2 * kZigTable;
 constexpr int kZigOffD = 2 * kZigTable + kZigLayers;
 constexpr int kZigOffXdf = 2 * kZigTable + 2 * kZigLayers;
 constexpr int kZigWords = 2 * kZigTable + 3 * kZigLayers;
+constexpr uint32_t kDepAll = 0xFFF;  // see SsaArgs::dep_head
 
 struct SsaArgs {
     // packed network (see network.hpp: Packed)
@@ -59,7 +60,8 @@ struct SsaArgs {
     uint64_t *events;        // [n_traj]
 
     // scratch: [0] trajectory ticket, [1] total accepted events,
-    // [2] set to 1 when the time budget ran out, [3] exact interval re-runs
+    // [2] set to 1 when the time budget ran out, [3] exact interval re-runs,
+    // [4] (a batch's persistent launch) thread unit ticket
     unsigned long long *work;
     // Speculative kernels, nullable: [n_samples] per sample row, the number of
     // trajectories whose row of `out` is written and visible device-wide (the
@@ -95,17 +97,17 @@ struct SsaArgs {
     // slots (every trajectory gets the same number of steps).
     int32_t sched;
 
-    // Warp-per-trajectory kernel: dep_tab holds, per reaction j and lane l,
-    // ceil(C / 32) words (C = ceil(R / 32) reactions a lane, words of
-    // dep_bytes bytes: 1 for C <= 8, 2 for C <= 16, else 4) whose bit i is set
-    // when lane l's reaction l*C + i reads a species that j changes:
-    // word w of (j, l) at index (j * ceil(C / 32) + w) * 32 + l, one coalesced
-    // load per step.  After j fires only those are re-evaluated.  Null: every
-    // propensity is re-evaluated at every step.
-    const void *dep_tab;
-    int32_t dep_bytes;
-    // Warp-per-trajectory kernel: [blocks x warps per block][S] counts at the
-    // start of each warp's current sample interval (read only by an exact
+    // Warp kernel: lanes per trajectory (8, 16 or 32).
+    int32_t group;
+    // Warp kernel: the reactions whose propensity reads a species that
+    // reaction j changes are dep_list[8 (dep_head[j] >> 12)] and the
+    // (dep_head[j] & 0xFFF) - 1 after it; the low 12 bits are kDepAll when
+    // there are so many that every propensity is re-evaluated after j fires.
+    // Null dep_list: always.
+    const uint16_t *dep_list;
+    const uint32_t *dep_head;
+    // Warp kernel: [blocks x groups per block][S] counts at the
+    // start of each group's current sample interval (read only by an exact
     // re-run of the interval, so they stay out of shared memory).
     int64_t *warp_cnt0;
     // Warp-per-trajectory kernel: decide every choice with the exact fold, as
@@ -115,19 +117,20 @@ struct SsaArgs {
     // Warp kernel over a batch of networks (batch != null): item k is
     // batch[k], its trajectories are the tickets batch_start[k] ..
     // batch_start[k+1] - 1; the launch's own S, R, P, Q are the largest of the
-    // items'.  An item's lm_* fields point to its lane-major tables (reaction
-    // l*C + i at position i*32 + l, C = ceil(R/32)): float-pair rates,
-    // two-slot shapes (null unless every reaction has order <= 2) and factors
-    // ([C][P][32], species | order << 16).
+    // items'.  An item's lm_rdf are its float-pair rates [R], lm_shape its
+    // two-slot shapes [R] when every reaction has order <= 2 (and S < 32767),
+    // else its factors [R][P] (species | order << 16).
     const SsaArgs *batch;
     const int64_t *batch_start;
     int32_t batch_n;
     const float2 *lm_rdf;
     const uint32_t *lm_shape;
-    const int32_t *lm_fac;
-    // The same launch also runs thread units (batch != null): tickets below
-    // n_warp_tickets are the warp items' trajectories, ticket
-    // n_warp_tickets + u is thread unit u -- up to 32 trajectories of one
+    // An item's jumps [R][Q], species | delta << 16; null when a delta needs
+    // more than 16 bits.
+    const uint32_t *lm_jump;
+    // The same launch also runs thread units (batch != null): n_warp_tickets
+    // are the warp items' trajectories, the other n_traj - n_warp_tickets
+    // tickets (counted in work[4]) are thread units -- up to 32 trajectories of one
     // small-network item, one per lane, each run by the exact per-lane step.
     // Thread item k is tbatch[k]; its units are tbatch_unit[k] ..
     // tbatch_unit[k + 1] - 1, 32 trajectories each (the last one partial);
@@ -170,8 +173,11 @@ int launch_ssa_spec(const SsaArgs &a, int block, int grid, size_t smem, void *st
 // in smem_limit (0: none).
 bool ssa_warp_supported(const SsaArgs &a, int max_order);
 int ssa_warp_warps(const SsaArgs &a, size_t smem_limit);
+// Lanes per trajectory (SsaArgs::group; RB_WARP_GROUP = 8, 16 or 32 overrides)
+// for a launch of n_traj trajectories whose dependency lists hold mean_deps
+// entries on average.
+int ssa_warp_group(const SsaArgs &a, int64_t n_traj, double mean_deps, size_t smem_limit, int sms);
 size_t ssa_warp_smem(const SsaArgs &a, int warps);
-int ssa_warp_occupancy(const SsaArgs &a, int warps, size_t smem);
 int launch_ssa_warp(const SsaArgs &a, int warps, int grid, size_t smem, void *stream);
 // Two-slot shape word of reaction r for the lane-major tables of a batch item.
 uint32_t warp_shape_word(const int32_t *fac_sp, const int32_t *fac_ord, int P, int S, int r);

@@ -1,26 +1,31 @@
-// Warp-per-trajectory SSA kernel for large networks (hundreds of species,
-// thousands of reactions), where one trajectory's propensity pass is itself
-// data-parallel work.
+// SSA kernel for networks beyond the thread-per-trajectory kernels (dozens of
+// species, up to thousands of reactions): a group of G = 8, 16 or 32 lanes runs
+// one trajectory, whose propensity pass is itself data-parallel work, so a warp
+// runs 4, 2 or 1 of them side by side.
 //
 // Each step of rebop's direct method (gillespie.rs:315-344) recomputes every
 // propensity and folds them left to right into cumulative sums
-// (make_cumrates, gillespie.rs:357-364).  Here the 32 lanes of a warp own
+// (make_cumrates, gillespie.rs:357-364).  Here the lanes of a group own
 // contiguous chunks of the reaction list and keep every propensity as a 64-bit
-// fixed-point number (units of 2^-E, E chosen per trajectory so that the total
-// fills 52 to 60 bits).  Integer sums are exact and associative, so
-//   * after a reaction fires each lane re-evaluates only those of its own
-//     reactions that read a changed species (a bit mask per reaction and
-//     lane, SsaArgs::dep_tab) and adds the differences to its chunk sum: no
-//     re-summation, no drift, nothing handed between lanes;
+// fixed-point number, scaled per trajectory so that the total fills 46 to 51
+// bits.  Integer sums are exact and associative, so
+//   * after a reaction fires only the propensities that read a species it
+//     changed are re-evaluated (SsaArgs::dep_list), spread evenly over the
+//     lanes, and their differences added to the chunk sums that hold them
+//     (shared-memory adds): no re-summation and no drift;
 //   * one shuffle scan of the chunk sums (two adds a step) gives every
 //     chunk's prefix and the total, a second one over the chunk that holds
 //     total * U the chosen reaction.
 // The clock is a 64-bit fixed-point number too, counted from the interval's
-// start in units of 2^-58 of the interval.  The random words are generated
-// ahead, 32 at a time, one kept per lane: the lanes then turn all 32 into
-// Exp1 candidates at once, and a step picks up the two words it consumes with
-// shuffles.  The clock arithmetic runs on every lane alike, so no decision has
-// to be handed around.
+// start in units of 2^-50 of the interval.  Draws and clock arithmetic run on
+// every lane of a group alike, so no decision has to be handed around.
+//
+// The groups of a warp run in lockstep: one pass of the loop is one step of
+// each of them, with full-warp shuffles and votes, so the serial part of a step
+// -- draws, clock, scans -- is issued once for all.  What only some groups need
+// in a pass (a sample to record, a new trajectory, a new scale, an exact
+// re-run) is done by those before the next pass, on their own lanes; a group
+// without work goes along without committing anything.
 //
 // The reference's sums are a sequential binary64 fold, within (R + M + 2)
 // 2^-53 of the exact sums; a fixed-point propensity is within (M + 1) 2^-44 of
@@ -34,13 +39,17 @@
 // draws in native binary64, so counts, event numbers and the random stream
 // equal rebop's bit for bit.
 //
-// Bound: instruction issue and, at 16 warps per SM, the dependent chain of a
-// step: 618 warp instructions per event at 60 % issue on 200 species and 1000
-// reactions (1 216 at 71 % with float-pair sums), 10 000 trajectories of 6.0e4
-// events each in 569 ms.
+// Bound: the dependent chain of a step (about 1 us alone: two scans, the
+// clock's conversions and division, the shared-memory round trips of the jump
+// and the re-evaluation), which 16 warps per SM hide until issue takes over
+// (63 % of cycles).  10 000 trajectories of 200 species and 1000 reactions,
+// 6.0e4 events each: 400 ms (float-pair sums 950 ms); 9 728 of 40 x 120: 10.9
+// ms, 5.0e9 events/s, on 8 lanes each.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
+#include <cstdlib>
 
 #include "ssa_spec_body.cuh"
 
@@ -53,82 +62,134 @@ constexpr int kWarpMaxWarps = 16;
 constexpr int kWarpMaxWarpsBatch = 24;
 
 struct WarpLayout {
-    size_t block_bytes, warp_bytes;
+    size_t block_bytes, group_bytes, warp_bytes;
 };
 
-// Lane l owns the C = ceil(R / 32) reactions l*C .. l*C + C - 1.  Arrays the
-// lanes walk together are stored lane-major -- reaction l*C + i at position
-// i*32 + l -- so one step of the walk touches 32 consecutive words.
-__host__ __device__ inline int warp_chunk(int R) { return (R + 31) / 32; }
+// Lane l of a group owns the C = ceil(R / G) reactions l*C .. l*C + C - 1.
+__host__ __device__ inline int warp_chunk(int R, int G) { return (R + G - 1) / G; }
 
 // Every reaction of order <= 2 over fewer than 32767 species: propensities
 // come from two-slot shapes (shape_word) and the factor list is not needed.
 __host__ __device__ inline bool warp_shape2(const SsaArgs &a) { return a.max_mults <= 2 && a.S < 32767; }
 
 // Shared memory: block tables (Exp1 tables, float-pair rates when shared,
-// shapes or factors, jumps), then per warp: the generator at the word buffer's
-// start and at the interval's, counts, fixed-point propensities (and
-// float-pair rates when per trajectory).  The counts at the interval start go
-// to global memory (SsaArgs::warp_cnt0).
-constexpr size_t kWarpState = 96;  // generator states: buffer start, before its last word, interval start
-__host__ __device__ inline WarpLayout warp_layout(const SsaArgs &a) {
+// shapes or factors, jumps, dependency list heads), then per group: where its
+// trajectory stands, chunk sums, counts, fixed-point propensities (and float-pair rates
+// when per trajectory).  The counts at the interval start go to global memory
+// (SsaArgs::warp_cnt0).
+struct GroupNet {  // the network of a group's trajectory
+    const float2 *rdf;          // float-pair rates [R]
+    const uint32_t *shape;      // two-slot shapes [R], or factors [R][P]
+    const uint32_t *jump;       // [R][Q] species | delta << 16; null: from the descriptor
+    const uint16_t *dep_list;
+    const uint32_t *dep_head;
+    const int32_t *jmp_sp;
+    const int64_t *jmp_d;
+    int R, C, E, P, Q;          // E: reactions a lane takes in the walk through a chunk
+    uint32_t c_inv;             // r / C = hi32(r c_inv), r < 65536
+    int sh_q, sh_p;             // error bounds, see group_net
+    bool use_shape;
+};
+struct GroupRun {  // where a group's trajectory stands
+    uint64_t g0[4];             // generator at the interval's start
+    double T, t0;               // the interval
+    long long traj, i;          // trajectory, sample index
+    unsigned long long ev;      // events up to the interval's start
+    const SsaArgs *it;
+    const double *sample_t;     // of *it:
+    const int32_t *save_idx;
+    int64_t *out;               //   where sample i goes
+    long long n_traj;
+    int n_save, S;
+    GroupNet net;               // (batch)
+};
+constexpr size_t kGroupState = (sizeof(GroupRun) + 15) & ~(size_t)15;
+__host__ __device__ inline WarpLayout warp_layout(const SsaArgs &a, int G) {
     WarpLayout l;
-    const size_t RP = 32 * (size_t)warp_chunk(a.R);     // lane-major positions
+    const size_t RP = (size_t)G * warp_chunk(a.R, G);
     size_t b = 16 * 256 + 8 * 257 + 8 * 256 + 8 * 256;  // zxk, zf, zd, xdf
     if (!a.batch) {  // a batch's networks stay in global memory
-        b += 8 * RP;                                        // shared float-pair rates (lane-major)
-        if (!warp_shape2(a)) b += 4 * RP * a.P;             // factors (lane-major), when shapes do not cover
-        b += 4 * RP;                                        // two-slot reaction shapes (lane-major)
+        b += 8 * (size_t)a.R;                               // shared float-pair rates
+        b += 4 * (size_t)a.R * (warp_shape2(a) ? 1 : a.P);  // two-slot shapes, or factors
         b += 4 * (size_t)a.R * a.Q;                         // jumps: species, delta (16 bit each)
+        b += 4 * (size_t)a.R;                               // dependency list heads
     }
     l.block_bytes = (b + 15) & ~(size_t)15;
-    size_t w = kWarpState + 8 * (size_t)a.S;            // generator states, counts
+    size_t w = kGroupState + 8 * (size_t)G;             // the trajectory's state, chunk sums
+    w += 8 * (size_t)a.S;                               // counts
+    w += 8 * RP;                                        // propensities
+    if (a.rate_stride) w += 8 * (size_t)a.R;            // per-trajectory float-pair rates
     w += 4 * ((size_t)a.S + 1);                         // counts as floats, plus the constant 1
-    w += 8 * RP + 8;                                    // propensities (lane-major), alignment
-    if (a.rate_stride) w += 8 * RP;                     // per-trajectory float-pair rates
+    l.group_bytes = (w + 15) & ~(size_t)15;
+    l.warp_bytes = l.group_bytes * (32 / G);
     const size_t wt = 8 * 32 * (2 * (size_t)a.tbatch_S + 4);  // a thread unit's counts, their copy, generator
-    if (a.batch && wt > w) w = wt;
-    l.warp_bytes = (w + 15) & ~(size_t)15;
+    if (a.batch && wt > l.warp_bytes) l.warp_bytes = wt;
     return l;
 }
 
-// Physical slot of the propensity at lane-major position pos
-// (reaction l*C + i at i*32 + l): the lane bits are XORed with the row, so a
-// row read by the 32 lanes (the chunk sums) and a column read by the 32 lanes
-// (the walk through one lane's chunk to the chosen reaction) both touch 32
-// distinct banks.  Without it every lane of the walk hit the same bank.
-__device__ __forceinline__ int pz(int pos) { return pos ^ ((pos >> 5) & 31); }
-
-__device__ __forceinline__ int64_t shfl_i64(int64_t v, int src) {
-    return (int64_t)__shfl_sync(0xffffffffu, (long long)v, src);
-}
-
-// Inclusive sum over the lanes of a warp, over the nearest 2 * last lanes
-// (16: all 32): the shuffle's own range predicate guards the two adds.
-template <int D>
-__device__ __forceinline__ void scan_step(int64_t &v) {
-    asm volatile(
-        "{\n .reg .u32 lo, hi, rl, rh;\n .reg .pred p;\n mov.b64 {lo, hi}, %0;\n"
-        " shfl.sync.up.b32 rl|p, lo, %1, 0, 0xffffffff;\n shfl.sync.up.b32 rh, hi, %1, 0, 0xffffffff;\n"
-        " @p add.cc.u32 lo, lo, rl;\n @p addc.u32 hi, hi, rh;\n mov.b64 %0, {lo, hi};\n}\n"
-        : "+l"(v)
-        : "n"(D));
-}
-__device__ __forceinline__ int64_t scan_i64(int64_t v, int width) {
-    scan_step<1>(v);
-    if (width > 2) scan_step<2>(v);
-    if (width > 4) scan_step<4>(v);
-    if (width > 8) scan_step<8>(v);
-    if (width > 16) scan_step<16>(v);
-    return v;
-}
+// A group of G lanes of the warp.  `mask` is the lanes that take part in its
+// shuffles and votes: the group's own, or the whole warp's where all groups run
+// together (each still sees its own lanes only).
+template <int G>
+struct Group {
+    static constexpr uint32_t kAll = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+    int gl, first;
+    uint32_t mask;
+    __device__ __forceinline__ explicit Group(bool whole_warp) {
+        const int lane = threadIdx.x & 31;
+        gl = lane & (G - 1);
+        first = lane & ~(G - 1);
+        mask = whole_warp ? 0xffffffffu : kAll << first;
+    }
+    __device__ __forceinline__ uint32_t ballot(bool v) const {
+        return G == 32 ? __ballot_sync(mask, v) : __ballot_sync(mask, v) >> first & kAll;
+    }
+    __device__ __forceinline__ bool any(bool v) const { return ballot(v) != 0; }
+    __device__ __forceinline__ void sync() const { __syncwarp(mask); }
+    __device__ __forceinline__ int get(int v, int src) const { return __shfl_sync(mask, v, src, G); }
+    __device__ __forceinline__ int64_t get(int64_t v, int src) const {
+        return (int64_t)__shfl_sync(mask, (long long)v, src, G);
+    }
+    __device__ __forceinline__ double get(double v, int src) const {
+        return __longlong_as_double(__shfl_sync(mask, __double_as_longlong(v), src, G));
+    }
+    __device__ __forceinline__ float sum(float v) const {
+#pragma unroll
+        for (int d = G / 2; d > 0; d >>= 1) v = __fadd_rn(v, __shfl_xor_sync(mask, v, d, G));
+        return v;
+    }
+    __device__ __forceinline__ int sum(int v) const {
+#pragma unroll
+        for (int d = G / 2; d > 0; d >>= 1) v += __shfl_xor_sync(mask, v, d, G);
+        return v;
+    }
+    // One step of an inclusive sum over the group's lanes: the shuffle's own
+    // range predicate guards the two adds.
+    template <int D>
+    __device__ __forceinline__ void scan_step(int64_t &v) const {
+        asm volatile(
+            "{\n .reg .u32 lo, hi, rl, rh;\n .reg .pred p;\n mov.b64 {lo, hi}, %0;\n"
+            " shfl.sync.up.b32 rl|p, lo, %1, %2, %3;\n shfl.sync.up.b32 rh, hi, %1, %2, %3;\n"
+            " @p add.cc.u32 lo, lo, rl;\n @p addc.u32 hi, hi, rh;\n mov.b64 %0, {lo, hi};\n}\n"
+            : "+l"(v)
+            : "n"(D), "n"((32 - G) << 8), "r"(mask));
+    }
+    // Inclusive sum over the group's lanes up to this one.
+    __device__ __forceinline__ int64_t scan(int64_t v) const {
+        scan_step<1>(v);
+        scan_step<2>(v);
+        scan_step<4>(v);
+        if (G > 8) scan_step<8>(v);
+        if (G > 16) scan_step<16>(v);
+        return v;
+    }
+};
 
 // The warp kernel's fixed-point numbers have 22 fraction bits below the part a
 // 32-bit conversion reaches: v = floor(a) 2^22 + the rest.  64-bit conversions
 // from and to float run on the FP64 pipe here and kept it 67 % busy; the
 // 32-bit ones do not.
 constexpr int kFxLow = 22;
-constexpr int kFxLim = 52;  // single values stay below 2^52: a below 2^30
 
 // round((h + l) 2^22) within one unit (and 2^-47 of the value) for a float pair
 // with 0 <= h < 2^31, |l| <= 2^-20 h; l22 = 2^22 l.
@@ -163,21 +224,16 @@ __device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t
 __device__ __forceinline__ int ilog2f(float v) { return (int)(__float_as_uint(v) >> 23) - 127; }
 __device__ __forceinline__ int ilog2d(double v) { return (int)((uint64_t)__double_as_longlong(v) >> 52) - 1023; }
 
-__device__ __forceinline__ double shfl_d(double v, int src) {
-    return __longlong_as_double(__shfl_sync(0xffffffffu, __double_as_longlong(v), src));
-}
-
 // Exact binary64 propensity of reaction r in the reference's multiply order:
 // Rate::rate's fold (gillespie.rs:71-90), or the macro's integer falling
 // factorials (gillespie_macro.rs:133-146).
-template <bool MACRO>
 __device__ __forceinline__ double exact_propensity(const SsaArgs &it, const int64_t *cnt, double rate, int r) {
     double acc = rate;
     for (int p = 0; p < it.P; ++p) {
         const int o = it.fac_ord[r * it.P + p];
         if (o == 0) continue;
         const int64_t n = cnt[it.fac_sp[r * it.P + p]];
-        if (MACRO) {
+        if (it.macro_mode) {
             int64_t ff = n;
             for (int j = 1; j < o; ++j) ff *= n - j;
             acc = __dmul_rn(acc, (double)ff);
@@ -188,35 +244,34 @@ __device__ __forceinline__ double exact_propensity(const SsaArgs &it, const int6
     return acc;
 }
 
-// Exact binary64 propensities and their running sums, in scr: this warp's
-// shared-memory scratch of 32 * ceil(R / 32) doubles, lane-major like the
-// chunks.  Lane l evaluates and folds its own reactions l*C .. l*C + C - 1, in
-// order, starting from the running sum lane l - 1 hands over, so the sums are
-// the reference's sequential fold (make_cumrates, gillespie.rs:357-364) while
-// every lane reads only its own column.  Returns the total on every lane.
-template <bool MACRO>
-__device__ __forceinline__ double warp_exact_fold(const SsaArgs &it, const int64_t *cnt, const double *rates,
-                                                  double *scr) {
-    const int lane = threadIdx.x & 31, R = it.R, C = warp_chunk(R);
-    const int r_lo = min(R, lane * C), n_own = min(R, r_lo + C) - r_lo;
-    for (int i = 0; i < n_own; ++i) scr[i * 32 + lane] = exact_propensity<MACRO>(it, cnt, rates[r_lo + i], r_lo + i);
+// Exact binary64 propensities and their running sums, in scr: this group's
+// shared-memory scratch of R doubles.  Lane l evaluates and folds its own
+// reactions l*C .. l*C + C - 1, in order, starting from the running sum lane
+// l - 1 hands over, so the sums are the reference's sequential fold
+// (make_cumrates, gillespie.rs:357-364).  Returns the total on every lane.
+template <int G>
+__device__ __forceinline__ double warp_exact_fold(const SsaArgs &it, const Group<G> &gr, const int64_t *cnt,
+                                                  const double *rates, double *scr) {
+    const int R = it.R, C = warp_chunk(R, G);
+    const int r_lo = min(R, gr.gl * C), n_own = min(R, r_lo + C) - r_lo;
+    for (int i = 0; i < n_own; ++i) scr[r_lo + i] = exact_propensity(it, cnt, rates[r_lo + i], r_lo + i);
     // one lane's chunk after the other; loads go ahead in blocks of 8
     double run = 0.0;
-    for (int l = 0; l < 32; ++l) {
-        if (lane == l) {
+    for (int l = 0; l < G; ++l) {
+        if (gr.gl == l) {
             for (int i0 = 0; i0 < n_own; i0 += 8) {
                 double v[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] = i0 + j < n_own ? scr[(i0 + j) * 32 + lane] : 0.0;
+                for (int j = 0; j < 8; ++j) v[j] = i0 + j < n_own ? scr[r_lo + i0 + j] : 0.0;
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
                     if (i0 + j < n_own) {
                         run = __dadd_rn(run, v[j]);
-                        scr[(i0 + j) * 32 + lane] = run;
+                        scr[r_lo + i0 + j] = run;
                     }
             }
         }
-        run = shfl_d(run, l);
+        run = gr.get(run, l);
     }
     return run;
 }
@@ -224,37 +279,36 @@ __device__ __forceinline__ double warp_exact_fold(const SsaArgs &it, const int64
 // The reaction the reference picks for `chosen` from the running sums in scr:
 // #{r : cum_r < chosen} (gillespie.rs:402-407), or for define_system! the
 // first r with chosen < cum_r (gillespie_macro.rs:150-171); R if none.
-template <bool MACRO>
-__device__ __forceinline__ int warp_exact_pick(const SsaArgs &it, const double *scr, double chosen) {
-    const int lane = threadIdx.x & 31, R = it.R, C = warp_chunk(R);
-    const int r_lo = min(R, lane * C), n_own = min(R, r_lo + C) - r_lo;
-    if (MACRO) {
+template <int G>
+__device__ __forceinline__ int warp_exact_pick(const SsaArgs &it, const Group<G> &gr, const double *scr,
+                                               double chosen) {
+    const int R = it.R, C = warp_chunk(R, G);
+    const int r_lo = min(R, gr.gl * C), n_own = min(R, r_lo + C) - r_lo;
+    if (it.macro_mode) {
         int first = n_own;
         for (int i = n_own - 1; i >= 0; --i)
-            if (chosen < scr[i * 32 + lane]) first = i;
-        const unsigned int has = __ballot_sync(0xffffffffu, first < n_own);
+            if (chosen < scr[r_lo + i]) first = i;
+        const uint32_t has = gr.ballot(first < n_own);
         if (!has) return R;
         const int l = __ffs((int)has) - 1;
-        return l * C + __shfl_sync(0xffffffffu, first, l);
+        return l * C + gr.get(first, l);
     }
     int c = 0;
-    for (int i = 0; i < n_own; ++i) c += scr[i * 32 + lane] < chosen ? 1 : 0;
-    for (int off = 16; off > 0; off >>= 1) c += __shfl_xor_sync(0xffffffffu, c, off);
-    return c;
+    for (int i = 0; i < n_own; ++i) c += scr[r_lo + i] < chosen ? 1 : 0;
+    return gr.sum(c);
 }
 
-// One exact step of the whole warp from the committed state (lane 0 holds the
-// generator).  Returns 1 when a reaction fires (its index in idx, the clock in
-// t), 0 when the step records the sample.
-template <bool MACRO>
-__device__ __noinline__ int warp_exact_step(const SsaArgs &it, const int64_t *cnt, const double *rates,
-                                            const double *zig, double *scr, Xoshiro &g, double &t, double T,
-                                            int &idx) {
-    const int lane = threadIdx.x & 31;
-    const double total = warp_exact_fold<MACRO>(it, cnt, rates, scr);
+// One exact step of the whole group from the committed state (its first lane
+// holds the generator).  Returns 1 when a reaction fires (its index in idx, the
+// clock in t), 0 when the step records the sample.
+template <int G>
+__device__ __noinline__ int warp_exact_step(const SsaArgs &it, const Group<G> &gr, const int64_t *cnt,
+                                            const double *rates, const double *zig, double *scr, Xoshiro &g, double &t,
+                                            double T, int &idx) {
+    const double total = warp_exact_fold<G>(it, gr, cnt, rates, scr);
     int fire = 0;
     double chosen = 0.0;
-    if (lane == 0 && 0.0 < total) {
+    if (gr.gl == 0 && 0.0 < total) {
         const double tn = __dadd_rn(t, __ddiv_rn(xo_exp1(g, zig, zig + kZigOffF), total));
         if (!(tn > T)) {
             fire = 1;
@@ -262,23 +316,23 @@ __device__ __noinline__ int warp_exact_step(const SsaArgs &it, const int64_t *cn
             chosen = __dmul_rn(total, xo_uniform(g));
         }
     }
-    fire = __shfl_sync(0xffffffffu, fire, 0);
-    t = shfl_d(t, 0);
+    fire = gr.get(fire, 0);
+    t = gr.get(t, 0);
     if (!fire) return 0;
-    idx = warp_exact_pick<MACRO>(it, scr, shfl_d(chosen, 0));
+    idx = warp_exact_pick<G>(it, gr, scr, gr.get(chosen, 0));
     return 1;
 }
 
-// The exact choice alone, for a step whose clock the float pairs decided
-// (the reaction fires) but whose choice they left close: the reference's
-// total, chosen = total * U for the uniform's top 53 bits u53, and the pick.
+// The exact choice alone, for a step whose clock the fixed point decided (the
+// reaction fires) but whose choice it left close: the reference's total,
+// chosen = total * U for the uniform's top 53 bits u53, and the pick.
 // Overwrites scr.
-template <bool MACRO>
-__device__ __noinline__ int warp_exact_choice(const SsaArgs &it, const int64_t *cnt, const double *rates,
-                                              double *scr, uint64_t u53) {
-    const double total = warp_exact_fold<MACRO>(it, cnt, rates, scr);
+template <int G>
+__device__ __noinline__ int warp_exact_choice(const SsaArgs &it, const Group<G> &gr, const int64_t *cnt,
+                                              const double *rates, double *scr, uint64_t u53) {
+    const double total = warp_exact_fold<G>(it, gr, cnt, rates, scr);
     const double chosen = __dmul_rn(total, __dmul_rn((double)u53, 0x1.0p-53));
-    return warp_exact_pick<MACRO>(it, scr, chosen);
+    return warp_exact_pick<G>(it, gr, scr, chosen);
 }
 
 // Two-slot shape of reaction r (reactant order <= 2): slots (species, offset)
@@ -311,6 +365,17 @@ __device__ __forceinline__ DF exp1_df_rel(Xoshiro &g, const ExactTables &ex, con
         if (i == 0) return df_from_double(__dsub_rn(kZigR, log(xo_uniform(g))));
         if (wedge_df(ex, i, k, x.h, xo_next(g) >> 11)) return x;
     }
+}
+
+// The draw whose first candidate (draw b, float pair x) failed the fast test
+// when the next draw b2 is already taken: b2 is the wedge's or the tail's
+// uniform.
+__device__ __noinline__ DF exp1_df_rel_cont(Xoshiro &g, uint64_t b, uint64_t b2, DF x, const ExactTables &ex,
+                                            const float2 *xdf) {
+    const int i = (int)(b & 0xff);
+    if (i == 0) return df_from_double(__dsub_rn(kZigR, log(uniform53(b2))));
+    if (wedge_df(ex, i, b >> 12, x.h, b2 >> 11)) return x;
+    return exp1_df_rel(g, ex, xdf);
 }
 
 // One thread unit of a persistent batch: lane l runs trajectory first + l of
@@ -459,29 +524,81 @@ __device__ __noinline__ unsigned long long thread_unit(const SsaArgs &it, const 
     return ev;
 }
 
+// The fields of a group's network that follow from its item.
+template <int G>
+__device__ __forceinline__ void group_net(GroupNet &n, const SsaArgs &it) {
+    n.R = it.R;
+    n.P = it.P;
+    n.Q = it.Q;
+    n.C = warp_chunk(it.R, G);
+    n.E = (n.C + G - 1) / G;
+    n.c_inv = n.C > 1 ? 0xFFFFFFFFu / (uint32_t)n.C + 1u : 0u;
+    n.use_shape = warp_shape2(it);
+    n.dep_list = it.dep_list;
+    n.dep_head = it.dep_head;
+    n.jmp_sp = it.jmp_sp;
+    n.jmp_d = it.jmp_d;
+    // Fixed point: the total is scaled to 2^49 .. 2^50 and scaled anew when it
+    // falls below 2^46 or reaches 2^51, or when the propensities one lane
+    // re-evaluates in a step add up to 1.9 2^50; below that no chunk sum
+    // reaches 2^56 (2^51 + 32 * 1.9 2^50), where its two words wrap.
+    // Relative error bound of a propensity or sum against the reference's
+    // binary64 one, apart from one unit per propensity:
+    const int mm = n.use_shape ? 2 : it.max_mults;  // multiplies per propensity
+    const float c_p = (float)(mm + 2) * kGamma + (float)(it.R + mm + 4) * 0x1p-53f;
+    // Exp1 / total: the total's bound (its units at the smallest total), the
+    // Exp1 pair, the total's pair and the division
+    const float c_q = (c_p + (float)(it.R + 2) * 0x1p-46f + 9.0f * kGamma) * 1.001f;
+    n.sh_q = -ilog2f(c_q) - 1;         // 2^-sh_q >= c_q
+    n.sh_p = -ilog2f(2.0f * c_p) - 1;  // choice: both operands' bounds
+}
+
+// Clock of the interval (t0, T]: units of 2^-et = 1 / etf, in which the interval
+// (the sample time itself when it is empty or lies behind t0) fills 2^50 ..
+// 2^51.  err_step is what a step adds to the clock's error bound beside the
+// quotient's: the reference's rounding (2^-52 T), the conversions' units.
+// False if it has to run exactly.
+__device__ __noinline__ bool interval_clock(double T, double t0, float &etf, int64_t &D, int64_t &err_step) {
+    if (!(T < 0x1p60) || (T != 0.0 && !(T >= 0x1p-60))) return false;
+    const double len = __dsub_rn(T, t0);
+    const double base = len > 0.0 ? len : (T > 0.0 ? T : 1.0);
+    if (!(base >= 0x1p-60) || !(fabs(len) <= base * 0x1p2)) return false;
+    const int et = 50 - ilog2d(base);
+    const double ets = __longlong_as_double((long long)(1023 + et) << 52);
+    etf = pow2f(et);
+    D = __double2ll_rn(__dmul_rn(len, ets));
+    err_step = __double2ll_ru(__dmul_ru(__dmul_ru(T, 0x1p-52), ets)) + 4;
+    return true;
+}
+
+// What a group does before the next pass of the loop.
+enum { kRunning = 0, kRecord, kTake, kBegin, kFull, kExact };
+
 // BATCH: the launch runs a.batch's networks (each item's tables in global
-// memory, lane-major) and a.tbatch's thread units; otherwise the one network
-// of `a`, whose tables the block copies to shared memory.
-template <bool MACRO, bool BATCH>
+// memory), then a.tbatch's thread units in the arithmetic a.macro_mode;
+// otherwise the one network of `a`, whose tables the block copies to shared
+// memory.
+template <bool BATCH, int G>
 __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWarps), 1)
     ssa_warp_kernel(const __grid_constant__ SsaArgs a) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-    const WarpLayout L = warp_layout(a);  // sized for the largest network of the launch
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const Group<G> gr(false), al(true);
+    const int gl = gr.gl;
+    const WarpLayout L = warp_layout(a, G);  // sized for the largest network of the launch
 
     // ---- block tables: Exp1 tables; in single-network mode also the
-    // network's lane-major rates, factors, shapes and its jumps
+    // network's rates, shapes or factors, jumps and dependency list heads
     ulonglong2 *zxk = reinterpret_cast<ulonglong2 *>(g_spec_smem);
     uint64_t *zf = reinterpret_cast<uint64_t *>(zxk + 256);
     uint64_t *zd = zf + 257;
     float2 *xdf = reinterpret_cast<float2 *>(zd + 256);
     float2 *rdf_sh = xdf + 256;
-    const int C0 = warp_chunk(a.R), RP0 = 32 * C0;
     const bool shape2 = warp_shape2(a);
-    int32_t *facl_sh = reinterpret_cast<int32_t *>(rdf_sh + RP0);  // absent (size 0) when shape2
-    uint32_t *shape_sh = reinterpret_cast<uint32_t *>(facl_sh + (shape2 ? 0 : (size_t)RP0 * a.P));
+    uint32_t *shape_sh = reinterpret_cast<uint32_t *>(rdf_sh + a.R);  // or the factors [R][P]
     // jumps of the one network: species as 16-bit indices (S < 65536) below
     // deltas of 16 bits when every one fits (else read from the descriptor)
-    uint32_t *jump_sh = shape_sh + RP0;
+    uint32_t *jump_sh = shape_sh + (size_t)a.R * (shape2 ? 1 : a.P);
+    uint32_t *dep_sh = jump_sh + (size_t)a.R * a.Q;
     for (int k = tid; k < 256; k += blockDim.x) {
         zxk[k] = make_ulonglong2((uint64_t)__double_as_longlong(a.zig[k]),
                                  (uint64_t)__double_as_longlong(a.zig[kZigOffK + k]));
@@ -495,19 +612,16 @@ __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWar
             jump_sh[k] = (uint32_t)a.jmp_sp[k] | ((uint32_t)(uint16_t)dlt << 16);
             jd_wide |= dlt != (int64_t)(int16_t)dlt;
         }
-        for (int q = tid; q < RP0; q += blockDim.x) {
-            const int i = q >> 5, l = q & 31, r = l * C0 + i;
+        for (int r = tid; r < a.R; r += blockDim.x) {
             if (!a.rate_stride) {
-                const DF d = r < a.R ? df_from_double(a.rate[r]) : DF{0.f, 0.f};
-                rdf_sh[q] = make_float2(d.h, d.l);
+                const DF d = df_from_double(a.rate[r]);
+                rdf_sh[r] = make_float2(d.h, d.l);
             }
-            if (shape2) {
-                shape_sh[q] = r < a.R ? shape_word(a.fac_sp, a.fac_ord, a.P, a.S, r) : (uint32_t)a.S << 16 | a.S;
-            } else {
+            if (shape2) shape_sh[r] = shape_word(a.fac_sp, a.fac_ord, a.P, a.S, r);
+            else
                 for (int p = 0; p < a.P; ++p)
-                    facl_sh[(i * a.P + p) * 32 + l] =
-                        r < a.R ? (a.fac_sp[r * a.P + p] | (a.fac_ord[r * a.P + p] << 16)) : 0;
-            }
+                    shape_sh[r * a.P + p] = (uint32_t)(a.fac_sp[r * a.P + p] | (a.fac_ord[r * a.P + p] << 16));
+            dep_sh[r] = a.dep_list ? a.dep_head[r] : kDepAll;
         }
     }
     for (int k = tid; k < 256; k += blockDim.x) {
@@ -518,29 +632,481 @@ __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWar
     // the Exp1 draws use the ziggurat tables only
     const ExactTables ex{zxk, zf, zd, nullptr, nullptr, nullptr};
 
-    // ---- this warp's region (sized for the largest network)
+    // ---- this group's region (sized for the largest network)
     unsigned char *wbase = g_spec_smem + L.block_bytes + (size_t)warp * L.warp_bytes;
-    uint64_t *gst = reinterpret_cast<uint64_t *>(wbase);  // [12]: buffer start, before its last word, interval start
-    int64_t *cnt = reinterpret_cast<int64_t *>(wbase + kWarpState);
-    int64_t *cnt0 = a.warp_cnt0 + ((size_t)blockIdx.x * nw + warp) * (size_t)a.S;  // global
-    float *cntf = reinterpret_cast<float *>(cnt + a.S);  // [S + 1]
-    int64_t *prop = reinterpret_cast<int64_t *>((reinterpret_cast<uintptr_t>(cntf + a.S + 1) + 7) & ~(uintptr_t)7);
-    float2 *rdf_w = reinterpret_cast<float2 *>(prop + RP0);  // per-trajectory float-pair rates (single-network mode)
-    // exact steps use the propensity array as their scratch (32 * C doubles)
+    unsigned char *gbase = wbase + (size_t)(lane / G) * L.group_bytes;
+    GroupRun &gs = *reinterpret_cast<GroupRun *>(gbase);
+    uint2 *csum = reinterpret_cast<uint2 *>(gbase + kGroupState);  // [G] chunk sums: low 24 bits' sum, the rest's
+    int64_t *cnt = reinterpret_cast<int64_t *>(csum + G);
+    int64_t *prop = cnt + a.S;
+    float2 *rdf_w = reinterpret_cast<float2 *>(prop + (size_t)G * warp_chunk(a.R, G));  // per-trajectory rates
+    float *cntf = reinterpret_cast<float *>(rdf_w + (a.rate_stride ? a.R : 0));         // [S + 1]
+    int64_t *cnt0 = a.warp_cnt0 + ((size_t)blockIdx.x * (blockDim.x / G) + tid / G) * (size_t)a.S;  // global
+    // exact steps use the propensity array as their scratch
     double *scr = reinterpret_cast<double *>(prop);
+    GroupNet one;
+    if (!BATCH) {
+        group_net<G>(one, a);
+        one.rdf = a.rate_stride ? rdf_w : rdf_sh;
+        one.shape = shape_sh;
+        one.jump = jd_wide ? nullptr : jump_sh;
+        one.dep_head = dep_sh;
+    } else if (gl == 0) {
+        gs.net = GroupNet{};
+    }
+    const GroupNet &n = BATCH ? gs.net : one;
+    __syncwarp();
+
+    // fixed-point propensity of reaction r, sc times its value in units of
+    // 2^-22; mx collects the largest count it read (as float bits: a count
+    // outside [0, 2^23) has bits >= 0x4B000000), hsum the sum of sc * propensity
+    auto eval_prop = [&](int r, float sc, uint32_t &mx, float &hsum) -> int64_t {
+        const float2 k = n.rdf[r];
+        DF acc{k.x, k.y};
+        if (n.use_shape) {
+            const uint32_t w = n.shape[r];  // the first slot's offset is 0
+            const float n1 = cntf[w & 0x7FFFu], n2 = cntf[(w >> 16) & 0x7FFFu];
+            mx = max(mx, max(__float_as_uint(n1), __float_as_uint(n2)));
+            acc = df_mul_fu(df_mul_fu(acc, n1), fmaxf(__fsub_rn(n2, (float)(w >> 31)), 0.0f));
+        } else {
+            for (int p = 0; p < n.P; ++p) {
+                const uint32_t f = n.shape[r * n.P + p];
+                const int o = (int)(f >> 16);
+                if (o == 0) continue;
+                const float c = cntf[f & 0xFFFFu];
+                mx = max(mx, __float_as_uint(c));
+                for (int j = 0; j < o; ++j) acc = df_mul_fu(acc, fmaxf(__fsub_rn(c, (float)j), 0.0f));
+                acc = fast2sum(acc.h, acc.l);
+            }
+        }
+        const float hs = __fmul_rn(acc.h, sc);
+        hsum = __fadd_rn(hsum, hs);
+        return fx_from_df(hs, __fmul_rn(acc.l, __fmul_rn(sc, 0x1p22f)));
+    };
+    // every propensity of this lane's chunk and their sum, its two words the
+    // sums of the propensities' words (what the list updates add to; without
+    // lists, for chunks of any length, those of the sum itself)
+    auto eval_own = [&](float sc, uint32_t &mx, float &hsum) {
+        int64_t s = 0;
+        uint32_t low = 0;
+        const int r_hi = min(n.R, gl * n.C + n.C);
+        for (int r = min(n.R, gl * n.C); r < r_hi; ++r) {
+            const int64_t v = eval_prop(r, sc, mx, hsum);
+            prop[r] = v;
+            s += v;
+            low += (uint32_t)v & 0xFFFFFFu;
+        }
+        if (!n.dep_list) low = (uint32_t)s & 0xFFFFFFu;
+        csum[gl] = make_uint2(low, (uint32_t)((s - (int64_t)low) >> 24));
+    };
+
     const int64_t t_start = global_ns();
-    unsigned long long warp_events = 0;
-    bool abort_run = false;
+    unsigned long long group_events = 0;
+    bool idle = false, aborted = false;
+    int attn = kTake;
+    bool stale = true;        // every propensity to be evaluated, the scale chosen anew
+    bool exact_traj = false;  // every interval of the trajectory runs exactly
+    bool absorbed = false;    // every propensity is 0
+    float sc = 1.0f;          // scale of the fixed point
+    float etf = 1.0f;         // clock: units of 1 / etf from the interval's start on
+    int64_t D = 0, clk = 0, err = 0, err_step = 0;  // interval, clock, its error bound, a step's share
+    uint32_t nev = 0;         // events of the interval
+    double T_next = 0.0;      // the next interval's end
+    Xoshiro g{0, 0, 0, 0};    // the same on every lane
+    unsigned int steps = 0;
 
     for (;;) {
-        long long ticket = 0;
-        if (lane == 0) ticket = (long long)atomicAdd(a.work, 1ull);
-        ticket = __shfl_sync(0xffffffffu, ticket, 0);
-        if (ticket >= a.n_traj) break;
+        __syncwarp();
+        if (attn != kRunning) {
+            if (attn == kRecord) {
+                // ---- record sample i at t = T
+                const long long i = gs.i, n_traj = gs.n_traj;
+                int64_t *o = gs.out;
+                const int n_save = gs.n_save;
+                for (int k = gl; k < n_save; k += G) o[(size_t)k * n_traj] = cnt[gs.save_idx[k]];
+                const unsigned long long ev = gs.ev + nev;
+                const bool last = i + 1 == gs.it->n_samples;
+                gr.sync();
+                if (gl == 0) {
+                    gs.ev = ev;
+                    gs.i = i + 1;
+                    gs.out = o + (size_t)n_save * n_traj;
+                    gs.t0 = gs.T;
+                }
+                attn = kBegin;
+                if (last) {
+                    attn = kTake;
+                    const SsaArgs &it = *gs.it;
+                    const long long traj = gs.traj;
+                    if (it.fin_species)
+                        for (int s = gl; s < it.S; s += G) it.fin_species[traj * it.S + s] = cnt[s];
+                    if (gl == 0) {
+                        if (it.fin_t) it.fin_t[traj] = gs.T;
+                        if (it.fin_rng) {
+                            it.fin_rng[traj * 4 + 0] = g.s0;
+                            it.fin_rng[traj * 4 + 1] = g.s1;
+                            it.fin_rng[traj * 4 + 2] = g.s2;
+                            it.fin_rng[traj * 4 + 3] = g.s3;
+                        }
+                        if (it.events) it.events[traj] = ev;
+                        group_events += ev;
+                    }
+                }
+                gr.sync();
+            }
+            if (attn == kTake) {
+                // ---- the next trajectory, if there is one
+                long long ticket = 0;
+                if (gl == 0) ticket = (long long)atomicAdd(a.work, 1ull);
+                ticket = gr.get((int64_t)ticket, 0);
+                if (ticket >= (BATCH ? a.n_warp_tickets : a.n_traj)) {
+                    idle = true;
+                    attn = kRunning;
+                } else {
+                    long long traj = ticket;
+                    const SsaArgs *itp = &a;
+                    if (BATCH) {
+                        int lo = 0, hi = a.batch_n - 1;  // last item with batch_start <= ticket
+                        while (lo < hi) {
+                            const int mid = (lo + hi + 1) >> 1;
+                            if (a.batch_start[mid] <= ticket) lo = mid;
+                            else hi = mid - 1;
+                        }
+                        itp = a.batch + lo;
+                        traj = ticket - a.batch_start[lo];
+                    }
+                    const SsaArgs &it = *itp;
+                    const int S = it.S, R = it.R;
+                    double t = 0.0;
+                    if (it.in_species) {
+                        for (int s = gl; s < S; s += G) cnt[s] = it.in_species[traj * S + s];
+                        t = it.in_t[traj];
+                        g = Xoshiro{it.in_rng[traj * 4], it.in_rng[traj * 4 + 1], it.in_rng[traj * 4 + 2],
+                                    it.in_rng[traj * 4 + 3]};
+                    } else {
+                        for (int s = gl; s < S; s += G) cnt[s] = it.x0[traj * it.x0_stride + s];
+                        xo_seed(g, it.seeds[traj]);
+                    }
+                    const double *rates = it.rate + traj * it.rate_stride;
+                    bool ex_t = !spec_rate_ok((uint64_t)__double_as_longlong(t)) || !(t < 0x1p60);
+                    for (int r = gl; r < R; r += G) ex_t |= !spec_rate_ok((uint64_t)__double_as_longlong(rates[r]));
+                    if (!BATCH && it.rate_stride)
+                        for (int r = gl; r < R; r += G) {
+                            const DF d = df_from_double(rates[r]);
+                            rdf_w[r] = make_float2(d.h, d.l);
+                        }
+                    // (choice margins stay below 2^32 units)
+                    exact_traj = gr.any(ex_t) || it.max_mults > 1024;
+                    stale = true;
+                    if (gl == 0) {
+                        gs.it = itp;
+                        gs.traj = traj;
+                        gs.i = 0;
+                        gs.ev = 0;
+                        gs.t0 = t;
+                        gs.sample_t = it.sample_t;
+                        gs.save_idx = it.save_idx;
+                        gs.out = it.out + traj;
+                        gs.n_traj = it.n_traj;
+                        gs.n_save = it.n_save;
+                        gs.S = S;
+                        if (BATCH) {
+                            group_net<G>(gs.net, it);
+                            gs.net.rdf = it.lm_rdf;
+                            gs.net.shape = it.lm_shape;
+                            gs.net.jump = it.lm_jump;
+                        }
+                    }
+                    T_next = it.sample_t[0];
+                    gr.sync();
+                    for (int s = gl; s <= S; s += G) cntf[s] = s < S ? (float)cnt[s] : 1.0f;
+                    gr.sync();
+                    attn = kBegin;
+                }
+            }
+            if (attn == kBegin) {
+                // ---- interval start: save what an exact re-run needs
+                const double T = T_next, t0 = gs.t0;
+                const long long i = gs.i;
+                for (int s = gl; s < gs.S; s += G) cnt0[s] = cnt[s];
+                if (gl == 0) {
+                    gs.T = T;
+                    gs.g0[0] = g.s0;
+                    gs.g0[1] = g.s1;
+                    gs.g0[2] = g.s2;
+                    gs.g0[3] = g.s3;
+                }
+                // the next interval's end, asked for an interval ahead
+                T_next = i + 1 < gs.it->n_samples ? gs.sample_t[i + 1] : T;
+                nev = 0;
+                clk = 0;
+                // the ordinary interval in integers (interval_clock's numbers;
+                // its FP64 chain took as long as a step): T - t0 = 1.m 2^k has D
+                // = 1.m 2^50, and 2^-52 T is below 2^(e - k) units for T < 2^(e + 1)
+                const uint64_t Tb = (uint64_t)__double_as_longlong(T);
+                const uint64_t lb = (uint64_t)__double_as_longlong(__dsub_rn(T, t0));
+                const int eT = (int)(Tb >> 52), el = (int)(lb >> 52);  // 2048 and more: negative
+                bool exact = exact_traj;
+                if (el >= 1023 - 60 && el <= eT && eT < 1023 + 60) {
+                    etf = pow2f(50 + 1023 - el);
+                    D = (int64_t)(((lb & 0xFFFFFFFFFFFFFull) | 1ull << 52) >> 2);
+                    err_step = (1ll << min(eT - el, 50)) + 4;
+                } else if (!interval_clock(T, t0, etf, D, err_step)) {
+                    exact = true;
+                }
+                err = 2 * err_step;
+                attn = exact ? kExact : stale ? kFull : kRunning;
+                gr.sync();
+            }
+            if (attn == kFull) {
+                // ---- every propensity, after the scale: 2^27 <= total * sc < 2^28
+                uint32_t mx = 0u;
+                float tf = 0.0f;
+                const int r_hi = min(n.R, gl * n.C + n.C);
+                for (int r = min(n.R, gl * n.C); r < r_hi; ++r) eval_prop(r, 1.0f, mx, tf);
+                tf = gr.sum(tf);
+                // an undecided step: a count out of range, a total beyond 2^90
+                // (a positive one is at least 2^-60)
+                if (gr.any(mx >= 0x4B000000u) || !(tf <= 0x1p90f) || (tf > 0.0f && tf < 0x1p-60f)) {
+                    attn = kExact;
+                } else {
+                    absorbed = tf == 0.0f;
+                    sc = absorbed ? 1.0f : pow2f(27 - ilog2f(tf));
+                    float unused = 0.0f;
+                    eval_own(sc, mx, unused);
+                    stale = false;
+                    attn = kRunning;
+                }
+                gr.sync();
+            }
+            if (attn == kExact) {
+                // ---- exact re-run of the interval from its saved start
+                const SsaArgs &it = *gs.it;
+                const double *rates = it.rate + gs.traj * it.rate_stride;
+                const double T = gs.T;
+                double t = gs.t0;
+                if (!exact_traj && gl == 0) atomicAdd(a.work + 3, 1ull);
+                for (int s = gl; s < it.S; s += G) cnt[s] = cnt0[s];
+                Xoshiro h{gs.g0[0], gs.g0[1], gs.g0[2], gs.g0[3]};
+                nev = 0;
+                gr.sync();
+                attn = kRecord;
+                for (unsigned int k = 1;; ++k) {
+                    if ((k & 255u) == 0) {
+                        int late = gl == 0 && global_ns() - t_start > a.budget_ns;
+                        if (gr.get(late, 0)) {
+                            aborted = idle = true;
+                            attn = kRunning;
+                            break;
+                        }
+                    }
+                    int idx = 0;
+                    if (!warp_exact_step<G>(it, gr, cnt, rates, a.zig, scr, h, t, T, idx)) break;
+                    ++nev;
+                    if (idx < it.R)
+                        for (int q = gl; q < it.Q; q += G) {
+                            const int64_t dlt = it.jmp_d[idx * it.Q + q];
+                            if (dlt != 0) cnt[it.jmp_sp[idx * it.Q + q]] += dlt;
+                        }
+                    gr.sync();
+                }
+                for (int s = gl; s < it.S; s += G) cntf[s] = (float)cnt[s];
+                stale = true;
+                // the first lane drew: its generator is the trajectory's
+                g.s0 = (uint64_t)gr.get((int64_t)h.s0, 0);
+                g.s1 = (uint64_t)gr.get((int64_t)h.s1, 0);
+                g.s2 = (uint64_t)gr.get((int64_t)h.s2, 0);
+                g.s3 = (uint64_t)gr.get((int64_t)h.s3, 0);
+                gr.sync();
+            }
+        }
+        if (__all_sync(0xffffffffu, idle)) break;
+        if ((++steps & 255u) == 0 && __any_sync(0xffffffffu, global_ns() - t_start > a.budget_ns)) {
+            aborted |= !idle;
+            idle = true;
+        }
+        const bool run = attn == kRunning && !idle;
 
-        // ---- a thread unit: 32 trajectories of a small network, one per lane
-        if (BATCH && ticket >= a.n_warp_tickets) {
-            const long long u = ticket - a.n_warp_tickets;
+        // ---- one step of every group (a group that is not running commits
+        // nothing): chunk prefixes and the total
+        const uint2 cs = csum[gl];
+        const int64_t ls = (int64_t)(((uint64_t)cs.y << 24) + cs.x);
+        const int64_t incl = al.scan(ls);
+        const int64_t tot = al.get(incl, G - 1);
+        const bool in_scale = (uint64_t)tot - (1ull << 46) < (1ull << 51) - (1ull << 46);
+        // ---- both draws the step may make, taken ahead (stepped back when
+        // fewer are committed)
+        const uint64_t b1 = xo_next(g);
+        uint64_t bu = xo_next(g);
+        const int layer = (int)(b1 & 0xff);
+        const float2 X = xdf[layer];
+        DF x = df_mul(df_u53_rel(2 * (b1 >> 12) + 1), DF{X.x, X.y});
+        if (!((b1 >> 12) < zxk[layer].y) && run && in_scale) {
+            // wedge or tail (1.2 % of draws): the choice takes the draw after
+            Xoshiro h = g;
+            x = exp1_df_rel_cont(h, b1, bu, x, ex, xdf);
+            bu = xo_next(h);
+            g = h;
+        }
+        // ---- Exp1 / total in clock units, the decision
+        const DF td = df_from_fx(tot);
+        const DF q = df_div(x, td, rcp_approx(td.h));  // / (sc 2^22)
+        const float qh = fminf(__fmul_rn(__fmul_rn(q.h, sc), etf), 0x1p30f);
+        const float ql = fmaxf(fminf(__fmul_rn(__fmul_rn(q.l, __fmul_rn(sc, 0x1p22f)), etf), 0x1p30f), -0x1p30f);
+        const int64_t qc = fx_from_df(qh, ql);
+        const int64_t clk_n = clk + qc;
+        const int64_t err_n = err + err_step + (qc >> n.sh_q);
+        const int64_t d = D - clk_n;
+        const bool fire = run && in_scale && d > err_n && q.h >= 0x1p-100f;
+        // ---- the choice: #{r : cum_r < total * U}
+        const int64_t ch = (int64_t)__umul64hi((uint64_t)tot, bu & ~0x7FFull);
+        const int64_t di = incl - ch;
+        const int k = __popc(al.ballot(di < 0)) & (G - 1);       // chunks entirely below the choice
+        const int64_t carry = al.get(incl - ls, k) - ch;         // running sum before chunk k
+        // some |running sum - choice| below 2^32: looked at again below
+        bool near = (uint32_t)((int)(di >> 32) + 1) <= 1u;
+        // walk chunk k with the whole group: lane j takes its reactions
+        // j*E .. j*E + E - 1
+        const int R = n.R, C = n.C, E = n.E;
+        const int w_end = min(R, k * C + C), w_lo = min(w_end, k * C + gl * E), w_hi = min(w_end, w_lo + E);
+        int idx = k * C;
+        if (BATCH ? __all_sync(0xffffffffu, E <= 1) : E <= 1) {
+            const int64_t dr = carry + al.scan(w_lo < w_hi ? prop[w_lo] : 0);
+            idx += __popc(al.ballot(w_lo < w_hi && dr < 0));
+            near |= (uint32_t)((int)(dr >> 32) + 1) <= 1u;
+        } else {
+            // a lane's first 4 reactions at once, more in a loop
+            int64_t v[4], s = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[j] = w_lo + j < w_hi ? prop[w_lo + j] : 0;
+                s += v[j];
+            }
+            for (int r = w_lo + 4; r < w_hi; ++r) s += prop[r];
+            int64_t dr = carry + al.scan(s) - s;
+            int below = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                dr += v[j];
+                below += w_lo + j < w_hi && dr < 0 ? 1 : 0;
+                near |= (uint32_t)((int)(dr >> 32) + 1) <= 1u;
+            }
+            for (int r = w_lo + 4; r < w_hi; ++r) {
+                dr += prop[r];
+                below += dr < 0 ? 1 : 0;
+                near |= (uint32_t)((int)(dr >> 32) + 1) <= 1u;
+            }
+            // the first lane whose reactions are not all below has the choice
+            const int kl = __popc(al.ballot(dr < 0)) & (G - 1);
+            idx += kl * E + al.get(below, kl);
+        }
+        if ((al.any(near) || a.exact_choice) && fire) {
+            // within the margin the choice alone is redone exactly (the clock
+            // is decided; the fixed-point propensities are overwritten)
+            const int64_t m = (tot >> n.sh_p) + 4 * (int64_t)R + 16;
+            bool close = di <= m && di >= -m;
+            int64_t s = 0;
+            for (int r = w_lo; r < w_hi; ++r) s += prop[r];
+            int64_t dr = carry + gr.scan(s) - s;
+            for (int r = w_lo; r < w_hi; ++r) {
+                dr += prop[r];
+                close |= dr <= m && dr >= -m;
+            }
+            if (gr.any(close) || a.exact_choice) {
+                gr.sync();
+                const SsaArgs &it = *gs.it;
+                idx = warp_exact_choice<G>(it, gr, cnt, it.rate + gs.traj * it.rate_stride, scr, bu >> 11);
+                stale = true;
+                attn = kFull;
+            }
+        }
+        uint32_t head = 0;  // the propensities to re-evaluate
+        if (fire) {
+            // ---- clock and jump
+            clk = clk_n;
+            err = err_n;
+            ++nev;
+            if (idx < R) {
+                if (attn == kRunning) head = n.dep_list ? n.dep_head[idx] : kDepAll;
+                int q2 = gl;
+                do {
+                    int sp = 0;
+                    int64_t dlt = 0;
+                    if (q2 < n.Q) {
+                        if (n.jump) {
+                            const uint32_t e = n.jump[idx * n.Q + q2];
+                            sp = (int)(e & 0xFFFFu);
+                            dlt = (int64_t)((int32_t)e >> 16);
+                        } else {
+                            sp = n.jmp_sp[idx * n.Q + q2];
+                            dlt = n.jmp_d[idx * n.Q + q2];
+                        }
+                    }
+                    if (dlt != 0) {
+                        cnt[sp] += dlt;
+                        cntf[sp] = __fadd_rn(cntf[sp], (float)dlt);
+                    }
+                    q2 += G;
+                } while (q2 - gl < n.Q);
+            }
+        } else {
+            xo_prev(g);  // the uniform was not drawn,
+            if (!run || !in_scale) xo_prev(g);  // nor the Exp1
+            // out of scale: nothing can fire (the sample records), or a new
+            // scale; an undecided clock: the interval again, exactly; else the
+            // sample records
+            if (run) attn = !in_scale ? (absorbed ? kRecord : kFull)
+                            : d + err_n >= 0 || !(q.h >= 0x1p-100f) ? kExact : kRecord;
+        }
+        __syncwarp();
+        // ---- re-evaluate the propensities that read a changed species; their
+        // differences go to the chunk sums
+        uint32_t mx = 0u;
+        float hsum = 0.0f;
+        const int nd = (int)(head & kDepAll);
+        if (nd == (int)kDepAll) {
+            eval_own(sc, mx, hsum);
+        } else {
+            const uint16_t *list = n.dep_list + 8 * (size_t)(head >> 12);
+            auto update = [&](int r, int64_t v) {
+                const int64_t old = prop[r];
+                prop[r] = v;
+                const int o = C > 1 ? (int)__umulhi((uint32_t)r, n.c_inv) : r;
+                atomicAdd(&csum[o].x, ((uint32_t)v & 0xFFFFFFu) - ((uint32_t)old & 0xFFFFFFu));
+                atomicAdd(&csum[o].y, (uint32_t)(v >> 24) - (uint32_t)(old >> 24));
+            };
+            if (nd <= G) {
+                if (gl < nd) {
+                    const int r = list[gl];
+                    update(r, eval_prop(r, sc, mx, hsum));
+                }
+            } else {
+                // two reactions a lane at a time, their chains side by side
+                for (int j = gl; j < nd; j += 2 * G) {
+                    const bool two = j + G < nd;
+                    const int r0 = list[j], r1 = two ? list[j + G] : r0;
+                    const int64_t v0 = eval_prop(r0, sc, mx, hsum), v1 = eval_prop(r1, sc, mx, hsum);
+                    update(r0, v0);
+                    if (two) update(r1, v1);
+                }
+            }
+        }
+        // a count out of range makes the next step undecided, sums that outgrew
+        // the fixed point ask for a new scale
+        const bool out = mx >= 0x4B000000u;
+        if (al.any(out || !(hsum < 1.9f * 0x1p28f))) attn = gr.any(out) ? kExact : kFull;
+    }
+    if (aborted && gl == 0) atomicExch(a.work + 2, 1ull);
+    if (BATCH) {
+        // ---- thread units, taken by whole warps once the warp's groups have
+        // found no trajectory left: 32 trajectories of a small network, one
+        // per lane
+        bool stop = __any_sync(0xffffffffu, aborted);
+        while (!stop) {
+            long long u = 0;
+            if (lane == 0) u = (long long)atomicAdd(a.work + 4, 1ull);
+            u = __shfl_sync(0xffffffffu, u, 0);
+            if (u >= a.n_traj - a.n_warp_tickets) break;
             int lo = 0, hi = a.tbatch_n - 1;  // last item with tbatch_unit <= u
             while (lo < hi) {
                 const int mid = (lo + hi + 1) >> 1;
@@ -550,487 +1116,107 @@ __global__ void __launch_bounds__(32 * (BATCH ? kWarpMaxWarpsBatch : kWarpMaxWar
             bool late = false;
             const SsaArgs &ti = a.tbatch[lo];
             const long long first = (u - a.tbatch_unit[lo]) * 32;
-            unsigned long long ev = ti.R <= 4   ? thread_unit<MACRO, 4>(ti, ex, xdf, wbase, first, t_start, late)
-                                    : ti.R <= 8 ? thread_unit<MACRO, 8>(ti, ex, xdf, wbase, first, t_start, late)
-                                                : thread_unit<MACRO, 16>(ti, ex, xdf, wbase, first, t_start, late);
-            for (int off = 16; off > 0; off >>= 1) ev += __shfl_xor_sync(0xffffffffu, ev, off);
-            warp_events += ev;
-            if (__any_sync(0xffffffffu, late)) {
-                if (lane == 0) atomicExch(a.work + 2, 1ull);
-                break;
-            }
-            __syncwarp();
-            continue;
-        }
-
-        // ---- the trajectory's network and run
-        long long traj = ticket;
-        const SsaArgs *itp = &a;
-        if (BATCH) {
-            int lo = 0, hi = a.batch_n - 1;  // last item with batch_start <= ticket
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (a.batch_start[mid] <= ticket) lo = mid;
-                else hi = mid - 1;
-            }
-            itp = a.batch + lo;
-            traj = ticket - a.batch_start[lo];
-        }
-        const SsaArgs &it = *itp;
-        const int S = it.S, R = it.R, P = it.P, Q = it.Q;
-        const int C = warp_chunk(R);
-        const float2 *rdf = BATCH ? it.lm_rdf : (it.rate_stride ? rdf_w : rdf_sh);
-        const int32_t *facl = BATCH ? it.lm_fac : facl_sh;
-        const uint32_t *shape = BATCH ? it.lm_shape : shape_sh;
-        const bool use_shape = BATCH ? it.lm_shape != nullptr : (it.max_mults <= 2 && it.S < 32767);
-        // lane l owns reactions [l * C, min(R, (l + 1) * C)); local index i sits at i*32 + l
-        const int r_lo = min(R, lane * C), r_hi = min(R, r_lo + C);
-        const int n_own = r_hi - r_lo;
-        const int mm = use_shape ? 2 : it.max_mults;  // multiplies per propensity
-        // dependency masks; without them every propensity is re-evaluated
-        const int dep_bytes = it.dep_bytes, n_words = (C + 31) >> 5;
-        const void *dep_tab = it.dep_tab;
-        // Fixed point: single propensities and the 32 chunk sums stay below
-        // 2^52, so nothing overflows (up to 256 reactions a lane); the total is
-        // scaled to 2^50 .. 2^51, and scaled anew when it falls below 2^47 or a
-        // chunk sum reaches 2^52.
-        // Relative error bound of a propensity or sum against the reference's
-        // binary64 one, apart from one unit per propensity:
-        const float c_p = (float)(mm + 2) * kGamma + (float)(R + mm + 4) * 0x1p-53f;
-        // Exp1 / total: the total's bound (its units at the smallest total),
-        // the Exp1 pair, the total's pair and the division
-        const float c_q = (c_p + (float)(R + 2) * 0x1p-47f + 9.0f * kGamma) * 1.001f;
-        const int sh_q = -ilog2f(c_q) - 1;         // 2^-sh_q >= c_q
-        const int sh_p = -ilog2f(2.0f * c_p) - 1;  // choice: both operands' bounds
-        // fixed-point propensity of the reaction at lane-major position pos, sc
-        // times its value in units of 2^-22; mx collects the largest count it read (as float
-        // bits: a count outside [0, 2^23) has bits >= 0x4B000000), mh the
-        // largest sc * propensity
-        auto eval_prop = [&](int pos, float sc, uint32_t &mx, float &mh) -> int64_t {
-            const float2 k = rdf[pos];
-            DF acc{k.x, k.y};
-            if (use_shape) {
-                const uint32_t w = shape[pos];  // the first slot's offset is 0
-                const float n1 = cntf[w & 0x7FFFu], n2 = cntf[(w >> 16) & 0x7FFFu];
-                mx = max(mx, max(__float_as_uint(n1), __float_as_uint(n2)));
-                acc = df_mul_fu(df_mul_fu(acc, n1), fmaxf(__fsub_rn(n2, (float)(w >> 31)), 0.0f));
-            } else {
-                const int i2 = pos >> 5, l = pos & 31;
-                for (int p = 0; p < P; ++p) {
-                    const int f = facl[(i2 * P + p) * 32 + l];
-                    const int o = f >> 16;
-                    if (o == 0) continue;
-                    const float n = cntf[f & 0xFFFF];
-                    mx = max(mx, __float_as_uint(n));
-                    for (int j = 0; j < o; ++j) acc = df_mul_fu(acc, fmaxf(__fsub_rn(n, (float)j), 0.0f));
-                    acc = fast2sum(acc.h, acc.l);
-                }
-            }
-            const float hs = __fmul_rn(acc.h, sc);
-            mh = fmaxf(mh, hs);
-            return fx_from_df(hs, __fmul_rn(acc.l, __fmul_rn(sc, 0x1p22f)));
-        };
-        bool need_full = true;  // every propensity to be evaluated, the scale chosen anew
-        bool amb_next = false;  // a re-evaluated propensity read a count out of range
-        bool absorbed = false;  // every propensity is 0
-        float sc = 1.0f;        // scale of the fixed point
-        int64_t ls = 0;         // this lane's chunk sum
-
-        // ---- start (or resume) the trajectory.  g (the same on every lane) is
-        // the generator past the word buffer, word p of which comes next
-        // (p = 32: empty); x and acc_mask are the words' Exp1 candidates and
-        // which of them the ziggurat's first test accepts.
-        Xoshiro g;
-        int p = 32;
-        uint64_t word = 0;
-        DF x{0.f, 0.f};
-        uint32_t acc_mask = 0;
-        double t;
-        if (it.in_species) {
-            for (int s = lane; s < S; s += 32) cnt[s] = it.in_species[traj * S + s];
-            t = it.in_t[traj];
-            g = Xoshiro{it.in_rng[traj * 4], it.in_rng[traj * 4 + 1], it.in_rng[traj * 4 + 2], it.in_rng[traj * 4 + 3]};
-        } else {
-            for (int s = lane; s < S; s += 32) cnt[s] = it.x0[traj * it.x0_stride + s];
-            t = 0.0;
-            xo_seed(g, it.seeds[traj]);
-        }
-        const double *rates = it.rate + traj * it.rate_stride;
-        bool exact_traj = !spec_rate_ok((uint64_t)__double_as_longlong(t)) || !(t < 0x1p60);
-        for (int r = lane; r < R; r += 32) exact_traj |= !spec_rate_ok((uint64_t)__double_as_longlong(rates[r]));
-        if (!BATCH && it.rate_stride)
-            for (int q = lane; q < 32 * C; q += 32) {
-                const int r = (q & 31) * C + (q >> 5);
-                const DF d = r < R ? df_from_double(rates[r]) : DF{0.f, 0.f};
-                rdf_w[q] = make_float2(d.h, d.l);
-            }
-        exact_traj = __any_sync(0xffffffffu, exact_traj) || mm > 1024;  // (choice margins stay below 2^32 units)
-        for (int s = lane; s <= S; s += 32) cntf[s] = s < S ? (float)cnt[s] : 1.0f;
-        __syncwarp();
-        unsigned long long ev = 0;
-
-        // the generator before word q of the buffer that starts at state st
-        auto state_at = [&](const uint64_t *st, int q) {
-            Xoshiro h{st[0], st[1], st[2], st[3]};
-            for (int k = 0; k < q; ++k) xo_next(h);
-            return h;
-        };
-        for (long long i = 0; i < it.n_samples && !abort_run; ++i) {
-            const double T = it.sample_t[i];
-            // ---- interval start: save what an exact re-run needs
-            for (int s = lane; s < S; s += 32) cnt0[s] = cnt[s];
-            const int p0 = p;
-            __syncwarp();
-            if (lane == 0) {
-                const bool empty = p == 32;  // then the generator itself is the state
-                gst[8] = empty ? g.s0 : gst[0];
-                gst[9] = empty ? g.s1 : gst[1];
-                gst[10] = empty ? g.s2 : gst[2];
-                gst[11] = empty ? g.s3 : gst[3];
-            }
-            const double t0 = t;
-            const unsigned long long ev0 = ev;
-            bool replay = exact_traj || !(T < 0x1p60) || (T != 0.0 && !(T >= 0x1p-60));
-            // clock: units of 2^-et from t0 on; the interval (the sample time
-            // itself when it is empty or lies behind t0) fills 2^50 .. 2^51
-            const double len = __dsub_rn(T, t0);
-            const double base = len > 0.0 ? len : (T > 0.0 ? T : 1.0);
-            replay |= !(base >= 0x1p-60) || !(fabs(len) <= base * 0x1p2);
-            const int et = replay ? 0 : 50 - ilog2d(base);
-            const double ets = __longlong_as_double((long long)(1023 + et) << 52);
-            const float etf = pow2f(et);
-            const int64_t D = replay ? 0 : __double2ll_rn(__dmul_rn(len, ets));
-            // what a step adds to the clock's error bound beside the quotient's:
-            // the reference's rounding (2^-52 T), the conversions' units
-            const int64_t err_step = replay ? 0 : __double2ll_ru(__dmul_ru(__dmul_ru(T, 0x1p-52), ets)) + 4;
-            int64_t clk = 0, err = 2 * err_step;
-            __syncwarp();
-            unsigned int steps = 0;
-            while (!replay) {
-                if ((++steps & 255u) == 0) {
-                    int late = lane == 0 && global_ns() - t_start > a.budget_ns;
-                    if (__shfl_sync(0xffffffffu, late, 0)) {
-                        abort_run = true;
-                        break;
-                    }
-                }
-                if (need_full || amb_next) {
-                    // ---- every propensity of this lane's chunk, after the
-                    // scale: 2^28 <= total * sc < 2^29
-                    uint32_t mx = amb_next ? 0x7F800000u : 0u;
-                    float mh = 0.0f, tf = 0.0f;
-                    for (int i2 = 0; i2 < n_own && !amb_next; ++i2) {
-                        float h = 0.0f;
-                        eval_prop(i2 * 32 + lane, 1.0f, mx, h);
-                        tf = __fadd_rn(tf, h);
-                    }
-#pragma unroll
-                    for (int d = 16; d > 0; d >>= 1) tf = __fadd_rn(tf, __shfl_xor_sync(0xffffffffu, tf, d));
-                    // an undecided step: a count out of range, a total beyond
-                    // 2^90 or below 2^-90 (where a positive one is possible)
-                    if (__any_sync(0xffffffffu, mx >= 0x4B000000u) || !(tf <= 0x1p90f) || (tf > 0.0f && tf < 0x1p-60f)) {
-                        replay = true;
-                        break;
-                    }
-                    absorbed = tf == 0.0f;
-                    sc = absorbed ? 1.0f : pow2f(28 - ilog2f(tf));
-                    ls = 0;
-                    for (int i2 = 0; i2 < n_own; ++i2) {
-                        const int64_t v = eval_prop(i2 * 32 + lane, sc, mx, mh);
-                        prop[pz(i2 * 32 + lane)] = v;
-                        ls += v;
-                    }
-                    need_full = false;
-                    __syncwarp();
-                }
-                // ---- chunk prefixes and the total
-                const int64_t incl = scan_i64(ls, 32);
-                const int64_t tot = shfl_i64(incl, 31);
-                if (tot < (1ll << 47)) {
-                    if (absorbed) break;  // no reaction can fire: the sample records, no draw is made
-                    need_full = true;     // too few bits left (a new scale's total has 50)
-                    continue;
-                }
-                // ---- draws: refill the buffer when fewer than two words are left
-                if (p > 30) {
-                    __syncwarp();
-                    int first = 0;
-                    uint64_t w0 = 0;
-                    if (p == 31) {  // the last word is still to come
-                        first = 1;
-                        w0 = (uint64_t)shfl_i64((int64_t)word, 31);
-                        if (lane < 4) gst[lane] = gst[4 + lane];
-                    } else if (lane == 0) {
-                        gst[0] = g.s0;
-                        gst[1] = g.s1;
-                        gst[2] = g.s2;
-                        gst[3] = g.s3;
-                    }
-                    word = w0;
-                    for (int k = first; k < 31; ++k) {
-                        const uint64_t w = xo_next(g);
-                        if (lane == k) word = w;
-                    }
-                    __syncwarp();
-                    if (lane == 0) {
-                        gst[4] = g.s0;
-                        gst[5] = g.s1;
-                        gst[6] = g.s2;
-                        gst[7] = g.s3;
-                    }
-                    const uint64_t w = xo_next(g);
-                    if (lane == 31) word = w;
-                    p = 0;
-                    const int layer = (int)(word & 0xff);
-                    const float2 X = xdf[layer];
-                    x = df_mul(df_u53_rel(2 * (word >> 12) + 1), DF{X.x, X.y});
-                    acc_mask = __ballot_sync(0xffffffffu, (word >> 12) < zxk[layer].y);
-                    __syncwarp();
-                }
-                DF xe{__shfl_sync(0xffffffffu, x.h, p), __shfl_sync(0xffffffffu, x.l, p)};
-                uint64_t bu = (uint64_t)shfl_i64((int64_t)word, p + 1);
-                int used = p + 1;  // words consumed by the Exp1 draw, counted from the buffer's start
-                const bool slow = !((acc_mask >> p) & 1u);
-                Xoshiro gs{0, 0, 0, 0};
-                if (slow) {
-                    // wedge or tail (1.2 % of draws): the generator itself from
-                    // here on, the buffer is given up
-                    gs = state_at(gst, p);
-                    xe = exp1_df_rel(gs, ex, xdf);
-                }
-                // ---- Exp1 / total in clock units, the decision
-                const DF td = df_from_fx(tot);
-                const DF q = df_div(xe, td, rcp_approx(td.h));  // / (sc 2^22)
-                const float qh = fminf(__fmul_rn(__fmul_rn(q.h, sc), etf), 0x1p30f);
-                const float ql = fmaxf(fminf(__fmul_rn(__fmul_rn(q.l, __fmul_rn(sc, 0x1p22f)), etf), 0x1p30f), -0x1p30f);
-                const int64_t qc = fx_from_df(qh, ql);
-                const int64_t clk_n = clk + qc;
-                const int64_t err_n = err + err_step + (qc >> sh_q);
-                const int64_t d = D - clk_n;
-                if (d <= err_n || q.h < 0x1p-100f) {  // not a clear fire
-                    if (d + err_n >= 0 || q.h < 0x1p-100f) {
-                        replay = true;
-                        break;
-                    }
-                    // the sample records; the Exp1 draw was made
-                    if (slow) {
-                        g = gs;
-                        p = 32;
-                    } else {
-                        p = used;
-                    }
-                    break;
-                }
-                clk = clk_n;
-                err = err_n;
-                if (slow) {
-                    bu = xo_next(gs);
-                    g = gs;
-                    p = 32;
-                } else {
-                    p = used + 1;
-                }
-                // ---- the choice: #{r : cum_r < total * U}
-                const int64_t ch = (int64_t)__umul64hi((uint64_t)tot, bu & ~0x7FFull);
-                const int64_t di = incl - ch;
-                const int k = __popc(__ballot_sync(0xffffffffu, di < 0));  // chunks entirely below the choice
-                const int64_t before = shfl_i64(incl - ls, k & 31);        // running sum before chunk k
-                bool near = (uint32_t)((int)(di >> 32) + 1) <= 1u;         // |di| < 2^32
-                // walk chunk k with the whole warp: lane j takes its reaction k*C + j
-                int count = 0;
-                int64_t carry = before - ch, dr = di;
-                for (int seg = 0; seg < C; seg += 32) {
-                    const int j = seg + lane;
-                    const bool valid = j < C && k * C + j < R;
-                    dr = carry + scan_i64(valid ? prop[pz(j * 32 + k)] : 0, C);
-                    count += __popc(__ballot_sync(0xffffffffu, valid && dr < 0));
-                    near |= (uint32_t)((int)(dr >> 32) + 1) <= 1u;
-                    if (C > 32) carry = shfl_i64(dr, 31);
-                }
-                int idx = k * C + count;
-                if (__any_sync(0xffffffffu, near) || a.exact_choice) {
-                    // some sum lies within 2^32 units of the choice: within the
-                    // margin the choice alone is redone exactly (the clock is
-                    // decided; the fixed-point propensities are overwritten)
-                    const int64_t m = (tot >> sh_p) + 4 * (int64_t)R + 16;
-                    bool close = di <= m && di >= -m;
-                    for (int seg = 0; seg < C; seg += 32) {
-                        const int j = seg + lane;
-                        if (seg == 0) carry = before - ch;
-                        dr = carry + scan_i64(j < C && k * C + j < R ? prop[pz(j * 32 + k)] : 0, 32);
-                        close |= dr <= m && dr >= -m;
-                        carry = shfl_i64(dr, 31);
-                    }
-                    if (__any_sync(0xffffffffu, close) || a.exact_choice) {
-                        __syncwarp();
-                        idx = warp_exact_choice<MACRO>(it, cnt, rates, scr, bu >> 11);
-                        need_full = true;
-                    }
-                }
-                // ---- jump
-                ++ev;
-                if (idx < R)
-                    for (int q2 = lane; q2 < Q; q2 += 32) {
-                        int sp;
-                        int64_t dlt;
-                        if (BATCH || jd_wide) {
-                            sp = it.jmp_sp[idx * Q + q2];
-                            dlt = it.jmp_d[idx * Q + q2];
-                        } else {
-                            const uint32_t e = jump_sh[idx * Q + q2];
-                            sp = (int)(e & 0xFFFFu);
-                            dlt = (int64_t)((int32_t)e >> 16);
-                        }
-                        if (dlt != 0) {
-                            cnt[sp] += dlt;
-                            cntf[sp] = __fadd_rn(cntf[sp], (float)dlt);
-                        }
-                    }
-                __syncwarp();
-                // ---- re-evaluate this lane's propensities that read a changed
-                // species; their differences go to the chunk sum
-                if (idx < R && !need_full) {
-                    uint32_t mx = 0u;
-                    float mh = 0.0f;
-                    for (int w = 0; w < n_words; ++w) {
-                        const size_t e = ((size_t)idx * n_words + w) * 32 + lane;
-                        const int left = n_own - 32 * w;
-                        uint32_t m = left >= 32 ? 0xFFFFFFFFu : left > 0 ? (1u << left) - 1u : 0u;
-                        if (dep_tab)
-                            m = dep_bytes == 1   ? reinterpret_cast<const uint8_t *>(dep_tab)[e]
-                                : dep_bytes == 2 ? reinterpret_cast<const uint16_t *>(dep_tab)[e]
-                                                 : reinterpret_cast<const uint32_t *>(dep_tab)[e];
-                        while (m) {
-                            const int pos = (32 * w + __ffs((int)m) - 1) * 32 + lane;
-                            m &= m - 1u;
-                            const int64_t v = eval_prop(pos, sc, mx, mh);
-                            const int ps = pz(pos);
-                            ls += v - prop[ps];
-                            prop[ps] = v;
-                        }
-                    }
-                    __syncwarp();
-                    // a count out of range makes the next step undecided, a
-                    // sum that outgrew the fixed point asks for a new scale
-                    const bool out = mx >= 0x4B000000u;
-                    if (__any_sync(0xffffffffu, out || !(mh < 0x1p30f) || (uint64_t)ls >> kFxLim != 0)) {
-                        amb_next = __any_sync(0xffffffffu, out);
-                        need_full = true;
-                    }
-                }
-            }
-            if (abort_run) break;
-            if (replay) {
-                // ---- exact re-run of the interval from its saved start
-                if (!exact_traj && lane == 0) atomicAdd(a.work + 3, 1ull);
-                for (int s = lane; s < S; s += 32) cnt[s] = cnt0[s];
-                g = state_at(gst + 8, p0 == 32 ? 0 : p0);
-                p = 32;
-                t = t0;
-                ev = ev0;
-                __syncwarp();
-                for (unsigned int n = 1;; ++n) {
-                    if ((n & 255u) == 0) {
-                        int late = lane == 0 && global_ns() - t_start > a.budget_ns;
-                        if (__shfl_sync(0xffffffffu, late, 0)) {
-                            abort_run = true;
-                            break;
-                        }
-                    }
-                    int idx = 0;
-                    if (!warp_exact_step<MACRO>(it, cnt, rates, a.zig, scr, g, t, T, idx)) break;
-                    ++ev;
-                    if (idx < R)
-                        for (int q = lane; q < Q; q += 32) {
-                            const int64_t dlt = it.jmp_d[idx * Q + q];
-                            if (dlt != 0) cnt[it.jmp_sp[idx * Q + q]] += dlt;
-                        }
-                    __syncwarp();
-                }
-                if (abort_run) break;
-                for (int s = lane; s < S; s += 32) cntf[s] = (float)cnt[s];
-                need_full = true;
-                amb_next = false;
-                // lane 0 drew: its generator is the trajectory's
-                g.s0 = (uint64_t)shfl_i64((int64_t)g.s0, 0);
-                g.s1 = (uint64_t)shfl_i64((int64_t)g.s1, 0);
-                g.s2 = (uint64_t)shfl_i64((int64_t)g.s2, 0);
-                g.s3 = (uint64_t)shfl_i64((int64_t)g.s3, 0);
-                __syncwarp();
-            }
-            // ---- record sample i at t = T
-            t = T;
-            int64_t *o = it.out + (size_t)i * it.n_save * it.n_traj + traj;
-            for (int k = lane; k < it.n_save; k += 32) o[(size_t)k * it.n_traj] = cnt[it.save_idx[k]];
+            if (a.macro_mode)
+                group_events += ti.R <= 4   ? thread_unit<true, 4>(ti, ex, xdf, wbase, first, t_start, late)
+                                : ti.R <= 8 ? thread_unit<true, 8>(ti, ex, xdf, wbase, first, t_start, late)
+                                            : thread_unit<true, 16>(ti, ex, xdf, wbase, first, t_start, late);
+            else
+                group_events += ti.R <= 4   ? thread_unit<false, 4>(ti, ex, xdf, wbase, first, t_start, late)
+                                : ti.R <= 8 ? thread_unit<false, 8>(ti, ex, xdf, wbase, first, t_start, late)
+                                            : thread_unit<false, 16>(ti, ex, xdf, wbase, first, t_start, late);
+            stop = __any_sync(0xffffffffu, late);
+            if (stop && lane == 0) atomicExch(a.work + 2, 1ull);
             __syncwarp();
         }
-        if (abort_run) {
-            if (lane == 0) atomicExch(a.work + 2, 1ull);
-            break;
-        }
-        if (it.fin_species)
-            for (int s = lane; s < S; s += 32) it.fin_species[traj * S + s] = cnt[s];
-        if (it.fin_rng && p < 32) g = state_at(gst, p);
-        if (lane == 0) {
-            if (it.fin_t) it.fin_t[traj] = t;
-            if (it.fin_rng) {
-                it.fin_rng[traj * 4 + 0] = g.s0;
-                it.fin_rng[traj * 4 + 1] = g.s1;
-                it.fin_rng[traj * 4 + 2] = g.s2;
-                it.fin_rng[traj * 4 + 3] = g.s3;
-            }
-            if (it.events) it.events[traj] = ev;
-        }
-        warp_events += ev;
-        __syncwarp();
     }
-    if (lane == 0 && warp_events) atomicAdd(a.work + 1, warp_events);
+    for (int d = 16; d > 0; d >>= 1) group_events += __shfl_xor_sync(0xffffffffu, group_events, d);
+    if (lane == 0 && group_events) atomicAdd(a.work + 1, group_events);
 }
 
-template <bool MACRO, bool BATCH>
+template <bool BATCH, int G>
 int warp_launch(const SsaArgs &a, int block, int grid, size_t smem, cudaStream_t st) {
-    auto kern = ssa_warp_kernel<MACRO, BATCH>;
+    auto kern = ssa_warp_kernel<BATCH, G>;
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return (int)err;
     kern<<<grid, block, smem, st>>>(a);
     return (int)cudaGetLastError();
 }
 
+int group_of(const SsaArgs &a) { return a.group == 8 || a.group == 16 ? a.group : 32; }
+
 }  // namespace
 
 int ssa_warp_warps(const SsaArgs &a, size_t smem_limit) {
-    const WarpLayout l = warp_layout(a);
+    const WarpLayout l = warp_layout(a, group_of(a));
     if (l.block_bytes + l.warp_bytes > smem_limit) return 0;
     return (int)std::min<size_t>(a.batch ? kWarpMaxWarpsBatch : kWarpMaxWarps, (smem_limit - l.block_bytes) / l.warp_bytes);
 }
 
 size_t ssa_warp_smem(const SsaArgs &a, int warps) {
-    const WarpLayout l = warp_layout(a);
+    const WarpLayout l = warp_layout(a, group_of(a));
     return l.block_bytes + (size_t)warps * l.warp_bytes;
 }
 
 bool ssa_warp_supported(const SsaArgs &a, int max_order) {
-    return a.ex_off == nullptr && a.S < 65536 && max_order < 32768 && a.R >= 1;
+    return a.ex_off == nullptr && a.S < 65536 && a.R < 65536 && max_order < 32768 && a.R >= 1;
 }
 
-int ssa_warp_occupancy(const SsaArgs &a, int warps, size_t smem) {
-    int n = 0;
-    // the arithmetic variants share the block shape and shared memory use;
-    // batch launches have their own register budget
-    const auto k = a.batch ? ssa_warp_kernel<false, true> : ssa_warp_kernel<false, false>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 32 * warps, smem);
-    return n;
+// The group width with the shortest estimated launch: waves of resident
+// trajectories times a step's latency.  Measured latencies, relative to 32
+// lanes with a warp per scheduler (1.0 us on 40 species and 120 reactions and
+// on 200 x 1000): 16 lanes 1.18, 8 lanes 1.50 (two reactions a lane in the
+// walk, two rounds of 12 dependents), on 200 x 1000 1.47 and 2.63; 16 warps an
+// SM instead of 4 1.3 times that.  So 3000 trajectories of 40 x 120 run on 16
+// lanes (7.7 ms; 8 and 32 lanes 9 and 15 ms), 9728 on 8 (10.9 ms against 16.6),
+// and 200 x 1000, of which shared memory holds 17 trajectories an SM, on 32.
+//
+// A batch's trajectories part more often (networks of uneven size side by
+// side, a sample every few events) and its largest ones come first, so its
+// launch is rather n_traj / resident long: 16 lanes when there are 1.65 times as
+// many trajectories as 32 lanes hold at once (65 536 of the bench's random
+// networks: 32 / 16 / 8 lanes 71 / 59 / 68 ms, 4 608: 7.9 / 9.6 / 13.6 ms).
+int ssa_warp_group(const SsaArgs &a, int64_t n_traj, double mean_deps, size_t smem_limit, int sms) {
+    if (const char *e = std::getenv("RB_WARP_GROUP")) {
+        const int v = std::atoi(e);
+        if (v == 8 || v == 16 || v == 32) return a.batch && v == 8 ? 16 : v;
+    }
+    if (a.batch) {
+        SsaArgs b = a;
+        b.group = 32;
+        const int warps = ssa_warp_warps(b, smem_limit);
+        b.group = 16;
+        return warp_chunk(a.R, 16) <= 255 && ssa_warp_warps(b, smem_limit) >= 8 &&
+                       (double)n_traj > 1.65 * sms * warps ? 16 : 32;
+    }
+    int best = 32;
+    double best_t = 0.0;
+    for (int G : {32, 16, 8}) {
+        SsaArgs b = a;
+        b.group = G;
+        const int warps = ssa_warp_warps(b, smem_limit), C = warp_chunk(a.R, G);
+        if (warps < 1 || (G < 32 && C > 255)) continue;  // chunk sums within their words
+        const double side = 32.0 / G, per_wave = (double)sms * warps * side;
+        const double waves = std::max(1.0, std::ceil((double)n_traj / per_wave));
+        const double resident = std::min((double)warps, std::ceil((double)n_traj / (sms * side)));
+        const double lat = (1.0 + 0.17 * std::log2(side) + 0.05 * ((C + G - 1) / G - 1) +
+                            0.1 * std::max(0.0, mean_deps / G - 1.0)) * (1.0 + 0.3 * resident / 16.0);
+        if (best_t == 0.0 || waves * lat < best_t) {
+            best = G;
+            best_t = waves * lat;
+        }
+    }
+    return best;
 }
 
 int launch_ssa_warp(const SsaArgs &a, int warps, int grid, size_t smem, void *stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const bool batch = a.batch != nullptr;
-    if (a.macro_mode)
-        return batch ? warp_launch<true, true>(a, 32 * warps, grid, smem, st)
-                     : warp_launch<true, false>(a, 32 * warps, grid, smem, st);
-    return batch ? warp_launch<false, true>(a, 32 * warps, grid, smem, st)
-                 : warp_launch<false, false>(a, 32 * warps, grid, smem, st);
+    const int block = 32 * warps;
+    if (a.batch)
+        return a.group == 16 ? warp_launch<true, 16>(a, block, grid, smem, st)
+                             : warp_launch<true, 32>(a, block, grid, smem, st);
+    return a.group == 8    ? warp_launch<false, 8>(a, block, grid, smem, st)
+           : a.group == 16 ? warp_launch<false, 16>(a, block, grid, smem, st)
+                           : warp_launch<false, 32>(a, block, grid, smem, st);
 }
 
 uint32_t warp_shape_word(const int32_t *fac_sp, const int32_t *fac_ord, int P, int S, int r) {

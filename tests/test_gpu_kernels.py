@@ -54,3 +54,34 @@ def test_generated_kernel_of_17_to_32_reactions(rb, O, monkeypatch, S, R, seed, 
     assert res.stats["mapping"] == 4 and ev.max() > 20
     np.testing.assert_array_equal(res.counts, ref)
     np.testing.assert_array_equal(res.events, ev)
+
+
+# group width x network: one reaction a lane or several (C), in the walk through a chunk one, up
+# to four or more (E), lists longer than the group, an order-3 reaction (factor lists), networks
+# smaller than a group; a trajectory count that leaves groups of the last warp without work
+@pytest.mark.parametrize("G", [8, 16, 32])
+@pytest.mark.parametrize("S,R,seed,n,tmax", [(2, 2, 90, 37, 0.5), (9, 33, 91, 203, 2e-2), (12, 300, 92, 61, 2e-3),
+                                             (60, 1050, 93, 33, 1e-3), (6, 40, 94, 45, 1e-2)])
+def test_warp_kernel_group_widths(rb, O, monkeypatch, G, S, R, seed, n, tmax):
+    import bench
+
+    monkeypatch.setenv("RB_SSA_KERNEL", "warp")
+    monkeypatch.setenv("RB_WARP_GROUP", str(G))
+    reactions, x0 = bench.random_network(seed, S, R, x0_mean=60.0)
+    if seed == 94:
+        reactions[3] = (1e-4, [3] + [0] * (S - 1), [-1] + [0] * (S - 1))
+    net, onet = rb.Network(S), O.OracleNet(S)
+    for k, e, d in reactions:
+        net.add_reaction(rb.Rate.lma(k, e), d)
+        onet.add_lma(k, e, d)
+    rates = None
+    if seed == 91:  # per-trajectory rates, some trajectories exact throughout
+        rates = np.array([r[0] for r in reactions]) * 10.0 ** np.random.default_rng(seed).uniform(-1, 1, (n, R))
+        rates[::17, 2] = 1e-25
+    seeds = _seeds(n, seed)
+    res = net.run_ensemble(x0, seeds, tmax, 7, rates=rates, want_final=True)
+    ref, ev, _, _ = onet.run_ensemble(x0, seeds, tmax, 7, rates=rates)
+    assert res.stats["mapping"] == 5 and ev.max() > 10
+    np.testing.assert_array_equal(res.counts, ref)
+    np.testing.assert_array_equal(res.events, ev)
+    np.testing.assert_array_equal(res.final, ref[-1].T)
