@@ -148,7 +148,9 @@ for _name, _args in {
     "rbg_mdn_silu_backward": [_vp, _vp, _vp, _vp, C.c_int, C.c_int, _vp],
     "rbg_mdn_head_backward": [_vp, _vp, _vp, C.c_int, C.c_int, _vp],
     "rbg_mdn_loss": [_vp, _vp, C.c_int, C.c_int, _vp, _vp, _vp],
-    "rbg_mdn_adam": [_vp, _vp, _vp, _vp, _vp, C.c_int, _f32, _f32, _f32, _f32, C.c_int, _vp],
+    "rbg_mdn_adam_all": [P(_vp), P(_vp), P(_vp), P(_vp), P(_vp), P(C.c_int), C.c_int, _f32, _f32, _f32, _f32, C.c_int,
+                         _vp],
+    "rbg_mdn_count_grad": [_vp, _vp, C.c_int, C.c_int, _vp, _vp, P(_vp), P(_vp), _vp, _vp, _vp, _vp, _vp, _vp],
     "rbg_mdn_sample": [_vp, C.c_int, C.c_int, _u64, _vp, C.c_int, _vp, _vp],
     "rbg_mdn_rre": [_vp, _vp, C.c_int, C.c_int, C.c_int, _vp, _vp, _vp, C.c_int, _vp, C.c_int, _vp, _vp],
     "rbg_mdn_count_loss": [_vp, _vp, C.c_int, C.c_int, _vp, _vp, _vp],
@@ -158,6 +160,8 @@ for _name, _args in {
 }.items():
     getattr(lib, _name).argtypes = _args
     getattr(lib, _name).restype = C.c_int
+lib.rbg_mdn_count_grad_bytes.argtypes = [C.c_int, C.c_int]
+lib.rbg_mdn_count_grad_bytes.restype = _sz
 lib.rbg_internal_batch_times.argtypes = [_vp, P(C.c_float), P(C.c_float), P(C.c_float)]
 lib.rbg_internal_batch_times.restype = C.c_int
 lib.rbg_internal_jit_source.argtypes = [_vp, _cp, _sz]

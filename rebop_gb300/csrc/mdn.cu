@@ -22,23 +22,16 @@
 //     with respect to the head's raw outputs.
 //   * mdn_loss: the same for a K-component diagonal Gaussian mixture in two
 //     dimensions.
-//   * adam: FP32 master weights, BF16 copies refreshed in place.
 //   * rre: the reaction rate equations (RK4) at each query; an unrolled
 //     variant for networks of 4 species and 5 reactions.
 //   * mdn_sample / count_prep + count_draw: draws from each query's
 //     distribution.
-#include <cuda.h>
-#include <cudaTypedefs.h>
-#include <cuda_bf16.h>
-#include <cuda_runtime.h>
-
 #include <algorithm>
-#include <cstdint>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
-#include <utility>
-#include <vector>
+
+#include "mdn_tc.cuh"
 
 namespace rbg {
 
@@ -153,28 +146,11 @@ __global__ void __launch_bounds__(128) gemm_bf16_kernel(const __nv_bfloat16 *__r
 constexpr int kTcM = 128, kTcN = 32, kTcK = 64, kTcSlabs = 4;
 constexpr size_t kTcSmem = (size_t)kTcSlabs * (kTcM + kTcN) * kTcK * 2;  // 80 KB
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-
 // Shared-memory matrix descriptor: start >> 4, leading (K) byte offset >> 4,
 // stride (M/N) byte offset >> 4, descriptor version 1 (bits 46-48), no swizzle.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) |
            (1ull << 46);
-}
-
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-    for (int it = 0; it < (1 << 22); ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(mbar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
 }
 
 // Element index of (row r, k) of slab s in the canonical layout.
@@ -405,26 +381,6 @@ __global__ void split_reduce_kernel(const float *__restrict__ P, int splits, flo
 // iteration limit: one that runs out sets *err, no further copy or MMA is
 // issued, copies already issued are waited for (again with a limit), and
 // tensor memory is freed.
-constexpr int kTmM = 128, kTmN = 64, kTmK = 64, kTmStages = 4;
-constexpr int kTmABytes = kTmM * kTmK * 2, kTmBBytes = kTmN * kTmK * 2, kTmStage = kTmABytes + kTmBBytes;
-constexpr size_t kTmSmem = (size_t)kTmStages * kTmStage + 1024;  // + alignment slack to 1 KiB
-
-// Shared-memory descriptor of a K-major operand in the 128-byte swizzle:
-// stride between 8-row atoms 1024 B, leading offset unused (1), version 1,
-// layout type 2 (128-byte swizzle) in bits 61-63.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
-           (2ull << 61);
-}
-
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::
-            "r"(dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-}
-
 __global__ void __launch_bounds__(128) gemm_tma_kernel(const __grid_constant__ CUtensorMap tmA,
                                                        const __grid_constant__ CUtensorMap tmB, float *__restrict__ C,
                                                        int ldc, int M, int N, int K, float beta, int *err) {
@@ -552,8 +508,6 @@ __global__ void __launch_bounds__(128) gemm_tma_kernel(const __grid_constant__ C
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTmN));
 }
-
-__device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + __expf(-x)); }
 
 // ---------------------------------------------------------------- fused inference
 // The whole forward pass of the surrogate for 128 queries per tile, in one
@@ -871,8 +825,6 @@ __global__ void __launch_bounds__(kColX *kColY) head_backward_kernel(const float
     }
 }
 
-__device__ __forceinline__ float softplusf_(float x) { return x > 20.0f ? x : log1pf(__expf(x)); }
-
 // Head layout per row (K components): logits[K] | mu1[K] | mu2[K] | s1[K] | s2[K],
 // sigma = softplus(s) + 1e-3.  loss[row] = -log sum_k pi_k N(y1; mu1, s1) N(y2; mu2, s2);
 // G = d(mean loss)/d(raw head outputs).
@@ -921,8 +873,6 @@ __global__ void mdn_loss_kernel(const float *O, const float *Y, int B, int K, fl
 // (n_protein, n_dimer, y_protein, y_dimer).  loss[row] = sum_s -log P_s with
 // P_s = pi_c for a small count c, pi_tail * sum_k w_k N(y; mu_k, sigma_k) for
 // a tail count; G = d(mean loss)/d(raw head outputs).
-constexpr int kNC = 32, kKTMax = 16;
-
 __global__ void count_loss_kernel(const float *O, const float *Y, int B, int kKT, float *loss, float *G) {
     const int kHS = kNC + 3 * kKT;
     const int row = blockIdx.x * blockDim.x + threadIdx.x;
@@ -971,20 +921,6 @@ __global__ void count_loss_kernel(const float *O, const float *Y, int B, int kKT
         }
     }
     loss[row] = total;
-}
-
-__global__ void adam_kernel(float *w, __nv_bfloat16 *wb, const float *g, float *m, float *v, int n, float lr,
-                            float b1, float b2, float eps, float c1, float c2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.0f - b1) * gi;
-    const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    w[i] = wi;
-    if (wb) wb[i] = __float2bfloat16(wi);
 }
 
 __device__ __forceinline__ uint64_t mix64(uint64_t z) {
@@ -1357,22 +1293,6 @@ namespace {
 
 constexpr int kMaxDevices = 64;
 
-// Dynamic shared memory above 48 KB for `kern`, asked once per (kernel, device):
-// the attribute belongs to the current device's context.
-cudaError_t opt_in_smem(const void *kern, size_t bytes) {
-    static std::mutex mu;
-    static std::vector<std::pair<const void *, int>> done;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    std::lock_guard<std::mutex> lk(mu);
-    for (const auto &d : done)
-        if (d.first == kern && d.second == dev) return cudaSuccess;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) done.emplace_back(kern, dev);
-    return e;
-}
-
 // The TMA-fed kernel takes C = A B^T with both operands K-contiguous, rows
 // 16-byte multiples apart from a 16-byte aligned base (what a tensor map can
 // address) and K >= 8; RB_GEMM_TMA=0 sends every product to the staged kernel.
@@ -1381,29 +1301,6 @@ bool tma_gemm_ok(const void *A, int lda, int ta, const void *B, int ldb, int tb,
     const bool off = e && std::strcmp(e, "0") == 0;
     return !off && !ta && tb && K >= 8 && lda % 8 == 0 && ldb % 8 == 0 &&
            (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0;
-}
-
-// 2-D tensor map of a row-major BF16 matrix [rows][K] (row pitch ld elements)
-// read in boxes of 64 (K) x box_rows with the 128-byte swizzle; false if the
-// driver has no encoder or refuses the operands.
-bool encode_rows(CUtensorMap &map, const void *base, int rows, int K, int ld, int box_rows) {
-    static PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
-        void *fn = nullptr;
-        cudaDriverEntryPointQueryResult q{};
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) !=
-                cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            fn = nullptr;
-        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-    }();
-    if (!encode) return false;
-    const cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t stride[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)rbg::kTmK, (cuuint32_t)box_rows};
-    const cuuint32_t elem[2] = {1, 1};
-    return encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dim, stride, box, elem,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // Launch gemm_tma_kernel; returns a CUDA error code, or -1 when no tensor map
@@ -1541,14 +1438,6 @@ int rbg_mdn_head_backward(const float *G, void *Gb, float *db, int M, int N, voi
 int rbg_mdn_loss(const float *O, const float *Y, int B, int K, float *loss, float *G, void *stream) {
     if (K > 16) return (int)cudaErrorInvalidValue;
     rbg::mdn_loss_kernel<<<(B + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(O, Y, B, K, loss, G);
-    return (int)cudaGetLastError();
-}
-
-int rbg_mdn_adam(float *w, void *wb, const float *g, float *m, float *v, int n, float lr, float b1, float b2,
-                 float eps, int step, void *stream) {
-    const float c1 = 1.0f - powf(b1, (float)step), c2 = 1.0f - powf(b2, (float)step);
-    rbg::adam_kernel<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        w, static_cast<__nv_bfloat16 *>(wb), g, m, v, n, lr, b1, b2, eps, c1, c2);
     return (int)cudaGetLastError();
 }
 

@@ -1,0 +1,684 @@
+// Training pass of the surrogate with the count-aware head: loss and gradients
+// of every layer in 13 launches, all products on tcgen05.
+//
+//   prep       normalised inputs as BF16 (row-major and transposed), the hidden
+//              weights transposed (the input gradients' operand)
+//   forward    one product per layer; its drain adds the bias, keeps z in FP32
+//              and writes bf16(silu(z)) both row-major (the next product's
+//              operand) and transposed (the weight gradient's)
+//   loss       a warp per row: loss, the head's gradient as BF16 in both
+//              layouts, its column sums per block
+//   backward   one product per hidden layer; its drain multiplies by silu'(z)
+//              and writes the result as forward does, with column sums per tile
+//   weights    every layer's dW = dZ^T H in one launch, the batch (the K
+//              dimension) split over the grid
+//   reduce     dW and db from the partial sums, in a fixed order
+//
+// A separate elementwise pass over the FP32 products, column sums on 8 blocks
+// (4 x 123 us) and one launch per layer, split and bias cost 0.9 ms of GPU time
+// a step at a batch of 4096; transposing in the drain makes every operand of
+// every product contiguous along K, so all of them load by TMA.  Bound by
+// launches of a few microseconds each (5.6 GFLOP: 3 us at the measured BF16
+// rate; 40 MB of activations and partial sums: 6 us, in L2).  TRAIN_FIGURES
+//
+// Rounding is that of the layer-by-layer pass: FP32 products, z, gradients and
+// column sums, BF16 operands.
+#include <algorithm>
+
+#include "mdn_tc.cuh"
+
+namespace rbg {
+
+namespace {
+
+constexpr int kTrHid = 256, kTrIn = 8, kTrLayers = 5;
+
+// 128 x 64 tile of A B^T over the K slices [ks0, ks1) (64 wide each), in tensor
+// memory: the four-stage TMA ring of gemm_tma_kernel.  Thread 0 loads, thread
+// 32 issues the MMAs.  False (for every thread) when a wait ran out; copies in
+// flight have then landed.
+struct TileSync {
+    uint64_t full[kTmStages], empty[kTmStages], done;
+    uint32_t tmem_base;
+    int failed, issued;
+};
+
+__device__ __forceinline__ uint32_t tile_begin(TileSync &s) {
+    const int tid = threadIdx.x, warp = tid >> 5;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s.tmem_base)),
+                     "r"(kTmN));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+    }
+    if (tid == 0) {
+        for (int k = 0; k < kTmStages; ++k) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&s.full[k])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&s.empty[k])));
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&s.done)));
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        s.failed = 0;
+        s.issued = 0;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n");
+    return s.tmem_base;
+}
+
+__device__ __forceinline__ bool tile_product(TileSync &s, unsigned char *sm, uint32_t tmem, const CUtensorMap *ma,
+                                             const CUtensorMap *mb, int m0, int n0, int ks0, int ks1) {
+    const int tid = threadIdx.x, nk = ks1 - ks0;
+    volatile int *failed = &s.failed;
+    const uint32_t sbase = smem_u32(sm);
+    // idesc: F32 accumulator, BF16 A and B, both K-major, N >> 3, M >> 4
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTmN >> 3) << 17) |
+                           ((uint32_t)(kTmM >> 4) << 24);
+    if (tid == 0) {
+        for (int kb = 0; kb < nk && !*failed; ++kb) {
+            const int st = kb % kTmStages;
+            if (kb >= kTmStages && !mbar_wait(smem_u32(&s.empty[st]), (uint32_t)((kb / kTmStages - 1) & 1))) {
+                *failed = 1;
+                break;
+            }
+            const uint32_t fb = smem_u32(&s.full[st]);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb), "r"(kTmStage)
+                         : "memory");
+            const uint32_t dst = sbase + st * kTmStage;
+            tma_load_2d(dst, ma, (ks0 + kb) * kTmK, m0, fb);
+            tma_load_2d(dst + kTmABytes, mb, (ks0 + kb) * kTmK, n0, fb);
+            s.issued = kb + 1;
+        }
+    } else if (tid == 32) {
+        for (int kb = 0; kb < nk; ++kb) {
+            const int st = kb % kTmStages;
+            if (*failed || !mbar_wait(smem_u32(&s.full[st]), (uint32_t)((kb / kTmStages) & 1))) {
+                *failed = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;\n");
+            const uint32_t a_addr = sbase + st * kTmStage, b_addr = a_addr + kTmABytes;
+            for (int k = 0; k < kTmK / 16; ++k) {
+                const uint64_t ad = smem_desc_sw128(a_addr + k * 32), bd = smem_desc_sw128(b_addr + k * 32);
+                const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
+                asm volatile(
+                    "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+                    " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+                    "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                             smem_u32(&s.empty[st]))
+                         : "memory");
+        }
+        // the last commit: every MMA issued so far has completed when it fires
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                         smem_u32(&s.done))
+                     : "memory");
+    }
+    __syncwarp();
+    if (!mbar_wait(smem_u32(&s.done), 0u)) *failed = 1;
+    __syncthreads();
+    const bool ok = !*failed;
+    if (!ok && tid == 0)
+        for (int kb = max(0, s.issued - kTmStages); kb < s.issued; ++kb)
+            mbar_wait(smem_u32(&s.full[kb % kTmStages]), (uint32_t)((kb / kTmStages) & 1));
+    asm volatile("tcgen05.fence::after_thread_sync;\n");
+    return ok;
+}
+
+__device__ __forceinline__ void tile_end(uint32_t tmem) {
+    asm volatile("tcgen05.fence::before_thread_sync;\n");
+    __syncthreads();
+    if (threadIdx.x < 32)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTmN));
+}
+
+// 32 columns from c0 on of this thread's row of the tile: eight warps drain a
+// tile, warps w and w + 4 the two halves of the columns of lane quadrant w.
+__device__ __forceinline__ void tile_row(uint32_t tmem, int c0, float (&v)[32]) {
+#pragma unroll
+    for (int h = 0; h < 32; h += 16) {
+        uint32_t w[16];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+            : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]),
+              "=r"(w[8]), "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
+            : "r"(tmem + ((threadIdx.x & 96u) << 16) + (uint32_t)(c0 + h)));
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[h + j] = __uint_as_float(w[j]);
+    }
+}
+
+// One layer of the forward or backward pass: C tile = A B^T for A [M][K] and B
+// [N][K], K = 64 nk at most (the tensor maps zero-fill), drained as MODE says.
+enum { kFwdHidden, kFwdHead, kBwd };
+struct LayerArgs {
+    CUtensorMap a, b;
+    int M, N, nk;
+    const float *bias;        // forward [N]
+    float *z;                 // [M][N]: written (forward), read (backward)
+    __nv_bfloat16 *h, *ht;    // [M][N] (null: not wanted) and [N][ldt]
+    int ldt;
+    float *col;               // backward: column sums per row tile [tiles][N]
+    int *err;
+};
+
+template <int MODE>
+__global__ void __launch_bounds__(256) layer_kernel(const __grid_constant__ LayerArgs a) {
+    extern __shared__ unsigned char tr_raw[];
+    unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tr_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) TileSync sync;
+    __shared__ float part[4][kTmN];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m0 = blockIdx.y * kTmM, n0 = blockIdx.x * kTmN;
+    const uint32_t tmem = tile_begin(sync);
+    if (!tile_product(sync, sm, tmem, &a.a, &a.b, m0, n0, 0, a.nk)) {
+        if (tid == 0) atomicExch(a.err, 1);
+    } else {
+        // the operand stages are idle now: per warp a 32 x 33 transpose tile
+        float *tile = reinterpret_cast<float *>(sm) + warp * 32 * 33;
+        const int row0 = m0 + (warp & 3) * 32, rows = min(32, a.M - row0), row = row0 + lane;
+        const int c0 = (warp >> 2) * 32;
+        float v[32];
+        tile_row(tmem, c0, v);
+        const int n = n0 + c0 + lane;  // this lane's column in the coalesced passes
+        if (MODE == kBwd) {
+            // (all 32 loads in flight: one after the other they took 30 us)
+            float zr[32];
+#pragma unroll
+            for (int rr = 0; rr < 32; ++rr)
+                zr[rr] = rr < rows && n < a.N ? a.z[(size_t)(row0 + rr) * a.N + n] : 0.0f;
+#pragma unroll
+            for (int rr = 0; rr < 32; ++rr) tile[rr * 33 + lane] = zr[rr];
+            __syncwarp();
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            const int nj = n0 + c0 + j;
+            const bool in = nj < a.N && lane < rows;
+            if (MODE == kBwd) {
+                // dZ = dH silu'(z)
+                const float z = in ? tile[lane * 33 + j] : 0.0f, sg = sigmoidf_(z);
+                v[j] = in ? v[j] * sg * (1.0f + z * (1.0f - sg)) : 0.0f;
+            } else {
+                v[j] = in ? v[j] + a.bias[nj] : 0.0f;
+            }
+        }
+        if (MODE == kBwd) __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = v[j];
+        __syncwarp();
+        if (MODE == kBwd) {
+            float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int rr = 0; rr < 32; ++rr) s[rr & 3] += tile[rr * 33 + lane];
+            part[warp & 3][c0 + lane] = (s[0] + s[1]) + (s[2] + s[3]);
+        } else {
+#pragma unroll
+            for (int rr = 0; rr < 32; ++rr)
+                if (rr < rows && n < a.N) a.z[(size_t)(row0 + rr) * a.N + n] = tile[rr * 33 + lane];
+        }
+        if (MODE != kFwdHead) {
+            // BF16, transposed straight from the rows' registers ...
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                const int nj = n0 + c0 + j;
+                if (MODE == kFwdHidden) v[j] = v[j] * sigmoidf_(v[j]);
+                if (nj < a.N && lane < rows) a.ht[(size_t)nj * a.ldt + row] = __float2bfloat16(v[j]);
+            }
+            // ... and row-major through the tile
+            if (a.h) {
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = v[j];
+                __syncwarp();
+#pragma unroll
+                for (int rr = 0; rr < 32; ++rr)
+                    if (rr < rows && n < a.N) a.h[(size_t)(row0 + rr) * a.N + n] = __float2bfloat16(tile[rr * 33 + lane]);
+            }
+        }
+        if (MODE == kBwd) {
+            __syncthreads();
+            if (tid < kTmN && n0 + tid < a.N)
+                a.col[(size_t)blockIdx.y * a.N + n0 + tid] =
+                    ((part[0][tid] + part[1][tid]) + part[2][tid]) + part[3][tid];
+        }
+    }
+    tile_end(tmem);
+}
+
+// Weight gradients of every layer: tile `blockIdx.x` of the list (layer, m, n)
+// over the K slices of split blockIdx.y; partial sums to P[split][...].
+struct WeightArgs {
+    CUtensorMap a[kTrLayers], b[kTrLayers];  // dZ^T [out][B], H^T [in][B]
+    int out[kTrLayers], in[kTrLayers], off[kTrLayers], first[kTrLayers + 1];  // first tile of each layer
+    int slices, per_split, total;
+    float *P;
+    int *err;
+};
+
+__global__ void __launch_bounds__(256) weight_kernel(const __grid_constant__ WeightArgs a) {
+    extern __shared__ unsigned char tr_raw[];
+    unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tr_raw) + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) TileSync sync;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    int l = 0;
+    while (l + 1 < kTrLayers && (int)blockIdx.x >= a.first[l + 1]) ++l;
+    const int nt = (a.in[l] + kTmN - 1) / kTmN, t = (int)blockIdx.x - a.first[l];
+    const int m0 = (t / nt) * kTmM, n0 = (t % nt) * kTmN, M = a.out[l], N = a.in[l];
+    const int ks0 = blockIdx.y * a.per_split, ks1 = min(a.slices, ks0 + a.per_split);
+    const uint32_t tmem = tile_begin(sync);
+    if (!tile_product(sync, sm, tmem, &a.a[l], &a.b[l], m0, n0, ks0, ks1)) {
+        if (tid == 0) atomicExch(a.err, 1);
+    } else {
+        float *tile = reinterpret_cast<float *>(sm) + warp * 32 * 33;
+        float *P = a.P + (size_t)blockIdx.y * a.total + a.off[l];
+        const int row0 = m0 + (warp & 3) * 32, rows = min(32, M - row0), c0 = (warp >> 2) * 32, n = n0 + c0 + lane;
+        float v[32];
+        tile_row(tmem, c0, v);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = v[j];
+        __syncwarp();
+#pragma unroll
+        for (int rr = 0; rr < 32; ++rr)
+            if (rr < rows && n < N) P[(size_t)(row0 + rr) * N + n] = tile[rr * 33 + lane];
+    }
+    tile_end(tmem);
+}
+
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, d));
+    return v;
+}
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    return v;
+}
+
+// dW[e] = sum over splits of P[s][e] for the `total` weights, then db[n] = sum
+// over row tiles of the column sums (the head's per loss block), both in order.
+struct ReduceArgs {
+    const float *P;
+    float *dW, *db;
+    int total, splits;
+    const float *col[kTrLayers];
+    int n[kTrLayers], tiles[kTrLayers];
+};
+
+__global__ void __launch_bounds__(256) reduce_kernel(const __grid_constant__ ReduceArgs a) {
+    const int w_blocks = (a.total + 255) / 256;
+    if ((int)blockIdx.x < w_blocks) {
+        const int e = blockIdx.x * 256 + threadIdx.x;
+        if (e >= a.total) return;
+        float s = 0.0f;
+#pragma unroll 8
+        for (int k = 0; k < a.splits; ++k) s += a.P[(size_t)k * a.total + e];
+        a.dW[e] = s;
+        return;
+    }
+    // a warp per bias: its lanes walk the tiles, then a fixed tree
+    int e = ((int)blockIdx.x - w_blocks) * 8 + (threadIdx.x >> 5);
+    const int out = e, lane = threadIdx.x & 31;
+    for (int l = 0; l < kTrLayers; ++l) {
+        if (e < a.n[l]) {
+            float s = 0.0f;
+            for (int k = lane; k < a.tiles[l]; k += 32) s += a.col[l][(size_t)k * a.n[l] + e];
+            s = warp_sum(s);
+            if (lane == 0) a.db[out] = s;
+            return;
+        }
+        e -= a.n[l];
+    }
+}
+
+// Inputs: H0 = bf16((x - mean) / std) row-major [B][8] and transposed [8][ldt];
+// the hidden and head weights transposed: wt[l] [in][out] from w[l] [out][in].
+struct PrepArgs {
+    const float *x, *mean, *std;
+    __nv_bfloat16 *h, *ht;
+    int B, ldt;
+    const __nv_bfloat16 *w[kTrLayers - 1];
+    __nv_bfloat16 *wt[kTrLayers - 1];
+    int out[kTrLayers - 1];
+    int x_blocks;
+};
+
+__global__ void __launch_bounds__(256) prep_kernel(const __grid_constant__ PrepArgs a) {
+    const int tid = threadIdx.x;
+    int b = blockIdx.x;
+    if (b < a.x_blocks) {
+        const int r = b * 256 + tid;
+        if (r >= a.B) return;
+#pragma unroll
+        for (int j = 0; j < kTrIn; ++j) {
+            const __nv_bfloat16 v = __float2bfloat16((a.x[(size_t)r * kTrIn + j] - a.mean[j]) / a.std[j]);
+            a.h[(size_t)r * kTrIn + j] = v;
+            a.ht[(size_t)j * a.ldt + r] = v;
+        }
+        return;
+    }
+    // 32 x 32 tiles of the weights
+    __shared__ __nv_bfloat16 tile[32][34];
+    b -= a.x_blocks;
+    int l = 0;
+    while (b >= (kTrHid / 32) * ((a.out[l] + 31) / 32)) {
+        b -= (kTrHid / 32) * ((a.out[l] + 31) / 32);
+        ++l;
+    }
+    const int i0 = (b % (kTrHid / 32)) * 32, o0 = (b / (kTrHid / 32)) * 32, x = tid & 31;
+    const int ldw = (a.out[l] + 7) & ~7;  // 16-byte row pitch
+    for (int y = tid >> 5; y < 32; y += 8)
+        if (o0 + y < a.out[l]) tile[y][x] = a.w[l][(size_t)(o0 + y) * kTrHid + i0 + x];
+    __syncthreads();
+    for (int y = tid >> 5; y < 32; y += 8)
+        if (o0 + x < a.out[l]) a.wt[l][(size_t)(i0 + y) * ldw + o0 + x] = tile[x][y];
+}
+
+// Loss and head gradient (the formulas of count_loss_kernel) with a warp per
+// row: lane k holds class k's logit, lanes below KT the tail components.  A
+// block takes 16 rows; their gradients pass through shared memory to be written
+// as BF16 row-major [B][ldg] and transposed [n_out][ldt], with the block's
+// column sums (FP32) beside them.  (A thread per row took 28 us at 4096 rows.)
+constexpr int kLossRows = 16;
+struct LossArgs {
+    const float *O, *Y;
+    int B, KT, ldg, ldt;
+    float *loss;
+    __nv_bfloat16 *g, *gt;
+    float *col;
+};
+
+__global__ void __launch_bounds__(512) loss_rows_kernel(const __grid_constant__ LossArgs a) {
+    const int HS = kNC + 3 * a.KT, N = 2 * HS;
+    extern __shared__ float ls_tile[];  // [16][N + 1]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r0 = blockIdx.x * kLossRows;
+    const float inv_b = 1.0f / (float)a.B;
+    for (int rr = warp; rr < kLossRows; rr += 16) {
+        const int row = r0 + rr;
+        float *gr = ls_tile + rr * (N + 1);
+        if (row >= a.B) {
+            for (int k = lane; k < N; k += 32) gr[k] = 0.0f;
+            continue;
+        }
+        float total = 0.0f;
+        for (int sp = 0; sp < 2; ++sp) {
+            const float *o = a.O + (size_t)row * N + sp * HS;
+            float *g = gr + sp * HS;
+            const float n = a.Y[4 * (size_t)row + sp], y = a.Y[4 * (size_t)row + 2 + sp];
+            const int c = n < (float)(kNC - 1) ? (int)n : kNC - 1;
+            const float lg = o[lane];
+            const float lmax = warp_max(lg);
+            const float logz = lmax + logf(warp_sum(__expf(lg - lmax)));
+            total += logz - __shfl_sync(0xffffffffu, lg, c & 31);
+            g[lane] = (__expf(lg - logz) - (lane == c ? 1.0f : 0.0f)) * inv_b;
+            const bool t = lane < a.KT;
+            if (c < kNC - 1) {
+                if (t) g[kNC + lane] = g[kNC + a.KT + lane] = g[kNC + 2 * a.KT + lane] = 0.0f;
+                continue;
+            }
+            const float tw = t ? o[kNC + lane] : -1e30f, tm = t ? o[kNC + a.KT + lane] : 0.0f;
+            const float ts = t ? o[kNC + 2 * a.KT + lane] : 0.0f;
+            const float wmax = warp_max(tw);
+            const float logw = wmax + logf(warp_sum(t ? __expf(tw - wmax) : 0.0f));
+            const float sg = softplusf_(ts) + 1e-3f, e = (y - tm) / sg;
+            const float lp = t ? (tw - logw) - 0.5f * e * e - logf(sg) - 0.9189385332f : -1e30f;
+            const float mx = warp_max(lp);
+            const float ll = mx + logf(warp_sum(t ? __expf(lp - mx) : 0.0f));
+            total -= ll;
+            if (t) {
+                const float r = __expf(lp - ll), w = __expf(tw - logw);
+                g[kNC + lane] = (w - r) * inv_b;
+                g[kNC + a.KT + lane] = -r * e / sg * inv_b;
+                g[kNC + 2 * a.KT + lane] = r * (1.0f - e * e) / sg * sigmoidf_(ts) * inv_b;
+            }
+        }
+        if (lane == 0) a.loss[row] = total;
+    }
+    __syncthreads();
+    const int rows = min(kLossRows, a.B - r0);
+    for (int rr = warp; rr < rows; rr += 16)
+        for (int k = lane; k < N; k += 32) a.g[(size_t)(r0 + rr) * a.ldg + k] = __float2bfloat16(ls_tile[rr * (N + 1) + k]);
+    for (int e = threadIdx.x; e < kLossRows * N; e += 512) {
+        const int k = e / kLossRows, rr = e % kLossRows;
+        if (rr < rows) a.gt[(size_t)k * a.ldt + r0 + rr] = __float2bfloat16(ls_tile[rr * (N + 1) + k]);
+    }
+    for (int k = threadIdx.x; k < N; k += 512) {
+        float s = 0.0f;
+#pragma unroll
+        for (int rr = 0; rr < kLossRows; ++rr) s += ls_tile[rr * (N + 1) + k];
+        a.col[(size_t)blockIdx.x * N + k] = s;
+    }
+}
+
+// Adam on every tensor of the model in one launch (adam_kernel's update).
+struct AdamArgs {
+    float *w[2 * kTrLayers], *m[2 * kTrLayers], *v[2 * kTrLayers];
+    const float *g[2 * kTrLayers];
+    __nv_bfloat16 *wb[2 * kTrLayers];  // null: no BF16 copy
+    int first[2 * kTrLayers + 1];
+    int n_tensors;
+    float lr, b1, b2, eps, c1, c2;
+};
+
+__global__ void __launch_bounds__(256) adam_all_kernel(const __grid_constant__ AdamArgs a) {
+    const int e = blockIdx.x * 256 + threadIdx.x;
+    if (e >= a.first[a.n_tensors]) return;
+    int t = 0;
+    while (e >= a.first[t + 1]) ++t;
+    const int i = e - a.first[t];
+    const float gi = a.g[t][i];
+    const float mi = a.b1 * a.m[t][i] + (1.0f - a.b1) * gi;
+    const float vi = a.b2 * a.v[t][i] + (1.0f - a.b2) * gi * gi;
+    a.m[t][i] = mi;
+    a.v[t][i] = vi;
+    const float wi = a.w[t][i] - a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps);
+    a.w[t][i] = wi;
+    if (a.wb[t]) a.wb[t][i] = __float2bfloat16(wi);
+}
+
+// The training pass's workspace: offsets from its start, 256-byte aligned.
+struct Workspace {
+    size_t h[kTrLayers], ht[kTrLayers], z[kTrLayers], d[kTrLayers], dt[kTrLayers], wt[kTrLayers], col[kTrLayers], P,
+        bytes;
+    int ldt, tiles, loss_blocks, splits, per_split, slices, total;
+};
+
+Workspace layout(int B, int n_out) {
+    Workspace w{};
+    size_t off = 0;
+    auto take = [&](size_t n) {
+        const size_t o = off;
+        off = (off + n + 255) & ~(size_t)255;
+        return o;
+    };
+    w.ldt = (B + 7) & ~7;
+    w.tiles = (B + kTmM - 1) / kTmM;
+    w.loss_blocks = (B + kLossRows - 1) / kLossRows;
+    // the batch in slices of 64, eight a split (30 tiles of the five layers x 8
+    // splits at 4096 rows: 240 blocks), at most 32 splits
+    w.slices = (B + kTmK - 1) / kTmK;
+    w.per_split = std::max(8, (w.slices + 31) / 32);
+    w.splits = (w.slices + w.per_split - 1) / w.per_split;
+    w.total = kTrHid * kTrIn + 3 * kTrHid * kTrHid + n_out * kTrHid;
+    for (int l = 0; l < kTrLayers; ++l) {
+        const int in = l == 0 ? kTrIn : kTrHid, out = l == kTrLayers - 1 ? n_out : kTrHid;
+        const size_t ld = (size_t)((out + 7) & ~7);
+        w.h[l] = take(2 * (size_t)B * in);
+        w.ht[l] = take(2 * (size_t)in * w.ldt);
+        w.z[l] = take(4 * (size_t)B * out);
+        w.d[l] = take(2 * (size_t)B * ld);
+        w.dt[l] = take(2 * (size_t)out * w.ldt);
+        w.wt[l] = l ? take(2 * (size_t)kTrHid * ld) : 0;
+        w.col[l] = take(4 * (size_t)(l == kTrLayers - 1 ? w.loss_blocks : w.tiles) * out);
+    }
+    w.P = take(4 * (size_t)w.splits * w.total);
+    w.bytes = off;
+    return w;
+}
+
+}  // namespace
+
+}  // namespace rbg
+
+extern "C" {
+
+// Bytes of workspace rbg_mdn_count_grad needs.
+size_t rbg_mdn_count_grad_bytes(int B, int n_out) { return rbg::layout(B, n_out).bytes; }
+
+// Loss rows and the gradients of every layer of the surrogate (8 -> 4 x 256 ->
+// 2 (32 + 3 KT), count-aware head): X [B][8] raw features, Y [B][4]; W: five
+// BF16 weights [out][in], b: five FP32 biases; loss [B]; dW: the five weight
+// gradients one after the other, db: the biases'; work: 256-byte aligned.
+// Device pointers; W and b are host arrays of them.  Returns a CUDA error code
+// (cudaErrorNotSupported: no tensor-map encoder; nothing was launched).
+int rbg_mdn_count_grad(const float *X, const float *Y, int B, int KT, const float *x_mean, const float *x_std,
+                       const void *const *W, const float *const *b, float *loss, float *dW, float *db, void *work,
+                       int *err, void *stream) {
+    using namespace rbg;
+    if (B < 1 || KT < 1 || KT > kKTMax) return (int)cudaErrorInvalidValue;
+    const int n_out = 2 * (kNC + 3 * KT);
+    const Workspace w = layout(B, n_out);
+    unsigned char *base = static_cast<unsigned char *>(work);
+    auto bf = [&](size_t o) { return reinterpret_cast<__nv_bfloat16 *>(base + o); };
+    auto fl = [&](size_t o) { return reinterpret_cast<float *>(base + o); };
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    auto in_of = [](int l) { return l == 0 ? kTrIn : kTrHid; };
+    auto out_of = [&](int l) { return l == kTrLayers - 1 ? n_out : kTrHid; };
+    auto pitch = [&](int l) { return (out_of(l) + 7) & ~7; };
+    for (int l = 0; l < kTrLayers; ++l)
+        if (reinterpret_cast<uintptr_t>(W[l]) & 15) return (int)cudaErrorInvalidValue;
+
+    // ---- every tensor map before the first launch
+    LayerArgs fwd[kTrLayers], bwd[kTrLayers];
+    WeightArgs wa{};
+    bool ok = true;
+    for (int l = 0; l < kTrLayers; ++l) {
+        const int in = in_of(l), out = out_of(l);
+        LayerArgs &f = fwd[l];
+        f = LayerArgs{};
+        ok = ok && encode_rows(f.a, bf(w.h[l]), B, in, in, kTmM) && encode_rows(f.b, W[l], out, in, in, kTmN);
+        f.M = B;
+        f.N = out;
+        f.nk = (in + kTmK - 1) / kTmK;
+        f.bias = b[l];
+        f.z = fl(w.z[l]);
+        f.h = l + 1 < kTrLayers ? bf(w.h[l + 1]) : nullptr;
+        f.ht = l + 1 < kTrLayers ? bf(w.ht[l + 1]) : nullptr;
+        f.ldt = w.ldt;
+        f.err = err;
+        if (l > 0) {  // dZ of layer l - 1 from dZ of layer l
+            LayerArgs &g = bwd[l];
+            g = LayerArgs{};
+            ok = ok && encode_rows(g.a, bf(w.d[l]), B, out, pitch(l), kTmM) &&
+                 encode_rows(g.b, bf(w.wt[l]), kTrHid, out, pitch(l), kTmN);
+            g.M = B;
+            g.N = kTrHid;
+            g.nk = (out + kTmK - 1) / kTmK;
+            g.z = fl(w.z[l - 1]);
+            g.h = l > 1 ? bf(w.d[l - 1]) : nullptr;
+            g.ht = bf(w.dt[l - 1]);
+            g.ldt = w.ldt;
+            g.col = fl(w.col[l - 1]);
+            g.err = err;
+        }
+        ok = ok && encode_rows(wa.a[l], bf(w.dt[l]), out, B, w.ldt, kTmM) &&
+             encode_rows(wa.b[l], bf(w.ht[l]), in, B, w.ldt, kTmN);
+        wa.out[l] = out;
+        wa.in[l] = in;
+        wa.off[l] = l == 0 ? 0 : wa.off[l - 1] + wa.out[l - 1] * wa.in[l - 1];
+        wa.first[l + 1] = wa.first[l] + ((out + kTmM - 1) / kTmM) * ((in + kTmN - 1) / kTmN);
+    }
+    if (!ok) return (int)cudaErrorNotSupported;
+    for (const void *k : {reinterpret_cast<const void *>(layer_kernel<kFwdHidden>),
+                          reinterpret_cast<const void *>(layer_kernel<kFwdHead>),
+                          reinterpret_cast<const void *>(layer_kernel<kBwd>),
+                          reinterpret_cast<const void *>(weight_kernel)}) {
+        const cudaError_t e = opt_in_smem(k, kTmSmem);
+        if (e != cudaSuccess) return (int)e;
+    }
+
+    // ---- inputs and transposed weights
+    PrepArgs p{};
+    p.x = X;
+    p.mean = x_mean;
+    p.std = x_std;
+    p.h = bf(w.h[0]);
+    p.ht = bf(w.ht[0]);
+    p.B = B;
+    p.ldt = w.ldt;
+    p.x_blocks = (B + 255) / 256;
+    int blocks = p.x_blocks;
+    for (int l = 1; l < kTrLayers; ++l) {
+        p.w[l - 1] = static_cast<const __nv_bfloat16 *>(W[l]);
+        p.wt[l - 1] = bf(w.wt[l]);
+        p.out[l - 1] = out_of(l);
+        blocks += (kTrHid / 32) * ((out_of(l) + 31) / 32);
+    }
+    prep_kernel<<<blocks, 256, 0, st>>>(p);
+    // ---- forward
+    for (int l = 0; l < kTrLayers; ++l) {
+        const dim3 grid((out_of(l) + kTmN - 1) / kTmN, w.tiles);
+        if (l + 1 < kTrLayers) layer_kernel<kFwdHidden><<<grid, 256, kTmSmem, st>>>(fwd[l]);
+        else layer_kernel<kFwdHead><<<grid, 256, kTmSmem, st>>>(fwd[l]);
+    }
+    // ---- loss and the head's gradient
+    const int L = kTrLayers - 1;
+    LossArgs la{fl(w.z[L]), Y, B, KT, pitch(L), w.ldt, loss, bf(w.d[L]), bf(w.dt[L]), fl(w.col[L])};
+    loss_rows_kernel<<<w.loss_blocks, 512, 4 * (size_t)kLossRows * (n_out + 1), st>>>(la);
+    // ---- backward
+    for (int l = L; l > 0; --l) layer_kernel<kBwd><<<dim3(kTrHid / kTmN, w.tiles), 256, kTmSmem, st>>>(bwd[l]);
+    // ---- weight gradients, reductions
+    wa.slices = w.slices;
+    wa.per_split = w.per_split;
+    wa.total = w.total;
+    wa.P = fl(w.P);
+    wa.err = err;
+    weight_kernel<<<dim3(wa.first[kTrLayers], w.splits), 256, kTmSmem, st>>>(wa);
+    ReduceArgs ra{};
+    ra.P = wa.P;
+    ra.dW = dW;
+    ra.db = db;
+    ra.total = w.total;
+    ra.splits = w.splits;
+    int n_b = 0;
+    for (int l = 0; l < kTrLayers; ++l) {
+        ra.col[l] = fl(w.col[l]);
+        ra.n[l] = out_of(l);
+        ra.tiles[l] = l == L ? w.loss_blocks : w.tiles;
+        n_b += out_of(l);
+    }
+    reduce_kernel<<<(w.total + 255) / 256 + (n_b + 7) / 8, 256, 0, st>>>(ra);
+    return (int)cudaGetLastError();
+}
+
+// Adam on n tensors (at most 10) at once: host arrays of device pointers (wb[i]
+// null: no BF16 copy) and lengths.
+int rbg_mdn_adam_all(float *const *w, void *const *wb, const float *const *g, float *const *m, float *const *v,
+                     const int *n, int n_tensors, float lr, float b1, float b2, float eps, int step, void *stream) {
+    using namespace rbg;
+    if (n_tensors < 1 || n_tensors > 2 * kTrLayers) return (int)cudaErrorInvalidValue;
+    AdamArgs a{};
+    for (int t = 0; t < n_tensors; ++t) {
+        a.w[t] = w[t];
+        a.m[t] = m[t];
+        a.v[t] = v[t];
+        a.g[t] = g[t];
+        a.wb[t] = static_cast<__nv_bfloat16 *>(wb[t]);
+        a.first[t + 1] = a.first[t] + n[t];
+    }
+    a.n_tensors = n_tensors;
+    a.lr = lr;
+    a.b1 = b1;
+    a.b2 = b2;
+    a.eps = eps;
+    a.c1 = 1.0f - powf(b1, (float)step);
+    a.c2 = 1.0f - powf(b2, (float)step);
+    adam_all_kernel<<<(a.first[n_tensors] + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+    return (int)cudaGetLastError();
+}
+
+}  // extern "C"

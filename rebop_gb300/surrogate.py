@@ -28,6 +28,8 @@ fallback for the rest all come from the SSA engine itself.
 
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 
 from ._lib import check, lib
@@ -129,6 +131,11 @@ def generate(n_traj: int, seed: int, nb_steps: int = 100, net=None, per_traj: in
     return x, y, b.astype(np.float32)
 
 
+def _ptrs(tensors):
+    """C array of the tensors' device addresses (None: null)."""
+    return (C.c_void_p * len(tensors))(*[None if t is None else t.data_ptr() for t in tensors])
+
+
 class MDN:
     """The surrogate network; see the module docstring."""
 
@@ -208,6 +215,9 @@ class MDN:
         """Mean negative log-likelihood and the gradients (dW, db) of every layer."""
         torch = self.torch
         B = x.shape[0]
+        fused = self._count_grad(x, y)
+        if fused is not None:
+            return fused
         o = self.forward(x)
         loss = torch.empty(B, dtype=torch.float32, device=self.dev)
         G = torch.empty_like(o)
@@ -243,16 +253,41 @@ class MDN:
             d = dz
         return loss.mean(), dW, db
 
+    def _count_grad(self, x, y):
+        """loss_and_grad of the count-aware head in one native call
+        (``rbg_mdn_count_grad``: 13 launches, activations kept in one
+        workspace); None for what it does not cover (other heads or layer sizes,
+        RB_GEMM=mma, inputs that are not contiguous FP32 on the GPU)."""
+        torch = self.torch
+        B = x.shape[0]
+        if (self.head != "count" or not self.use_tc05 or LAYERS != 4 or HIDDEN != 256 or N_IN != 8 or B < 1
+                or any(t.dtype != torch.float32 or not t.is_contiguous() or not t.is_cuda
+                       for t in (x, y, self.x_mean, self.x_std))
+                or tuple(x.shape) != (B, N_IN) or tuple(y.shape) != (B, 4)
+                or self.x_mean.numel() != N_IN or self.x_std.numel() != N_IN):
+            return None
+        sizes = [w.numel() for w in self.W]
+        flat = torch.empty(sum(sizes) + sum(b.numel() for b in self.b), dtype=torch.float32, device=self.dev)
+        loss = torch.empty(B, dtype=torch.float32, device=self.dev)
+        work = torch.empty(lib.rbg_mdn_count_grad_bytes(B, self.n_out), dtype=torch.uint8, device=self.dev)
+        rc = lib.rbg_mdn_count_grad(x.data_ptr(), y.data_ptr(), B, self.tail, self.x_mean.data_ptr(),
+                                    self.x_std.data_ptr(), _ptrs(self.Wb), _ptrs(self.b), loss.data_ptr(),
+                                    flat.data_ptr(), flat.data_ptr() + 4 * sum(sizes), work.data_ptr(),
+                                    self.tc_err.data_ptr(), self._s())
+        if rc == 801:  # cudaErrorNotSupported: no tensor maps here, nothing was launched
+            return None
+        check(rc)
+        parts = flat.split(sizes + [b.numel() for b in self.b])
+        n = len(self.W)
+        return loss.mean(), [g.view_as(w) for g, w in zip(parts, self.W)], list(parts[n:])
+
     def train_step(self, x, y, lr: float):
         loss, dW, db = self.loss_and_grad(x, y)
         self.step += 1
-        for i in range(len(self.W)):
-            check(lib.rbg_mdn_adam(self.W[i].data_ptr(), self.Wb[i].data_ptr(), dW[i].data_ptr(),
-                                   self.mW[i].data_ptr(), self.vW[i].data_ptr(), self.W[i].numel(), lr, 0.9, 0.999,
-                                   1e-8, self.step, self._s()))
-            check(lib.rbg_mdn_adam(self.b[i].data_ptr(), None, db[i].data_ptr(), self.mb[i].data_ptr(),
-                                   self.vb[i].data_ptr(), self.b[i].numel(), lr, 0.9, 0.999, 1e-8, self.step,
-                                   self._s()))
+        w, n = self.W + self.b, len(self.W)
+        check(lib.rbg_mdn_adam_all(_ptrs(w), _ptrs(self.Wb + [None] * n), _ptrs(dW + db), _ptrs(self.mW + self.mb),
+                                   _ptrs(self.vW + self.vb), (C.c_int * len(w))(*[t.numel() for t in w]), len(w), lr,
+                                   0.9, 0.999, 1e-8, self.step, self._s()))
         return loss
 
     def fit(self, x, y, epochs: int = 20, batch: int = 4096, lr: float = 2e-3, seed: int = 0, log=None):

@@ -85,3 +85,36 @@ def test_warp_kernel_group_widths(rb, O, monkeypatch, G, S, R, seed, n, tmax):
     np.testing.assert_array_equal(res.counts, ref)
     np.testing.assert_array_equal(res.events, ev)
     np.testing.assert_array_equal(res.final, ref[-1].T)
+
+
+# batches at the edges of the row tiles (128), of the loss blocks (32), of the weight gradients' K
+# slices (64) and splits (8 slices, more with 32 splits); heads whose width is no multiple of 8
+@pytest.mark.parametrize("B,tail", [(1, 8), (31, 5), (64, 16), (129, 8), (513, 1), (4096, 8), (16_500, 4)])
+def test_count_gradients_match_oracle(rb, B, tail):
+    import torch
+    from oracle import mdn_oracle
+    from rebop_gb300 import surrogate as sg
+
+    rng = np.random.default_rng(B)
+    model = sg.MDN(seed=3, tail=tail)
+    x = rng.uniform(-1, 1, size=(B, sg.N_IN)).astype(np.float32)
+    x[:, 5] = rng.uniform(0, 1, B)
+    x[:, 6:] = rng.uniform(0, 8, (B, 2))
+    n = np.where(rng.random((B, 2)) < 0.5, rng.integers(0, 31, (B, 2)), rng.integers(31, 5000, (B, 2)))
+    y = np.concatenate([n, rng.normal(0.0, 0.3, size=(B, 2))], axis=1).astype(np.float32)
+    model.x_mean = torch.tensor([0, 0, 0, 0, 0, 0.5, 4.0, 4.0], device="cuda")
+    model.x_std = torch.tensor([0.6] * 5 + [0.3, 2.3, 2.3], device="cuda")
+    for b in model.b:
+        b.copy_(torch.tensor(rng.normal(0, 0.1, b.shape), dtype=torch.float32))
+    loss, dW, db = model.loss_and_grad(torch.tensor(x).cuda(), torch.tensor(y).cuda())
+    model.check_errors()
+    W = [w.double().cpu().numpy() for w in model.Wb]
+    b = [v.double().cpu().numpy() for v in model.b]
+    rl, rW, rb_ = mdn_oracle.forward_backward(W, b, x.astype(np.float64), y.astype(np.float64),
+                                              model.x_mean.double().cpu().numpy(), model.x_std.double().cpu().numpy(),
+                                              head="count", tail=tail)
+    assert abs(float(loss) - rl) <= 1e-3 * abs(rl) + 1e-4
+    # BF16 operands round by 2^-9 each: a few layers of them stay below 2e-2 in norm
+    for g, r in list(zip(dW, rW)) + list(zip(db, rb_)):
+        g = g.double().cpu().numpy()
+        assert g.shape == r.shape and np.linalg.norm(g - r) <= 2e-2 * np.linalg.norm(r) + 1e-7
