@@ -6,6 +6,7 @@ importing this module raises.  There is no CPU fallback.
 
 from __future__ import annotations
 
+import atexit
 import ctypes as C
 import shutil
 
@@ -168,6 +169,10 @@ lib.rbg_internal_jit_source.argtypes = [_vp, _cp, _sz]
 lib.rbg_internal_jit_source.restype = C.c_int
 lib.rbg_internal_jit_compile.argtypes = [_vp, P(_u64)]
 lib.rbg_internal_jit_compile.restype = C.c_int
+lib.rbg_internal_jit_wait.argtypes = []
+lib.rbg_internal_jit_wait.restype = None
+# a background compilation must not outlive the interpreter's shutdown
+atexit.register(lib.rbg_internal_jit_wait)
 lib.rbg_internal_warp_dep_table.argtypes = [_vp, P(C.c_uint16), _sz]
 lib.rbg_internal_warp_dep_table.restype = C.c_int
 

@@ -315,6 +315,10 @@ class Network:
         x0 = _i64a(x0)
         save_arr, n_save = self._save(save)
         NS = self.nb_species if n_save < 0 else n_save
+        # room for the records of an ordinary run at once (32 MB of them at
+        # most; rows that no event fills are never touched): a run that does not
+        # fit is simulated again with room for all
+        cap = max(int(cap), min(65_536, (1 << 25) // (8 * (1 + NS))))
         while True:
             times = np.empty(cap, dtype=np.float64)
             out = np.empty((cap, NS), dtype=np.int64)

@@ -182,6 +182,7 @@ int events_run(const rbg::Network &net, int64_t *species, double *t, uint64_t *r
     a.gate = gate;
     a.max_steps = max_steps;
     a.record_initial = record_initial;
+    a.keep_state = gate == 0;  // rb_run_all_events (gate = 1) wants the records alone
     a.save_idx = reinterpret_cast<int32_t *>(b + o_save);
     a.n_save = (int32_t)NS;
     a.cap = (int64_t)K;
@@ -715,6 +716,9 @@ int rbg_internal_jit_source(const rb_network *net, char *buf, size_t len) {
     if (!rbg::jit_supported(p)) return fail(RB_ERR_UNSUPPORTED, "network not covered by the generator");
     return copy_name(rbg::jit_net_source(p, rbg::jit_block()), buf, len);
 }
+
+// Wait for background compilations (the Python package calls it at exit).
+void rbg_internal_jit_wait(void) { rbg::jit_wait(); }
 
 // The warp kernel's dependency lists for the network: row j of out ([R][32],
 // cap entries in all) holds the number of reactions reaction j's jump touches,

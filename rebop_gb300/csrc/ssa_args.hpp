@@ -183,8 +183,8 @@ int launch_ssa_warp(const SsaArgs &a, int warps, int grid, size_t smem, void *st
 uint32_t warp_shape_word(const int32_t *fac_sp, const int32_t *fac_ord, int P, int S, int r);
 
 // Every-event runs (src/pyo3_gillespie.rs:209-223) and single
-// _advance_one_reaction steps (src/gillespie.rs:269-297): one thread per
-// trajectory, state in place in global memory.
+// _advance_one_reaction steps (src/gillespie.rs:269-297): a block per
+// trajectory.
 struct EventArgs {
     int32_t S, R, P, Q;
     int32_t macro_mode;
@@ -201,6 +201,7 @@ struct EventArgs {
     int32_t gate;            // 1: step while t < tmax; 0: no horizon
     int64_t max_steps;       // < 0: unlimited
     int32_t record_initial;  // record the state before the first step
+    int32_t keep_state;      // species, t and rng are to hold the state after the run
     const int32_t *save_idx;
     int32_t n_save;
     int64_t cap;             // records kept per trajectory

@@ -62,9 +62,11 @@ struct Nvrtc {
 };
 
 std::mutex g_mu;
+std::mutex g_nvrtc_mu;
 Nvrtc g_nvrtc;
 
 Nvrtc *nvrtc() {
+    std::lock_guard<std::mutex> lk(g_nvrtc_mu);
     if (g_nvrtc.tried) return g_nvrtc.ok ? &g_nvrtc : nullptr;
     g_nvrtc.tried = true;
     std::vector<std::string> names = {"libnvrtc.so.13", "libnvrtc.so"};
@@ -342,24 +344,39 @@ bool jit_compile(const Packed &p, int block, size_t *image_bytes) {
 }
 
 namespace {
-// Background compiles, joined when the library unloads (this object is
-// destroyed before the statics the compiles use, which are defined above).
+// Background compiles.  They have to end before NVRTC is torn down: jit_wait
+// runs at exit, registered after NVRTC is loaded and so called before its own
+// handlers, and from the Python package's exit hook, ahead of all of them.
 struct Background {
     std::mutex mu;
     std::set<uint64_t> started;
     std::vector<std::thread> threads;
-    ~Background() {
-        for (std::thread &t : threads)
-            if (t.joinable()) t.join();
-    }
-} g_background;
+};
+Background &background() {
+    static Background *b = new Background();  // never destroyed
+    return *b;
+}
 }  // namespace
 
+void jit_wait() {
+    std::vector<std::thread> threads;
+    {
+        std::lock_guard<std::mutex> lk(background().mu);
+        threads.swap(background().threads);
+    }
+    for (std::thread &t : threads) t.join();
+}
+
 void jit_compile_async(const Packed &p, int block) {
+    static std::once_flag once;
+    std::call_once(once, [] {
+        nvrtc();
+        std::atexit(jit_wait);
+    });
     const uint64_t key = fnv1a(jit_net_source(p, block));
-    std::lock_guard<std::mutex> lk(g_background.mu);
-    if (!g_background.started.insert(key).second) return;
-    g_background.threads.emplace_back([p, block]() {
+    std::lock_guard<std::mutex> lk(background().mu);
+    if (!background().started.insert(key).second) return;
+    background().threads.emplace_back([p, block]() {
         size_t n = 0;
         jit_compile(p, block, &n);  // failures leave the descriptor kernel in use
     });

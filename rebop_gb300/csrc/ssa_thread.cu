@@ -27,6 +27,9 @@
 //               macro's first r with total * U < cum_r (gillespie_macro.rs:159)
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
+#include "b64.cuh"
 #include "rng.cuh"
 #include "ssa_args.hpp"
 
@@ -277,44 +280,97 @@ int ssa_thread_occupancy(const SsaArgs &a, int block, size_t smem) {
 }
 
 // Propensity of reaction r at counts sp (API fold or macro factorials).
+// Double of an integer, on the integer pipes where it is exact and small.
+__device__ __forceinline__ double event_double(int64_t n) {
+    if ((uint64_t)n >= 1ull << 53) return (double)n;
+    return __longlong_as_double(n == 0 ? 0 : (long long)b64::from_u53((uint64_t)n));
+}
+
+// Exact binary64 propensity of reaction r at counts sp; fac: the descriptor's
+// factors, species and order side by side.
 template <bool MACRO>
-__device__ __forceinline__ double event_propensity(const EventArgs &a, const int64_t *sp, int r) {
+__device__ __forceinline__ double event_propensity(const EventArgs &a, const double *rate, const int2 *fac,
+                                                   const int64_t *sp, int r) {
     if (a.ex_off && a.ex_off[r] < a.ex_off[r + 1])
         return expr_eval(a.ex_code, a.ex_off[r], a.ex_off[r + 1], a.ex_const, sp, 1);
-    double acc = a.rate[r];
+    double acc = rate[r];
     for (int p = 0; p < a.P; ++p) {
-        const int o = a.fac_ord[r * a.P + p];
+        const int2 f = fac[r * a.P + p];
+        const int o = f.y;
         if (o == 0) continue;
-        const int64_t n = sp[a.fac_sp[r * a.P + p]];
+        const int64_t n = sp[f.x];
         if (MACRO) {
             int64_t ff = n;
             for (int j = 1; j < o; ++j) ff *= n - j;
-            acc = __dmul_rn(acc, (double)ff);
+            acc = __dmul_rn(acc, event_double(ff));
         } else {
-            for (int j = o - 1; j >= 0; --j) acc = __dmul_rn(acc, (double)(n - j));
+            for (int j = o - 1; j >= 0; --j) acc = __dmul_rn(acc, event_double(n - j));
         }
     }
     return acc;
 }
 
-// _advance_one_reaction in a loop.  The cumulative propensities are not
-// stored: the choice pass recomputes the same running sum, which gives the
-// same binary64 values as the first pass.
-template <bool MACRO>
-__global__ void __launch_bounds__(128) ssa_events_kernel(const __grid_constant__ EventArgs a) {
-    __shared__ double zt[2 * kZigTable];
-    for (int k = threadIdx.x; k < 2 * kZigTable; k += blockDim.x) zt[k] = a.zig[k];
-    __syncthreads();
-    const long long traj = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (traj >= a.n_traj) return;
-    int64_t *sp = a.species + traj * a.S;
+// _advance_one_reaction in a loop, a warp per trajectory, for single steps and
+// for networks whose descriptor does not fit events_chain_kernel's shared
+// memory.  SMEM: counts, descriptor and running sums in shared memory,
+// otherwise in global memory.
+template <bool MACRO, bool SMEM>
+__global__ void __launch_bounds__(32) ssa_events_kernel(const __grid_constant__ EventArgs a) {
+    extern __shared__ __align__(16) unsigned char ev_smem[];
+    double *zt = reinterpret_cast<double *>(ev_smem);  // Exp1 tables
+    const int lane = threadIdx.x, R = a.R, P = a.P, Q = a.Q, S = a.S;
+    const long long traj = blockIdx.x;
+    for (int k = lane; k < 2 * kZigTable; k += 32) zt[k] = a.zig[k];
+    int64_t *sp = a.species + traj * S;
+    double *rate_s = zt + 2 * kZigTable;
+    double *cum = rate_s + R;
+    int64_t *jd_s = reinterpret_cast<int64_t *>(cum + R);
+    int64_t *sp_s = jd_s + (size_t)R * Q;
+    int2 *fac_s = reinterpret_cast<int2 *>(sp_s + S);
+    int32_t *jsp_s = reinterpret_cast<int32_t *>(fac_s + (size_t)R * P);
+    int32_t *save_s = jsp_s + (size_t)R * Q;
+    if (SMEM) {
+        for (int r = lane; r < R; r += 32) rate_s[r] = a.rate[r];
+        for (int k = lane; k < R * P; k += 32) fac_s[k] = make_int2(a.fac_sp[k], a.fac_ord[k]);
+        for (int k = lane; k < R * Q; k += 32) {
+            jd_s[k] = a.jmp_d[k];
+            jsp_s[k] = a.jmp_sp[k];
+        }
+        for (int k = lane; k < a.n_save; k += 32) save_s[k] = a.save_idx[k];
+        for (int s = lane; s < S; s += 32) sp_s[s] = sp[s];
+        sp = sp_s;
+    }
+    const int64_t *jd = SMEM ? jd_s : a.jmp_d;
+    const int32_t *jsp = SMEM ? jsp_s : a.jmp_sp, *save = SMEM ? save_s : a.save_idx;
+    auto propensity = [&](int r) {
+        if (SMEM) return event_propensity<MACRO>(a, rate_s, fac_s, sp, r);
+        // (factors pair by pair from the descriptor's two arrays)
+        if (a.ex_off && a.ex_off[r] < a.ex_off[r + 1])
+            return expr_eval(a.ex_code, a.ex_off[r], a.ex_off[r + 1], a.ex_const, sp, 1);
+        double acc = a.rate[r];
+        for (int p = 0; p < P; ++p) {
+            const int o = a.fac_ord[r * P + p];
+            if (o == 0) continue;
+            const int64_t n = sp[a.fac_sp[r * P + p]];
+            if (MACRO) {
+                int64_t ff = n;
+                for (int j = 1; j < o; ++j) ff *= n - j;
+                acc = __dmul_rn(acc, (double)ff);
+            } else {
+                for (int j = o - 1; j >= 0; --j) acc = __dmul_rn(acc, (double)(n - j));
+            }
+        }
+        return acc;
+    };
     double t = a.t[traj];
     Xoshiro g{a.rng[traj * 4 + 0], a.rng[traj * 4 + 1], a.rng[traj * 4 + 2], a.rng[traj * 4 + 3]};
     long long n = 0;
+    __syncwarp();
     auto record = [&]() {
         if (n < a.cap) {
-            a.rec_t[traj * a.cap + n] = t;
-            for (int k = 0; k < a.n_save; ++k) a.rec_out[(traj * a.cap + n) * a.n_save + k] = sp[a.save_idx[k]];
+            const size_t row = (size_t)(traj * a.cap + n);
+            if (lane == 0) a.rec_t[row] = t;
+            for (int k = lane; k < a.n_save; k += 32) a.rec_out[row * a.n_save + k] = sp[save[k]];
         }
         ++n;
     };
@@ -322,33 +378,71 @@ __global__ void __launch_bounds__(128) ssa_events_kernel(const __grid_constant__
     long long steps = 0;
     const int64_t t_start = global_ns();
     while ((!a.gate || t < a.tmax) && (a.max_steps < 0 || steps < a.max_steps)) {
-        if ((steps & 1023) == 1023 && global_ns() - t_start > a.budget_ns) {
-            atomicExch(a.flag, 1ull);
+        if ((steps & 1023) == 1023 && __any_sync(0xffffffffu, global_ns() - t_start > a.budget_ns)) {
+            if (lane == 0) atomicExch(a.flag, 1ull);
             break;
         }
-        double total = 0.0;
-        for (int r = 0; r < a.R; ++r) total = __dadd_rn(total, event_propensity<MACRO>(a, sp, r));
+        // running sums, 32 reactions at a time (R <= 32: in registers)
+        double total = 0.0, mine = 0.0;
+        for (int r0 = 0; r0 < R; r0 += 32) {
+            const int r = r0 + lane, m = min(32, R - r0);
+            const double acc = r < R ? propensity(r) : 0.0;
+            for (int j = 0; j < m; ++j) {
+                total = __dadd_rn(total, __longlong_as_double(__shfl_sync(0xffffffffu, __double_as_longlong(acc), j)));
+                if (lane == j) mine = total;
+            }
+            if (SMEM && R > 32 && r < R) cum[r] = mine;
+        }
         if (!(0.0 < total)) {
             t = __longlong_as_double(0x7FF0000000000000ll);  // +inf
         } else {
             t = __dadd_rn(t, __ddiv_rn(xo_exp1(g, zt, zt + kZigTable), total));
             const double chosen = __dmul_rn(total, xo_uniform(g));
-            double c = 0.0;
-            int idx = MACRO ? a.R : 0;
-            for (int r = 0; r < a.R; ++r) {
-                c = __dadd_rn(c, event_propensity<MACRO>(a, sp, r));
+            int idx = 0;  // #{r : cum_r < chosen}, or the macro's first r with chosen < cum_r
+            if (R <= 32) {
                 if (MACRO) {
-                    if (idx == a.R && chosen < c) idx = r;
+                    const unsigned int above = __ballot_sync(0xffffffffu, lane < R && chosen < mine);
+                    idx = above ? __ffs((int)above) - 1 : R;
                 } else {
-                    idx += (c < chosen) ? 1 : 0;
+                    idx = __popc(__ballot_sync(0xffffffffu, lane < R && mine < chosen));
+                }
+            } else {
+                double c = 0.0;
+                bool found = false;
+                for (int r0 = 0; r0 < R && !found; r0 += 32) {
+                    const int r = r0 + lane, m = min(32, R - r0);
+                    if (SMEM) {
+                        mine = r < R ? cum[r] : 0.0;
+                    } else {
+                        const double acc = r < R ? propensity(r) : 0.0;
+                        for (int j = 0; j < m; ++j) {
+                            c = __dadd_rn(c, __longlong_as_double(__shfl_sync(0xffffffffu, __double_as_longlong(acc), j)));
+                            if (lane == j) mine = c;
+                        }
+                    }
+                    if (MACRO) {
+                        const unsigned int above = __ballot_sync(0xffffffffu, r < R && chosen < mine);
+                        found = above != 0;
+                        idx = above ? r0 + __ffs((int)above) - 1 : R;
+                    } else {
+                        idx += __popc(__ballot_sync(0xffffffffu, r < R && mine < chosen));
+                    }
                 }
             }
-            if (idx < a.R)
-                for (int q = 0; q < a.Q; ++q) sp[a.jmp_sp[idx * a.Q + q]] += a.jmp_d[idx * a.Q + q];
+            __syncwarp();
+            if (idx < R)
+                for (int q = lane; q < Q; q += 32) {
+                    const int64_t d = jd[idx * Q + q];
+                    if (d != 0) sp[jsp[idx * Q + q]] += d;
+                }
+            __syncwarp();
         }
         ++steps;
         record();
     }
+    if (SMEM)
+        for (int s = lane; s < S; s += 32) a.species[traj * S + s] = sp[s];
+    if (lane != 0) return;
     a.t[traj] = t;
     a.rng[traj * 4 + 0] = g.s0;
     a.rng[traj * 4 + 1] = g.s1;
@@ -357,16 +451,266 @@ __global__ void __launch_bounds__(128) ssa_events_kernel(const __grid_constant__
     if (a.n_rec) a.n_rec[traj] = n;
 }
 
+// Every event of one trajectory up to the first at or after tmax
+// (EventArgs::gate).  Each time is a result, so the arithmetic is binary64
+// throughout, and an FP64 instruction of a warp holds its scheduler's pipe for
+// 64 cycles however few lanes take part (measured; a division 569): an event's
+// 55 of them took 1.75 us on one warp.  So the event is a pipeline of four
+// warps, each on a scheduler of its own:
+//   draws  the random words, Exp1 and the choice's uniform (every event consumes
+//          both, so they do not depend on the state)
+//   chain  counts -> propensities (one reaction a lane) -> their fold -> the
+//          reaction -> the jump; counts kept as doubles and comparisons done on
+//          integers leave it the products and the fold's adds
+//   clock  t + Exp1 / total, the recorded times, the horizon
+//   record the counts again from the reactions that fired, the recorded rows
+// over rings of 64 events in shared memory.  The chain stores nothing to global
+// memory and hands over eight events at a time; clock and record tell how far
+// they are every 16 events.  The chain runs ahead of the clock and past the
+// last event; records past the clock's last one are not counted.
+// The dimer network takes 1.0 us an event, its chain's 2 000 cycles (one lane on
+// descriptor and counts in global memory: 4.1 us, and twice that beyond 4 096
+// records, for which the run was made again).
+// Every wait has an iteration limit; one that runs out ends the run as an
+// exhausted time budget.
+constexpr unsigned int kEventRing = 64, kEventSpins = 1u << 24;
+
+template <bool MACRO>
+__global__ void __launch_bounds__(128) events_chain_kernel(const __grid_constant__ EventArgs a) {
+    extern __shared__ __align__(16) unsigned char ev_smem[];
+    __shared__ uint64_t ring_x[kEventRing], ring_u[kEventRing], ring_tot[kEventRing];
+    __shared__ int ring_idx[kEventRing];
+    __shared__ volatile unsigned int n_draws, n_chain, n_clock, n_rows;  // events each warp is done with
+    __shared__ volatile int stop, chain_end;  // the clock's end, or a wait's limit; the chain's
+    double *zt = reinterpret_cast<double *>(ev_smem);            // Exp1 tables
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, R = a.R, P = a.P, Q = a.Q, S = a.S;
+    const long long traj = blockIdx.x;
+    double *rate = zt + 2 * kZigTable;
+    double *cum = rate + R;
+    int64_t *jd = reinterpret_cast<int64_t *>(cum + R);
+    int64_t *sp = jd + (size_t)R * Q;
+    int2 *fac = reinterpret_cast<int2 *>(sp + S);
+    int32_t *jsp = reinterpret_cast<int32_t *>(fac + (size_t)R * P);
+    int32_t *save = jsp + (size_t)R * Q;
+    int64_t *sp_rows = reinterpret_cast<int64_t *>((reinterpret_cast<uintptr_t>(save + a.n_save) + 7) & ~(uintptr_t)7);
+    double *dv = reinterpret_cast<double *>(sp_rows + S);
+    for (int k = tid; k < 2 * kZigTable; k += 128) zt[k] = a.zig[k];
+    for (int r = tid; r < R; r += 128) rate[r] = a.rate[r];
+    for (int k = tid; k < R * P; k += 128) fac[k] = make_int2(a.fac_sp[k], a.fac_ord[k]);
+    for (int k = tid; k < R * Q; k += 128) {
+        jd[k] = a.jmp_d[k];
+        jsp[k] = a.jmp_sp[k];
+    }
+    for (int k = tid; k < a.n_save; k += 128) save[k] = a.save_idx[k];
+    for (int s = tid; s < S; s += 128) sp[s] = sp_rows[s] = a.species[traj * S + s];
+    if (tid == 0) {
+        n_draws = n_chain = n_clock = n_rows = 0;
+        stop = chain_end = 0;
+    }
+    __syncthreads();
+    const int64_t t_start = global_ns();
+    const long long first = a.record_initial ? 1 : 0;  // record of event 0
+    // wait until `count` is past event e (or within the ring of it); false to end
+    auto reached = [&](volatile unsigned int &count, unsigned int e, unsigned int slack, volatile int &end) {
+        for (unsigned int k = 0; k < kEventSpins; ++k) {
+            const int ended = end;  // before the count: what was published until then counts
+            __threadfence_block();
+            if ((int)(count + slack - e) > 0) {
+                __threadfence_block();
+                return true;
+            }
+            if (ended) return false;
+        }
+        stop = 1;
+        atomicExch(a.flag, 1ull);
+        return false;
+    };
+    auto publish = [&](volatile unsigned int &count, unsigned int e) {
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0) count = e + 1;
+    };
+    if (warp == 2) {
+        // ---------------------------------------------------------- draws
+        Xoshiro g{a.rng[traj * 4 + 0], a.rng[traj * 4 + 1], a.rng[traj * 4 + 2], a.rng[traj * 4 + 3]};
+        for (unsigned int e = 0;; ++e) {
+            const double x = xo_exp1(g, zt, zt + kZigTable);
+            const double u = xo_uniform(g);
+            if (e % 16 == 0 &&  // room for sixteen more
+                !__all_sync(0xffffffffu, reached(n_clock, e + 15, kEventRing, stop) && reached(n_rows, e + 15, kEventRing, stop)))
+                break;
+            if (lane == 0) {
+                ring_x[e % kEventRing] = (uint64_t)__double_as_longlong(x);
+                ring_u[e % kEventRing] = (uint64_t)__double_as_longlong(u);
+            }
+            if ((e & 7) == 7) publish(n_draws, e);
+        }
+    } else if (warp == 1) {
+        // ---------------------------------------------------------- clock
+        double t = a.t[traj];
+        long long n = first;  // records whose time is known
+        if (a.record_initial && a.cap > 0 && lane == 0) a.rec_t[traj * a.cap] = t;
+        unsigned int there = 0;  // events known to be there
+        for (unsigned int e = 0; t < a.tmax; ++e) {
+            if (e >= there) {
+                if (!__all_sync(0xffffffffu, reached(n_chain, e, 0, stop))) break;
+                there = __shfl_sync(0xffffffffu, n_chain, 0);
+            }
+            const uint64_t tb = ring_tot[e % kEventRing];
+            const double total = __longlong_as_double((long long)tb);
+            t = tb - 1 < 0x7FF0000000000000ull ? __dadd_rn(t, __ddiv_rn(__longlong_as_double((long long)ring_x[e % kEventRing]), total))
+                            : __longlong_as_double(0x7FF0000000000000ll);  // +inf
+            if (n < a.cap && lane == 0) a.rec_t[traj * a.cap + n] = t;
+            ++n;
+            if ((e & 15) == 15) publish(n_clock, e);
+            if ((e & 1023) == 1023 && __any_sync(0xffffffffu, global_ns() - t_start > a.budget_ns)) {
+                if (lane == 0) atomicExch(a.flag, 1ull);
+                break;
+            }
+        }
+        if (lane == 0) {
+            stop = 1;
+            a.t[traj] = t;
+            if (a.n_rec) a.n_rec[traj] = n;
+        }
+    } else if (warp == 3) {
+        // ---------------------------------------------------------- record
+        long long n = 0;
+        for (unsigned int e = 0;; ++e) {
+            if (n < a.cap)
+                for (int k = lane; k < a.n_save; k += 32)
+                    a.rec_out[(size_t)(traj * a.cap + n) * a.n_save + k] = sp_rows[save[k]];
+            n += e > 0 || a.record_initial;
+            if (!__all_sync(0xffffffffu, reached(n_chain, e, 0, chain_end))) break;
+            const int idx = ring_idx[e % kEventRing];
+            if (idx < R)
+                for (int q = lane; q < Q; q += 32) {
+                    const int64_t d = jd[idx * Q + q];
+                    if (d != 0) sp_rows[jsp[idx * Q + q]] += d;
+                }
+            __syncwarp();
+            if ((e & 15) == 15) publish(n_rows, e);
+        }
+    } else {
+        // ---------------------------------------------------------- chain
+        // Up to 32 reactions of order <= 2 in the run-time API's arithmetic:
+        // a lane's reaction is rate * dv[i1] * dv[i2], dv[2 s] and dv[2 s + 1]
+        // the doubles of n_s and n_s - 1 and dv[2 S] = 1 (a factor too many,
+        // exact), in the reference's order of factors.
+        int i1 = 2 * S, i2 = 2 * S;
+        bool two = !MACRO && R <= 32 && !a.ex_off;
+        if (two && lane < R)
+            for (int p = 0, k = 0; p < P; ++p) {
+                const int2 f = fac[lane * P + p];
+                for (int j = f.y - 1; j >= 0; --j, ++k) {
+                    two = two && k < 2 && f.y <= 2;
+                    if (k == 0) i1 = 2 * f.x + j;
+                    else i2 = 2 * f.x + j;
+                }
+            }
+        two = __all_sync(0xffffffffu, two);
+        for (int s = lane; s < S; s += 32) {
+            dv[2 * s] = event_double(sp[s]);
+            dv[2 * s + 1] = event_double(sp[s] - 1);
+        }
+        if (lane == 0) dv[2 * S] = 1.0;
+        __syncwarp();
+        const double my_rate = lane < R ? rate[lane] : 0.0;
+        unsigned int drawn = 0;  // draws known to be there
+        for (unsigned int e = 0;; ++e) {
+            // running sums, 32 reactions at a time (R <= 32: in registers)
+            double total = 0.0, mine = 0.0;
+            bool plain = true;  // no propensity below 0 (or NaN): sums compare as integers
+            for (int r0 = 0; r0 < R; r0 += 32) {
+                const int r = r0 + lane, m = min(32, R - r0);
+                const double acc = two     ? __dmul_rn(__dmul_rn(my_rate, dv[i1]), dv[i2])
+                                   : r < R ? event_propensity<MACRO>(a, rate, fac, sp, r)
+                                           : 0.0;
+                const uint64_t bits = (uint64_t)__double_as_longlong(acc);
+                plain = plain && (bits <= 0x7FF0000000000000ull || bits << 1 == 0);
+#pragma unroll 4
+                for (int j = 0; j < m; ++j) {
+                    total = __dadd_rn(total, __longlong_as_double(__shfl_sync(0xffffffffu, __double_as_longlong(acc), j)));
+                    if (lane == j) mine = total;
+                }
+                if (R > 32 && r < R) cum[r] = mine;
+            }
+            if (e >= drawn) {
+                if (!__all_sync(0xffffffffu, reached(n_draws, e, 0, stop))) break;
+                drawn = __shfl_sync(0xffffffffu, n_draws, 0);
+            }
+            const double u = __longlong_as_double((long long)ring_u[e % kEventRing]);
+            const uint64_t tb = (uint64_t)__double_as_longlong(total);
+            if (lane == 0) ring_tot[e % kEventRing] = tb;
+            const bool fires = 0.0 < total;
+            int idx = R;
+            if (fires) {
+                const double chosen = __dmul_rn(total, u);
+                const uint64_t cb = (uint64_t)__double_as_longlong(chosen);
+                const bool bits = __all_sync(0xffffffffu, plain);
+                idx = 0;  // #{r : cum_r < chosen}, or the macro's first r with chosen < cum_r
+                for (int r0 = 0; r0 < R; r0 += 32) {
+                    const int r = r0 + lane;
+                    if (R > 32) mine = r < R ? cum[r] : 0.0;
+                    const uint64_t mb = (uint64_t)__double_as_longlong(mine);
+                    if (MACRO) {
+                        const unsigned int has =
+                            __ballot_sync(0xffffffffu, r < R && (bits ? cb < mb : chosen < mine));
+                        idx = has ? r0 + __ffs((int)has) - 1 : R;
+                        if (has) break;
+                    } else {
+                        idx += __popc(__ballot_sync(0xffffffffu, r < R && (bits ? mb < cb : mine < chosen)));
+                    }
+                }
+                __syncwarp();
+                if (idx < R)
+                    for (int q = lane; q < Q; q += 32) {
+                        const int64_t d = jd[idx * Q + q];
+                        if (d != 0) {
+                            const int s = jsp[idx * Q + q];
+                            const int64_t n = sp[s] + d;
+                            sp[s] = n;
+                            if (two) {
+                                dv[2 * s] = event_double(n);
+                                dv[2 * s + 1] = event_double(n - 1);
+                            }
+                        }
+                    }
+            }
+            if (lane == 0) ring_idx[e % kEventRing] = idx;
+            __syncwarp();
+            // hand-overs eight events at a time (the clock's +inf ends the run
+            // when nothing can fire)
+            if ((e & 7) == 7 || !fires) publish(n_chain, e);
+            if (!fires) break;
+        }
+        __threadfence_block();
+        __syncwarp();
+        if (lane == 0) chain_end = 1;
+    }
+}
+
+template <bool MACRO>
+static int events_launch(const EventArgs &a, cudaStream_t st) {
+    const size_t tables = 16 * (size_t)kZigTable;
+    const size_t smem = tables + 16 * (size_t)a.R + 12 * (size_t)a.R * a.Q + 8 * (size_t)a.S + 8 * (size_t)a.R * a.P +
+                        4 * (size_t)std::max(a.n_save, 0) + 16 + 24 * (size_t)a.S;  // (the chain's: counts twice more, as doubles)
+    if (smem > 200 * 1024) {
+        ssa_events_kernel<MACRO, false><<<(unsigned)a.n_traj, 32, tables, st>>>(a);
+        return (int)cudaGetLastError();
+    }
+    const bool chain = a.gate && a.max_steps < 0 && !a.keep_state;
+    auto kern = chain ? events_chain_kernel<MACRO> : ssa_events_kernel<MACRO, true>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    kern<<<(unsigned)a.n_traj, chain ? 128 : 32, smem, st>>>(a);
+    return (int)cudaGetLastError();
+}
+
 int launch_ssa_events(const EventArgs &a, void *stream) {
     if (a.n_traj == 0) return 0;
-    const int block = 128;
-    const int grid = (int)((a.n_traj + block - 1) / block);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (a.macro_mode)
-        ssa_events_kernel<true><<<grid, block, 0, st>>>(a);
-    else
-        ssa_events_kernel<false><<<grid, block, 0, st>>>(a);
-    return (int)cudaGetLastError();
+    return a.macro_mode ? events_launch<true>(a, st) : events_launch<false>(a, st);
 }
 
 }  // namespace rbg

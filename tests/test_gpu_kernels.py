@@ -118,3 +118,28 @@ def test_count_gradients_match_oracle(rb, B, tail):
     for g, r in list(zip(dW, rW)) + list(zip(db, rb_)):
         g = g.double().cpu().numpy()
         assert g.shape == r.shape and np.linalg.norm(g - r) <= 2e-2 * np.linalg.norm(r) + 1e-7
+
+
+# the every-event pipeline: 1, 32 and 33 reactions (in registers, in shared memory), an order-3
+# reaction, macro arithmetic and a rate expression (general propensities), a run that nothing can fire
+# in any more, one that ends at its first event, one with more records than asked for
+@pytest.mark.parametrize("S,R,seed,tmax", [(1, 1, 60, 40.0), (5, 9, 61, 0.05), (16, 32, 62, 0.02), (9, 33, 63, 0.02),
+                                           (8, 20, 64, 0.02), (30, 200, 65, 2e-3)])
+def test_every_event_pipeline(rb, O, S, R, seed, tmax):
+    import bench
+
+    reactions, x0 = bench.random_network(seed, S, R, x0_mean=40.0)
+    if R == 1:
+        reactions = [(0.5, [1], [-1])]  # decays to nothing: the last record is at +inf
+    if seed == 64:
+        reactions[3] = (1e-3, [3] + [0] * (S - 1), [-1] + [0] * (S - 1))
+    net, onet = rb.Network(S), O.OracleNet(S)
+    for k, e, d in reactions:
+        net.add_reaction(rb.Rate.lma(k, e), d)
+        onet.add_lma(k, e, d)
+    for s in (1, 2, 3):
+        for tm, cap in ((tmax, 4096), (0.0, 4096), (tmax * 1e-6, 1)):
+            t, c = net.run_all_events(x0, s, tm, cap=cap)
+            rt, rc = onet.run_all_events(x0, s, tm)
+            np.testing.assert_array_equal(t, rt)
+            np.testing.assert_array_equal(c, rc)
