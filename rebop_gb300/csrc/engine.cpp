@@ -352,7 +352,8 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
     const int spec_grid = (int)std::max<int64_t>(
         1, std::min<int64_t>(ctx->sm_count, (r.n_traj + ssa_spec_block() - 1) / ssa_spec_block()));
     const int spec_slots = ssa_spec_slots(a, spec_grid, ctx->smem_optin, ssa_spec_block());
-    // Rate::Expr networks run on the generic kernel (native binary64 programs).
+    // Rate::Expr networks run on the generic kernel (native binary64 programs)
+    // or a generated one (below).
     const bool spec = !p.has_expr && !want_generic && !want_fast && !want_warp && r.times_ok && r.t_last < 0x1p60 &&
                       ssa_spec_supported(a, p.max_order) && spec_slots > 0;
     // Networks beyond the thread kernels' reach (more than 32 reactions, or
@@ -362,13 +363,31 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
                       (want_warp || (!spec && !(p.R <= 32 && ssa_thread_max_block(a, ctx->smem_optin) > 0)));
     const bool fast = !warp && !spec && !p.has_expr && !want_generic && r.times_ok && ssa_fast_supported(a, p.max_order) &&
                       ssa_fast_smem(a, 128) <= ctx->smem_optin;
+    // Networks with rate expressions run a generated kernel where it covers
+    // them (float pairs as for mass action; mapping 0 all the same: the
+    // program interpreter is what runs until it is compiled).  10 000
+    // trajectories of a 3-reaction enzyme network with a quotient (1.4e6
+    // events): 6.6 ms in the interpreter, which the binary64 pipe bounds, and
+    // 1.03 ms generated.  Counts beyond 2^23 throughout, where every interval
+    // is run again in binary64: 2.04 and 2.56 ms (20 000 trajectories, 6.7e6
+    // events).
+    const int expr_terms = p.has_expr && !pref && !force && !r.rates && r.times_ok && r.t_last < 0x1p60 &&
+                                   jit_supported(p) && p.max_order < 32768 && !p.macro_mode
+                               ? jit_expr_terms(p)
+                               : -1;
+    if (expr_terms >= 0) {
+        a.n_const = (int32_t)p.ex_const.size();
+        a.max_mults = std::max(a.max_mults, expr_terms);
+    }
+    const bool jit_expr = expr_terms >= 0 && ssa_spec_slots(a, spec_grid, ctx->smem_optin, 128) > 0;
     // Networks of 17 to 32 reactions run a generated kernel too (the lockstep
     // exact kernel until it is compiled): 20 000 trajectories of 12 species
     // and 24 reactions (2.4e7 events) take 21.1 ms in the lockstep kernel and
     // 2.1 ms generated, of 16 species and 32 reactions 42.9 and 3.1 ms.
-    const bool jit_only = !spec && !warp && !want_generic && !want_fast && !want_desc &&
-                          !(pref && std::strcmp(pref, "spec") == 0) && r.times_ok && r.t_last < 0x1p60 &&
-                          !p.has_expr && spec_jit_only(a, p, spec_grid, *ctx);
+    const bool jit_only = jit_expr ||
+                          (!spec && !warp && !want_generic && !want_fast && !want_desc &&
+                           !(pref && std::strcmp(pref, "spec") == 0) && r.times_ok && r.t_last < 0x1p60 &&
+                           !p.has_expr && spec_jit_only(a, p, spec_grid, *ctx));
     const bool strict = pref || force;  // a kernel asked for must run
     if (strict && ((want_fast && !fast) || (want_warp && !warp) || (want_desc && !spec) ||
                    (want_jit && !spec && !jit_only))) {
@@ -445,7 +464,7 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
         return true;
     }
     if (spec || jit_only) {
-        a.row_done = r.n_samples < 65536 ? r.row_done : nullptr;
+        a.row_done = r.n_samples < 65536 && !jit_expr ? r.row_done : nullptr;
         a.phase_steps = shape.phase;
         a.sched = shape.sched > 0 ? 1 : 0;
         if (const char *ph = std::getenv("RB_SPEC_PHASE")) a.phase_steps = std::atoi(ph);
@@ -487,8 +506,8 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
         // RB_SSA_KERNEL=spec (or a shape of kernel 3) asks for the
         // packed-descriptor kernel itself
         const bool off = (jit && std::strcmp(jit, "0") == 0) || want_desc;
-        // (a 17- to 32-reaction network compiles for longer: only a large
-        // ensemble run a second time waits for it)
+        // (networks of 17 to 32 reactions and rate expressions wait for the
+        // compiler only with a large ensemble run a second time)
         const bool compile = jit ? !off : (want_jit || (jit_only ? r.n_traj >= 4096 && run_no >= 2
                                                                  : r.n_traj >= 4096 || run_no >= 2));
         if (!off) {
@@ -542,7 +561,7 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
                      : launch_ssa_thread(a, block, grid, smem, stream);
     if (err != 0) return cuda_ok((cudaError_t)err, "SSA kernel launch");
     if (timed && !cuda_ok(cudaEventRecord(dn.ev_stop, stream), "cudaEventRecord")) return false;
-    if (mapping) *mapping = jk ? 4 : spec ? 3 : fast ? 2 : 0;
+    if (mapping) *mapping = jk && !jit_expr ? 4 : spec ? 3 : fast ? 2 : 0;
     return true;
 }
 

@@ -36,6 +36,9 @@ struct SsaArgs {
     const int32_t *ex_off;
     const int32_t *ex_code;
     const double *ex_const;
+    // Generated kernels of networks with rate expressions: the number of
+    // constants, kept behind the R shared rates (0 otherwise).
+    int32_t n_const;
 
     // trajectories
     int64_t n_traj;

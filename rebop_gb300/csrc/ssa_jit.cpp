@@ -19,6 +19,7 @@
 #include <nvrtc.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -168,18 +169,150 @@ bool jit_supported(const Packed &p) {
     return true;
 }
 
+// Error terms (gamma each) of reaction r's expression in float pairs: one per
+// constant and operation, four per division.  -1 if it has an operation that
+// the float pairs do not cover (a difference loses its relative error; exp and
+// powers have none), or a value that may leave 2^-90 .. 2^90 without being
+// zero (counts reach 2^23, a larger one takes the exact path): there low parts
+// would be lost.
+static int expr_terms(const Packed &p, int r) {
+    struct Range {
+        int lo, hi;  // zero, or 2^lo <= value < 2^hi
+    };
+    std::vector<Range> st;
+    int m = 0;
+    for (int32_t k = p.ex_off[(size_t)r]; k < p.ex_off[(size_t)r + 1]; k++) {
+        const int op = p.ex_code[(size_t)k] & 0xff, arg = p.ex_code[(size_t)k] >> 8;
+        Range v{0, 0};
+        if (op == 0) {
+            const double c = p.ex_const[(size_t)arg];
+            if (std::signbit(c) || (c != 0.0 && !(c >= 0x1p-60 && c < 0x1p60))) return -1;
+            if (c > 0.0) v = Range{std::ilogb(c), std::ilogb(c) + 1};
+            m += 1;
+        } else if (op == 1) {
+            v = Range{0, 23};
+        } else {
+            if (st.size() < 2) return -1;
+            const Range b = st.back();
+            st.pop_back();
+            const Range a = st.back();
+            st.pop_back();
+            switch (op) {
+                case 3: v = Range{std::min(a.lo, b.lo), std::max(a.hi, b.hi) + 1}, m += 1; break;
+                case 5: v = Range{a.lo + b.lo, a.hi + b.hi}, m += 1; break;
+                case 6: v = Range{a.lo - b.hi, a.hi - b.lo}, m += 4; break;
+                case 8: case 9: v = Range{std::min(a.lo, b.lo), std::max(a.hi, b.hi)}; break;
+                default: return -1;
+            }
+        }
+        if (v.lo < -90 || v.hi > 90) return -1;
+        st.push_back(v);
+    }
+    return st.size() == 1 ? m : -1;
+}
+
+int jit_expr_terms(const Packed &p) {
+    int m = 0;
+    for (int r = 0; r < p.R; r++) {
+        if (p.ex_off[(size_t)r] == p.ex_off[(size_t)r + 1]) continue;
+        const int e = expr_terms(p, r);
+        if (e < 0 || e > 64) return -1;
+        m = std::max(m, e);
+    }
+    return m;
+}
+
+// Straight-line binary64 evaluation of reaction r's expression (expr_eval's
+// operations); count(s) gives the text of a species count as a long long.
+// Returns the name of the result, its lines go to o.
+template <class Count>
+static std::string expr_exact(const Packed &p, int r, Count count, std::ostringstream &o) {
+    std::vector<std::string> st;
+    int n = 0;
+    for (int32_t k = p.ex_off[(size_t)r]; k < p.ex_off[(size_t)r + 1]; k++) {
+        const int op = p.ex_code[(size_t)k] & 0xff, arg = p.ex_code[(size_t)k] >> 8;
+        const std::string v = "x" + std::to_string(r) + "_" + std::to_string(n++);
+        if (op == 0) {
+            o << "    const double " << v << " = __longlong_as_double((long long)rl[" << p.R + arg << " * RS]);\n";
+        } else if (op == 1) {
+            o << "    const double " << v << " = (double)" << count(arg) << ";\n";
+        } else {
+            const std::string b = st.back();
+            st.pop_back();
+            const std::string a = st.back();
+            st.pop_back();
+            const char *f = op == 3 ? "__dadd_rn" : op == 5 ? "__dmul_rn" : op == 6 ? "__ddiv_rn" : op == 8 ? "fmax" : "fmin";
+            o << "    const double " << v << " = " << f << "(" << a << ", " << b << ");\n";
+        }
+        st.push_back(v);
+    }
+    return st.back();
+}
+
+// The same in float pairs: an operand is a count (an exact float) or a pair.
+// `bad` is set for a divisor of zero.
+static void expr_pairs(const Packed &p, int r, std::ostringstream &o) {
+    struct V {
+        bool pair;
+        std::string name;
+    };
+    auto df = [](const V &v) { return v.pair ? v.name : "DF{" + v.name + ", 0.0f}"; };
+    std::vector<V> st;
+    int n = 0;
+    for (int32_t k = p.ex_off[(size_t)r]; k < p.ex_off[(size_t)r + 1]; k++) {
+        const int op = p.ex_code[(size_t)k] & 0xff, arg = p.ex_code[(size_t)k] >> 8;
+        const std::string v = "y" + std::to_string(n++);
+        if (op == 1) {
+            st.push_back({false, "c.n[" + std::to_string(arg) + "]"});
+            continue;
+        }
+        if (op == 0) {
+            o << "            const float2 k" << v << " = rf[" << p.R + arg << " * RS];\n            const DF " << v
+              << "{k" << v << ".x, k" << v << ".y};\n";
+            st.push_back({true, v});
+            continue;
+        }
+        const V b = st.back();
+        st.pop_back();
+        const V a = st.back();
+        st.pop_back();
+        o << "            const DF " << v << " = ";
+        if (op == 3) {
+            o << "df_add(" << df(a) << ", " << df(b) << ");\n";
+        } else if (op == 5) {
+            if (a.pair && b.pair) o << "df_mul(" << a.name << ", " << b.name << ");\n";
+            else if (a.pair || b.pair) o << "df_mul_f(" << (a.pair ? a : b).name << ", " << (a.pair ? b : a).name << ");\n";
+            else o << "df_mul_f(DF{" << a.name << ", 0.0f}, " << b.name << ");\n";
+        } else if (op == 6) {
+            o << "df_div(" << df(a) << ", " << df(b) << ", rcp_approx((" << df(b) << ").h));\n";
+            o << "            bad |= !((" << df(b) << ").h > 0.0f);\n";
+        } else {
+            o << "df_less(" << df(a) << ", " << df(b) << ") " << (op == 8 ? "? " + df(b) + " : " + df(a) : "? " + df(a) + " : " + df(b))
+              << ";\n";
+        }
+        st.push_back({true, v});
+    }
+    o << "            const DF acc = " << df(st.back()) << ";\n";
+}
+
 std::string jit_net_source(const Packed &p, int block) {
     const int S = p.S, R = p.R;
     std::ostringstream o;
     o << "// generated network operations: " << S << " species, " << R << " reactions\n";
     o << "#include \"ssa_spec_body.cuh\"\n\nnamespace rbg {\n\n";
+    auto has_expr = [&](int r) { return p.has_expr && p.ex_off[(size_t)r] < p.ex_off[(size_t)r + 1]; };
     // exact binary64 choice for the rare close float comparisons
     o << "__device__ __noinline__ int net_exact_choice(float cn[" << S
       << "], const uint64_t *rl, int RS, uint64_t u53) {\n";
     o << "    double cum[" << R << "];\n    double total = 0.0, acc;\n";
     for (int r = 0; r < R; r++) {
-        o << "    acc = __longlong_as_double((long long)rl[" << r << " * RS]);\n";
-        for (int f = 0; f < p.P; f++) {
+        if (has_expr(r)) {
+            const std::string v =
+                expr_exact(p, r, [](int s) { return "(long long)cn[" + std::to_string(s) + "]"; }, o);
+            o << "    acc = " << v << ";\n";
+        } else
+            o << "    acc = __longlong_as_double((long long)rl[" << r << " * RS]);\n";
+        for (int f = 0; f < p.P && !has_expr(r); f++) {
             const int32_t ord = p.fac_ord[(size_t)r * p.P + f];
             const int32_t sp = p.fac_sp[(size_t)r * p.P + f];
             if (ord == 0) continue;
@@ -229,11 +362,16 @@ std::string jit_net_source(const Packed &p, int block) {
     o << "    __device__ static bool props(const SsaArgs &, const ExactTables &, const Counts &c, const int64_t *, int,\n"
          "                                 const float2 *rf, int RS, float *cum, DF &tot) {\n";
     o << "        RunSum sum;\n";
+    if (p.has_expr) o << "        bool bad = false;\n";
     o << "        float lo = c.n[0], hi = c.n[0];\n";
     for (int s = 1; s < S; s++) o << "        lo = fminf(lo, c.n[" << s << "]); hi = fmaxf(hi, c.n[" << s << "]);\n";
     for (int r = 0; r < R; r++) {
-        o << "        {\n            const float2 k = rf[" << r << " * RS];\n            DF acc{k.x, k.y};\n";
-        for (int f = 0; f < p.P; f++) {
+        if (has_expr(r)) {
+            o << "        {\n";
+            expr_pairs(p, r, o);
+        } else
+            o << "        {\n            const float2 k = rf[" << r << " * RS];\n            DF acc{k.x, k.y};\n";
+        for (int f = 0; f < p.P && !has_expr(r); f++) {
             const int32_t ord = p.fac_ord[(size_t)r * p.P + f];
             const int32_t sp = p.fac_sp[(size_t)r * p.P + f];
             for (int j = 0; j < ord; j++) {
@@ -251,12 +389,42 @@ std::string jit_net_source(const Packed &p, int block) {
         o << "            cum[" << r << "] = sum.s;\n        }\n";
     }
     o << "        tot = rs_total(sum);\n";
-    o << "        return !(lo >= 0.0f && hi < 8388608.0f);\n    }\n";
+    if (p.has_expr) o << "        return bad || !(lo >= 0.0f && hi < 8388608.0f);\n    }\n";
+    else o << "        return !(lo >= 0.0f && hi < 8388608.0f);\n    }\n";
     o << "    __device__ static int exact_choice(const SsaArgs &, const ExactTables &, const Counts &c, const int64_t "
          "*, int,\n                                       const uint64_t *rl, int RS, uint64_t u53) {\n";
     o << "        float cn[" << S << "];\n";
     for (int s = 0; s < S; s++) o << "        cn[" << s << "] = c.n[" << s << "];\n";
     o << "        return net_exact_choice(cn, rl, RS, u53);\n    }\n";
+    // exact re-run of an interval
+    const char *replay_args = "const SsaArgs &a, const ExactTables &ex, int64_t *sp, const int64_t *sps, uint64_t "
+                              "*gsv,\n        const uint64_t *rl, int RS, int NS, uint64_t t0, uint64_t T, bool nat, "
+                              "unsigned long long ev0, int64_t t_start";
+    o << "    __device__ static unsigned long long replay(" << replay_args << ") {\n";
+    if (p.has_expr) {
+        o << "        (void)nat;\n        return replay_native<NetOps>(a, ex, sp, sps, gsv, rl, RS, NS, t0, T, ev0, "
+             "t_start);\n    }\n";
+        o << "    __device__ static void exact_props(const int64_t *sp, int NS, const uint64_t *rl, int RS, double *out) "
+             "{\n    double acc;\n";
+        for (int r = 0; r < R; r++) {
+            if (has_expr(r)) {
+                const std::string v =
+                    expr_exact(p, r, [](int s) { return "sp[" + std::to_string(s) + " * NS]"; }, o);
+                o << "    out[" << r << "] = " << v << ";\n";
+                continue;
+            }
+            o << "    acc = __longlong_as_double((long long)rl[" << r << " * RS]);\n";
+            for (int f = 0; f < p.P; f++)
+                for (int j = p.fac_ord[(size_t)r * p.P + f] - 1; j >= 0; j--)
+                    o << "    acc = __dmul_rn(acc, (double)(sp[" << p.fac_sp[(size_t)r * p.P + f] << " * NS] - " << j
+                      << "));\n";
+            o << "    out[" << r << "] = acc;\n";
+        }
+        o << "    }\n";
+    } else {
+        o << "        return replay_interval<kMaxR, kMacro>(a, ex, sp, sps, gsv, rl, RS, NS, t0, T, nat, ev0, "
+             "t_start);\n    }\n";
+    }
     // jump: per species, the sum of the deltas of the reaction that fired
     o << "    __device__ static void jump(Counts &c, const SsaArgs &, const ExactTables &, int64_t *, int, int idx) "
          "{\n";

@@ -13,6 +13,11 @@ namespace rbg {
 // Networks the generator covers: 1..16 species, 1..32 reactions, jumps of
 // magnitude below 2^23.
 bool jit_supported(const Packed &p);
+// Rate expressions the generator covers (counts and non-negative constants
+// combined by + * / max min, so that every value keeps its relative error):
+// the most float-pair error terms of one of them, -1 if one is not covered.
+// jit_supported does not look at expressions.
+int jit_expr_terms(const Packed &p);
 // CUDA source of the speculative kernel specialised for the network, for
 // blocks of `block` lanes (a multiple of 32, at most 1024).
 std::string jit_net_source(const Packed &p, int block);

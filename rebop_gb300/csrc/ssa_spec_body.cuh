@@ -125,6 +125,8 @@ __device__ __forceinline__ DF df_div(DF a, DF b, float r) {
     return fast2sum(q1, __fmul_rn(res, r));
 }
 
+__device__ __forceinline__ bool df_less(DF a, DF b) { return a.h < b.h || (a.h == b.h && a.l < b.l); }
+
 // Exact float of an integer 0 <= x < 2^23.
 __device__ __forceinline__ float f23(uint32_t x) { return __fsub_rn(__uint_as_float(0x4B000000u | x), 8388608.0f); }
 
@@ -267,7 +269,7 @@ __host__ __device__ inline size_t spec_smem_bytes(const SsaArgs &a, int slots) {
     b += 24 * (size_t)spec_sample_cache(a);             // sample times: bits, float triple
     b += 4 * (size_t)a.n_save + 16;                     // saved species
     b += 8 * (size_t)R * Q;                             // jd
-    b += 16 * (size_t)R * (rate_per_traj ? slots : 1);  // exact rate bits, float-pair rates
+    b += 16 * ((size_t)R + a.n_const) * (rate_per_traj ? slots : 1);  // exact rate bits, float-pair rates
     b += 16 * (size_t)S * slots;                        // counts, counts at interval start
     b += 32 * (size_t)slots;                            // generator at interval start
     b += 80 * (size_t)slots;                            // 10 state words
@@ -300,6 +302,44 @@ __device__ __noinline__ unsigned long long replay_interval(const SsaArgs &a, con
         t = tx;
         ++e;
         if (ix < a.R)
+            for (int k = 0; k < a.Q; ++k) sp[ex.jsp[ix * a.Q + k] * BD] += ex.jd[ix * a.Q + k];
+    }
+    gsv[0] = h.s0;
+    gsv[BD] = h.s1;
+    gsv[2 * BD] = h.s2;
+    gsv[3 * BD] = h.s3;
+    return e;
+}
+
+// The same re-run in native binary64, for networks whose propensities the
+// factor lists do not describe (rate expressions): Ops::exact_props gives them.
+template <class Ops>
+__device__ __noinline__ unsigned long long replay_native(const SsaArgs &a, const ExactTables &ex, int64_t *sp,
+                                                         const int64_t *sps, uint64_t *gsv, const uint64_t *rl, int RS,
+                                                         int BD, uint64_t t0, uint64_t T_bits, unsigned long long ev0,
+                                                         int64_t t_start) {
+    constexpr int R = Ops::kMaxR;
+    for (int s = 0; s < a.S; ++s) sp[s * BD] = sps[s * BD];
+    Xoshiro h{gsv[0], gsv[BD], gsv[2 * BD], gsv[3 * BD]};
+    unsigned long long e = ev0;
+    double t = __longlong_as_double((long long)t0);
+    const double T = __longlong_as_double((long long)T_bits);
+    for (unsigned int n = 1;; ++n) {
+        if ((n & 255u) == 0 && global_ns() - t_start > a.budget_ns) return ~0ull;
+        double cum[R], total = 0.0;
+        Ops::exact_props(sp, BD, rl, RS, cum);
+#pragma unroll
+        for (int r = 0; r < R; ++r) cum[r] = total = __dadd_rn(total, cum[r]);
+        if (!(0.0 < total)) break;
+        const double tn = __dadd_rn(t, __ddiv_rn(xo_exp1(h, a.zig, a.zig + kZigOffF), total));
+        if (tn > T) break;
+        const double chosen = __dmul_rn(total, xo_uniform(h));
+        int ix = 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) ix += cum[r] < chosen ? 1 : 0;
+        t = tn;
+        ++e;
+        if (ix < R)
             for (int k = 0; k < a.Q; ++k) sp[ex.jsp[ix * a.Q + k] * BD] += ex.jd[ix * a.Q + k];
     }
     gsv[0] = h.s0;
@@ -474,6 +514,12 @@ struct TableOps {
                                        int NS, const uint64_t *rl, int RS, uint64_t u53) {
         return exact_choice_table<MAXR, MACRO>(a, ex, sp, NS, rl, RS, u53);
     }
+    __device__ static unsigned long long replay(const SsaArgs &a, const ExactTables &ex, int64_t *sp,
+                                                const int64_t *sps, uint64_t *gsv, const uint64_t *rl, int RS, int NS,
+                                                uint64_t t0, uint64_t T, bool nat, unsigned long long ev0,
+                                                int64_t t_start) {
+        return replay_interval<MAXR, MACRO>(a, ex, sp, sps, gsv, rl, RS, NS, t0, T, nat, ev0, t_start);
+    }
     __device__ static void jump(Counts &, const SsaArgs &a, const ExactTables &ex, int64_t *sp, int NS, int idx) {
         if (idx < a.R)
             for (int k = 0; k < a.Q; ++k) sp[ex.jsp[idx * a.Q + k] * NS] += ex.jd[idx * a.Q + k];
@@ -485,7 +531,6 @@ struct TableOps {
 template <class Ops>
 __device__ __forceinline__ void spec_body(const SsaArgs &a) {
     constexpr int MAXR = Ops::kMaxR;
-    constexpr bool MACRO = Ops::kMacro;
     const int BD = blockDim.x, tid = threadIdx.x;
     const int NS = a.n_slots;  // slots per block: a multiple of the warps, >= 32 per warp
     const int warp = tid >> 5, lane = tid & 31;
@@ -502,8 +547,9 @@ __device__ __forceinline__ void spec_body(const SsaArgs &a) {
     const bool rate_cols = a.rate_stride != 0;  // per-slot rate columns
     const int RS = rate_cols ? NS : 1;           // stride between two reactions' rates
     uint64_t *rate = reinterpret_cast<uint64_t *>(jd + (size_t)R * Q);
-    float2 *rdf = reinterpret_cast<float2 *>(rate + (size_t)R * RS);
-    int64_t *spa = reinterpret_cast<int64_t *>(rdf + (size_t)R * RS);
+    const int RT = R + a.n_const;  // rates, then expression constants
+    float2 *rdf = reinterpret_cast<float2 *>(rate + (size_t)RT * RS);
+    int64_t *spa = reinterpret_cast<int64_t *>(rdf + (size_t)RT * RS);
     int64_t *spsa = spa + (size_t)S * NS;
     uint64_t *gsva = reinterpret_cast<uint64_t *>(spsa + (size_t)S * NS);
     uint64_t *stw = gsva + 4 * (size_t)NS;                         // [10][NS]
@@ -538,8 +584,8 @@ __device__ __forceinline__ void spec_body(const SsaArgs &a) {
         xdf[k] = *reinterpret_cast<const float2 *>(&v);
     }
     if (!a.rate_stride)
-        for (int r = tid; r < R; r += BD) {
-            const uint64_t rb = (uint64_t)__double_as_longlong(a.rate[r]);
+        for (int r = tid; r < RT; r += BD) {
+            const uint64_t rb = (uint64_t)__double_as_longlong(r < R ? a.rate[r] : a.ex_const[r - R]);
             rate[r] = rb;
             const DF d = spec_rate_ok(rb) ? df_from_double(__longlong_as_double((long long)rb)) : DF{0.f, 0.f};
             rdf[r] = make_float2(d.h, d.l);
@@ -757,8 +803,7 @@ __device__ __forceinline__ void spec_body(const SsaArgs &a) {
                 if (replay) {
                     if (!exact_traj) atomicAdd(a.work + 3, 1ull);  // speculation undecided
                     const unsigned long long ev0 = st[8 * NS];
-                    ev = replay_interval<MAXR, MACRO>(a, ex, sp, sps, gsv, rl, RS, NS, st[4 * NS], st[5 * NS], nat,
-                                                      ev0, t_start);
+                    ev = Ops::replay(a, ex, sp, sps, gsv, rl, RS, NS, st[4 * NS], st[5 * NS], nat, ev0, t_start);
                     if (ev == ~0ull) {
                         ev = ev0;
                         abort_run = true;

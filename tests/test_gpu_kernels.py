@@ -17,24 +17,14 @@ def _seeds(n, salt):
     return np.random.default_rng(4321 + salt).integers(np.iinfo(np.uint64).max, size=n, dtype=np.uint64)
 
 
-def _random(rb, O, seed, S, R, macro=False):
+def _random(rb, O, seed, S, R):
     import bench
 
     reactions, x0 = bench.random_network(seed, S, R, x0_mean=60.0)
-    onet = O.OracleNet(S, macro=macro)
-    if macro:
-        lines = [f"r{k}: {' + '.join(f'{c} x{i}' for i, c in enumerate(e) if c)} => "
-                 f"{' + '.join(f'{a + b} x{i}' for i, (a, b) in enumerate(zip(e, d)) if a + b)} @ {k_!r}"
-                 for k, (k_, e, d) in enumerate(reactions)]
-        net = rb.Network.from_dsl("Net { " + ", ".join(f"x{i}" for i in range(S)) + " }\n" + "\n".join(lines))
-    else:
-        net = rb.Network(S)
+    net, onet = rb.Network(S), O.OracleNet(S)
     for k, e, d in reactions:
-        if macro:
-            onet.add_macro(k, [(i, x) for i, x in enumerate(e) if x], d)
-        else:
-            net.add_reaction(rb.Rate.lma(k, e), d)
-            onet.add_lma(k, e, d)
+        net.add_reaction(rb.Rate.lma(k, e), d)
+        onet.add_lma(k, e, d)
     return net, onet, x0
 
 
@@ -143,3 +133,44 @@ def test_every_event_pipeline(rb, O, S, R, seed, tmax):
             rt, rc = onet.run_all_events(x0, s, tm)
             np.testing.assert_array_equal(t, rt)
             np.testing.assert_array_equal(c, rc)
+
+
+# rate expressions on a generated kernel: every operation it covers, divisors that reach zero, a
+# constant of zero, counts at and beyond 2^23, one to 32 reactions; the last is beyond it (minus)
+EXPR = {
+    "divide": (["0.5 * A * B / (20 + B)", "0.02 * B * B", "3 * A / (A + B)"], [[-1, 1], [1, -2], [1, 0]], [40, 3]),
+    "zero divisor": (["2 * B / A", "0.3 * A"], [[1, -1], [-1, 1]], [1, 6]),
+    "max min": (["max(A, 0.5 * B) * 0.1", "min(A * 0.2, B) + 0 * A", "5 / max(B, 1)"], [[-1, 1], [1, -1], [2, 0]],
+                [30, 30]),
+    "constant": (["1.5"], [[1, 1]], [0, 0]),
+    "large": (["1e-8 * A * B", "0.05 * A + 0.1"], [[-1, 1], [2, 0]], [(1 << 23) - 3, 5_000_000]),
+    "32": ([f"0.0{k % 7 + 1} * {'AB'[k % 2]} / (1 + 0.{k + 1:02d} * {'BA'[k % 2]})" for k in range(32)],
+           [[1 - 2 * (k % 2), 2 * (k % 2) - 1] if k % 3 else [(k % 2) * 2 - 1, 0] for k in range(32)], [60, 60]),
+    "minus": (["4 * (A - 0.5 * B)", "0.1 * A"], [[1, 1], [-1, 0]], [50, 10]),
+}
+
+
+@pytest.mark.parametrize("n", [33, 5000])
+@pytest.mark.parametrize("case", EXPR)
+def test_rate_expressions_on_a_generated_kernel(rb, O, monkeypatch, case, n):
+    from rebop_gb300 import expr as E
+
+    monkeypatch.setenv("RB_JIT", "1")
+    texts, deltas, x0 = EXPR[case]
+    net, onet = rb.Network(2), O.OracleNet(2)
+    for s, d in zip(texts, deltas):
+        e = E.parse(s).to_expr({"A": 0, "B": 1}, {})
+        code, consts = e.to_program()
+        net.add_reaction(rb.Rate.expression(e), d)
+        onet.add_expr(code, consts, d)
+    # a mass-action reaction between them keeps the order of the sum visible
+    if len(texts) < 32:
+        net.add_reaction(rb.Rate.lma(0.05, [0, 1]), [0, -1])
+        onet.add_lma(0.05, [0, 1], [0, -1])
+    seeds = _seeds(n, 97)
+    tmax = 1e-4 if case == "large" else 2.0
+    res = net.run_ensemble(x0, seeds, tmax, 6)
+    ref, ev, _, _ = onet.run_ensemble(x0, seeds, tmax, 6)
+    assert res.stats["mapping"] == 0 and ev.max() > 1
+    np.testing.assert_array_equal(res.counts, ref)
+    np.testing.assert_array_equal(res.events, ev)
