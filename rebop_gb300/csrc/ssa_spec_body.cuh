@@ -31,9 +31,8 @@
 // two-sum errors and low parts) is within G = (M + R + 2 + (R (R + 1) / 2 +
 // R (M + 2)) / 16) gamma of the reference's and Exp1/total
 // within (G + 6 gamma) q plus the Exp1 abscissa's absolute error over the
-// total.  The triple-float clock add is exact up to its low part's rounding,
-// and the reference's own rounding of t + q adds at most 2^-53 (t + q): the
-// bound grows by 2^-52 t per event, accumulated with upward rounding.
+// total; SpecBound below adds the clock's roundings, its own and the
+// reference's.
 //
 // This header holds the device side, templated on the network operations of
 // the float-pair step: TableOps below walks the packed descriptor; a network
@@ -176,6 +175,47 @@ __device__ __forceinline__ TF tf_add(TF t, DF q) {
     return TF{h, __fsub_rn(m2, __fsub_rn(h, s)), l};
 }
 
+// t - (ah + al), exact but for the roundings into the low part; the parts need
+// not be normalised.
+__device__ __forceinline__ TF tf_sub(TF t, float ah, float al) {
+    float s, e1, m, e2, m2, e3, h, e4;
+    two_sum(t.h, -ah, s, e1);
+    two_sum(t.m, -al, m, e2);
+    two_sum(m, e1, m2, e3);
+    two_sum(s, m2, h, e4);
+    return TF{h, e4, __fadd_rn(t.l, __fadd_rn(e2, e3))};
+}
+
+// Error bound of the time left to a sample.  Within a phase of P steps (and
+// an interval) the time passed A is a float running sum of Exp1/total with the
+// two-sum errors and low parts beside it: |low| <= P 2^-23 A, so its roundings
+// and those of the comparison stay below (P^2 / 2 + 4 P + 64) 2^-48 of the time
+// that was left (what passes beyond it is past the sample by far).  The
+// quotients are within c_rem of themselves, their Exp1's absolute errors are
+// summed beside (xsum), and the reference's clock rounds by 2^-53 T a step,
+// counted as P steps.  2^-110: quotients below the float range's full
+// precision.  At the end of a phase the time left is kept in three floats.
+//
+// 15 instructions a step; a triple-float clock with its bound updated every
+// step took some 35: dimer ensemble 26.9 -> 23.2 ms, 24 reactions 2.08 -> 1.87,
+// 100 Vilar oscillators (one warp per scheduler) 316 -> 292.
+struct SpecBound {
+    float c_rem, c_T;
+    __device__ __forceinline__ float clock(float T) const { return __fmaf_ru(c_T, T, 0x1p-110f); }
+    __device__ __forceinline__ float margin(float rem, float low, float T, float err) const {
+        return __fmul_ru(1.01f, __fadd_ru(__fadd_ru(err, fabsf(low)), __fmaf_ru(c_rem, fabsf(rem), clock(T))));
+    }
+    // the interval from t0 to T: its length (two parts), T, the margin of its
+    // first phase (no decision for a length that the parts do not cover)
+    __device__ __forceinline__ float4 interval(double t0, double T) const {
+        const double len = __dsub_rn(T, t0);
+        const float h = __double2float_rn(len), Tf = __double2float_ru(T);
+        const bool ok = len == 0.0 || (fabs(len) >= 0x1p-80 && fabs(len) < 0x1p61);
+        return make_float4(h, __double2float_rn(__dsub_rn(len, (double)h)), Tf,
+                           ok ? margin(h, 0.f, Tf, 0.f) : __int_as_float(0x7f800000));
+    }
+};
+
 // Wedge test of the ziggurat, f[i+1] - |f[i] - f[i+1]| U < exp(-x), for the
 // candidate x = X_i (2k + 1) 2^-53 (xh its float within 2^-24 x) and U = mu
 // 2^-53.  First in float32: the float copies of the tables and U are within
@@ -266,14 +306,14 @@ __host__ __device__ inline size_t spec_smem_bytes(const SsaArgs &a, int slots) {
     const int S = a.S, R = a.R, P = a.P, Q = a.Q;
     const bool rate_per_traj = a.rate_stride != 0;
     size_t b = 16 * 256 + 8 * 257 + 8 * 256 + 8 * 256;  // zxk, zf, zd, xdf
-    b += 24 * (size_t)spec_sample_cache(a);             // sample times: bits, float triple
+    b += 16 * (size_t)spec_sample_cache(a);             // sample intervals
     b += 4 * (size_t)a.n_save + 16;                     // saved species
     b += 8 * (size_t)R * Q;                             // jd
     b += 16 * ((size_t)R + a.n_const) * (rate_per_traj ? slots : 1);  // exact rate bits, float-pair rates
     b += 16 * (size_t)S * slots;                        // counts, counts at interval start
     b += 32 * (size_t)slots;                            // generator at interval start
-    b += 80 * (size_t)slots;                            // 10 state words
-    b += 32 * (size_t)slots;                            // 7 float state words, flags
+    b += 72 * (size_t)slots;                            // 9 state words
+    b += 28 * (size_t)slots;                            // 6 float state words, flags
     b += 4 * (size_t)slots + 512;                       // slot list, block counters
     b += 8 * (size_t)slots;                             // rows recorded, not yet counted
     b += 4 * ((size_t)R * P + (size_t)R * Q);           // fac, jsp
@@ -395,7 +435,7 @@ __device__ __noinline__ int exact_choice_table(const SsaArgs &a, const ExactTabl
 }
 
 // Slot flags.
-constexpr uint32_t kLive = 1, kNat = 2, kExactTraj = 4, kBegin = 8, kHave = 16;
+constexpr uint32_t kLive = 1, kNat = 2, kExactTraj = 4, kHave = 8;
 
 // Rows [lo, hi) of `out` hold this lane's trajectory's samples: count them in
 // a.row_done, after a fence that makes the sample stores visible device-wide
@@ -552,9 +592,9 @@ __device__ __forceinline__ void spec_body(const SsaArgs &a) {
     int64_t *spa = reinterpret_cast<int64_t *>(rdf + (size_t)RT * RS);
     int64_t *spsa = spa + (size_t)S * NS;
     uint64_t *gsva = reinterpret_cast<uint64_t *>(spsa + (size_t)S * NS);
-    uint64_t *stw = gsva + 4 * (size_t)NS;                         // [10][NS]
-    float *stf = reinterpret_cast<float *>(stw + 10 * (size_t)NS);  // [7][NS]
-    uint32_t *stflag = reinterpret_cast<uint32_t *>(stf + 7 * (size_t)NS);
+    uint64_t *stw = gsva + 4 * (size_t)NS;                        // [9][NS]
+    float *stf = reinterpret_cast<float *>(stw + 9 * (size_t)NS);  // [6][NS]
+    uint32_t *stflag = reinterpret_cast<uint32_t *>(stf + 6 * (size_t)NS);
     int32_t *slot_list = reinterpret_cast<int32_t *>(stflag + NS);
     int32_t *ctr = slot_list + NS;  // [1] abort flag
     // rows a slot's trajectories recorded since the last count (a.row_done):
@@ -566,19 +606,27 @@ __device__ __forceinline__ void spec_body(const SsaArgs &a) {
     int32_t *jsp = fac + (size_t)R * P;
     int32_t *ssave = jsp + (size_t)R * Q;  // saved species indices
     const int n_cache = spec_sample_cache(a);
-    uint64_t *sTb = reinterpret_cast<uint64_t *>(
-        (reinterpret_cast<uintptr_t>(ssave + a.n_save) + 15) & ~(uintptr_t)15);  // sample time bits
-    float *sTf = reinterpret_cast<float *>(sTb + n_cache);                         // as float triples
+    float4 *const sInt = reinterpret_cast<float4 *>(
+        (reinterpret_cast<uintptr_t>(ssave + a.n_save) + 15) & ~(uintptr_t)15);  // sample intervals
+
+    // running-sum bound: the products and the reference's own roundings
+    // (M + R + 2 gamma), plus the float32 accumulation of the low parts,
+    // (r + M + 2) 2^-48 of the total at add r (1/16 gamma each)
+    const float G = ((float)(a.max_mults + R + 2) +
+                     (float)(R * (R + 1) / 2 + R * (a.max_mults + 2)) * 0.0625f) * kGamma;
+    const int phase_steps = a.phase_steps > 0 ? a.phase_steps : kSpecPhase;
+    const float ps = (float)phase_steps;
+    SpecBound bd;
+    bd.c_rem = G + 6.0f * kGamma + (0.5f * ps * ps + 4.0f * ps + 64.0f) * 0x1p-48f;
+    bd.c_T = ps * 0x1p-53f;
+    // float32 choice margin / total: running sums within (R + M + 2) 2^-24,
+    // U truncated to 2^-23, the product rounded (2^-24), the total's high
+    // part within 2^-24
+    const float c_sel = (float)(a.max_mults + R + 6) * 0x1p-24f * 1.001f;
+
     load_exact_tables(a, zxk, zf, zd, fac, jsp, jd);
     for (int k = tid; k < a.n_save; k += BD) ssave[k] = a.save_idx[k];
-    for (int k = tid; k < n_cache; k += BD) {
-        const double v = a.sample_t[k];
-        sTb[k] = (uint64_t)__double_as_longlong(v);
-        const TF f = tf_from_double(v);
-        sTf[3 * k] = f.h;
-        sTf[3 * k + 1] = f.m;
-        sTf[3 * k + 2] = f.l;
-    }
+    for (int k = tid; k < n_cache; k += BD) sInt[k] = bd.interval(k ? a.sample_t[k - 1] : 0.0, a.sample_t[k]);
     for (int k = tid; k < 256; k += BD) {
         const double v = a.zig[kZigOffXdf + k];
         xdf[k] = *reinterpret_cast<const float2 *>(&v);
@@ -601,32 +649,24 @@ __device__ __forceinline__ void spec_body(const SsaArgs &a) {
     __syncthreads();
     const ExactTables ex{zxk, zf, zd, fac, jsp, jd};
 
-    // running-sum bound: the products and the reference's own roundings
-    // (M + R + 2 gamma), plus the float32 accumulation of the low parts,
-    // (r + M + 2) 2^-48 of the total at add r (1/16 gamma each)
-    const float G = ((float)(a.max_mults + R + 2) +
-                     (float)(R * (R + 1) / 2 + R * (a.max_mults + 2)) * 0.0625f) * kGamma;
-    const float c_q = G + 6.0f * kGamma;                     // relative bound of Exp1/total
-    // float32 choice margin / total: running sums within (R + M + 2) 2^-24,
-    // U truncated to 2^-23, the product rounded (2^-24), the total's high
-    // part within 2^-24
-    const float c_sel = (float)(a.max_mults + R + 6) * 0x1p-24f * 1.001f;
     const int64_t t_start = global_ns();
-    const int phase_steps = a.phase_steps > 0 ? a.phase_steps : kSpecPhase;
     unsigned int rot = 0;
     unsigned long long lane_events = 0;
 
     // ---- this lane's slot; the hot state sits in registers during a phase,
-    // the cold words (interval start t0, sample time T, trajectory, event
-    // count at the interval start, sample index) stay in the slot's columns
+    // the cold words (the trajectory's first clock, its index, event counts,
+    // sample index) stay in the slot's columns
     int slot = lane < lanes ? wbase + lane : -1;
     int32_t *const wlist = slot_list + wbase;
     typename Ops::Counts c{};
     Xoshiro g{0, 0, 0, 0};
-    TF Tc{0.f, 0.f, 0.f}, tc{0.f, 0.f, 0.f};  // sample time, clock
-    float err_t = 0.f;                         // bound on |clock - reference clock|
+    TF rem{0.f, 0.f, 0.f};            // time to the sample, at the start of the phase or interval
+    float ah = 0.f, al = 0.f;         // time passed since: the sum of Exp1/total
+    float T_h = 0.f;                  // sample time
+    float err0 = 0.f, mrg = 0.f;      // bound on |rem - the reference's|, on |rem - a - ...| in this phase
+    float xsum = 0.f;                 // sum of the Exp1 draws' absolute error bounds / total, in gamma
     unsigned long long ev = 0;
-    bool live = slot >= 0, have = false, nat = false, exact_traj = false, begin = false, abort_run = false;
+    bool live = slot >= 0, have = false, nat = false, exact_traj = false, abort_run = false;
 
     for (;;) {
         // rows this lane's slot recorded in the phase, counted after it by the
@@ -641,74 +681,59 @@ __device__ __forceinline__ void spec_body(const SsaArgs &a) {
             uint64_t *const st = stw + slot;  // cold words: st[k * NS]
             uint64_t *const rl = rate + (rate_cols ? slot : 0);
             float2 *const rf = rdf + (rate_cols ? slot : 0);
-            for (int step = 0; step < phase_steps && live; ++step) {
-                if (!have || begin) {  // rare: one branch for both
-                    if (!have) {
-                        // take the next trajectory into this slot
-                        const long long traj = (long long)atomicAdd(a.work, 1ull);
-                        if (traj >= a.n_traj) {
-                            live = false;
-                            break;
-                        }
-                        uint64_t t0;
-                        if (a.in_species) {
-                            for (int s = 0; s < S; ++s) sp[s * NS] = a.in_species[traj * S + s];
-                            t0 = (uint64_t)__double_as_longlong(a.in_t[traj]);
-                            g.s0 = a.in_rng[traj * 4 + 0];
-                            g.s1 = a.in_rng[traj * 4 + 1];
-                            g.s2 = a.in_rng[traj * 4 + 2];
-                            g.s3 = a.in_rng[traj * 4 + 3];
-                        } else {
-                            for (int s = 0; s < S; ++s) sp[s * NS] = a.x0[traj * a.x0_stride + s];
-                            t0 = 0;
-                            xo_seed(g, a.seeds[traj]);
-                        }
-                        nat = !emul_domain(t0);
-                        exact_traj = (t0 >> 52) > 1023 + 60;
-                        for (int r = 0; r < R; ++r) {
-                            const uint64_t rb = (uint64_t)__double_as_longlong(a.rate[traj * a.rate_stride + r]);
-                            nat |= !emul_domain(rb);
-                            exact_traj |= !spec_rate_ok(rb);
-                            if (rate_cols) {
-                                rl[r * RS] = rb;
-                                const DF d = df_from_double(__longlong_as_double((long long)rb));
-                                rf[r * RS] = make_float2(d.h, d.l);
-                            }
-                        }
-                        exact_traj |= nat;
-                        exact_traj |= !Ops::load(c, a, sp, NS);
-                        tc = tf_from_double(__longlong_as_double((long long)t0));
-                        st[4 * NS] = t0;
-                        st[6 * NS] = (uint64_t)traj;
-                        st[9 * NS] = 0;
-                        ev = 0;
-                        have = true;
-                        begin = true;
+            auto begin_interval = [&](const float4 v) {
+                rem = TF{v.x, v.y, 0.f};
+                T_h = v.z;
+                mrg = v.w;
+                err0 = ah = al = xsum = 0.f;
+                gsv[0] = g.s0;
+                gsv[NS] = g.s1;
+                gsv[2 * NS] = g.s2;
+                gsv[3 * NS] = g.s3;
+                st[7 * NS] = ev;
+            };
+            for (int step = 0; step < phase_steps; ++step) {
+                if (!have) {
+                    // take the next trajectory into this slot
+                    const long long traj = (long long)atomicAdd(a.work, 1ull);
+                    if (traj >= a.n_traj) {
+                        live = false;
+                        break;
                     }
-                    if (begin) {
-                        // a sample interval starts at t0 (the clock tc holds t0
-                        // exactly): save what a re-run needs
-                        const int si = (int)st[9 * NS];
-                        if (si < n_cache) {
-                            st[5 * NS] = sTb[si];
-                            Tc = TF{sTf[3 * si], sTf[3 * si + 1], sTf[3 * si + 2]};
-                        } else {
-                            const double T = a.sample_t[si];
-                            st[5 * NS] = (uint64_t)__double_as_longlong(T);
-                            Tc = tf_from_double(T);
-                        }
-                        err_t = 0.f;
-                        if (exact_traj)
-                            for (int s = 0; s < S; ++s) sps[s * NS] = sp[s * NS];
-                        else
-                            Ops::save(c, a, sp, sps, NS);
-                        gsv[0] = g.s0;
-                        gsv[NS] = g.s1;
-                        gsv[2 * NS] = g.s2;
-                        gsv[3 * NS] = g.s3;
-                        st[8 * NS] = ev;
-                        begin = false;
+                    uint64_t t0;
+                    if (a.in_species) {
+                        for (int s = 0; s < S; ++s) sps[s * NS] = a.in_species[traj * S + s];
+                        t0 = (uint64_t)__double_as_longlong(a.in_t[traj]);
+                        g.s0 = a.in_rng[traj * 4 + 0];
+                        g.s1 = a.in_rng[traj * 4 + 1];
+                        g.s2 = a.in_rng[traj * 4 + 2];
+                        g.s3 = a.in_rng[traj * 4 + 3];
+                    } else {
+                        for (int s = 0; s < S; ++s) sps[s * NS] = a.x0[traj * a.x0_stride + s];
+                        t0 = 0;
+                        xo_seed(g, a.seeds[traj]);
                     }
+                    nat = !emul_domain(t0);
+                    exact_traj = (t0 >> 52) > 1023 + 60;
+                    for (int r = 0; r < R; ++r) {
+                        const uint64_t rb = (uint64_t)__double_as_longlong(a.rate[traj * a.rate_stride + r]);
+                        nat |= !emul_domain(rb);
+                        exact_traj |= !spec_rate_ok(rb);
+                        if (rate_cols) {
+                            rl[r * RS] = rb;
+                            const DF d = df_from_double(__longlong_as_double((long long)rb));
+                            rf[r * RS] = make_float2(d.h, d.l);
+                        }
+                    }
+                    exact_traj |= nat;
+                    for (int s = 0; s < S; ++s) sp[s * NS] = sps[s * NS];
+                    exact_traj |= !Ops::load(c, a, sp, NS);
+                    st[4 * NS] = t0;
+                    st[5 * NS] = (uint64_t)traj;
+                    st[8 * NS] = 0;
+                    ev = 0;
+                    have = true;
+                    begin_interval(bd.interval(__longlong_as_double((long long)t0), a.sample_t[0]));
                 }
 
                 bool fire = false, replay = exact_traj;
@@ -727,89 +752,95 @@ __device__ __forceinline__ void spec_body(const SsaArgs &a) {
                     const uint64_t K1 = ex.zxk[i1].y;
                     const float2 X1 = xdf[i1];
                     DF x = df_mul(df_u53(2 * k1 + 1), DF{X1.x, X1.y});
-                    float xerr = kGamma * X1.x;
+                    float xerr = X1.x;  // in gamma
                     float cum[MAXR];
                     DF tot;
-                    bool amb = Ops::props(a, ex, c, sp, NS, rf, RS, cum, tot);
+                    const bool wild = Ops::props(a, ex, c, sp, NS, rf, RS, cum, tot);
                     const bool slow = !(k1 < K1);
                     uint64_t bu = b2;
-                    if (tot.h > 0.0f) {
-                        if (slow) {
-                            // wedge or tail: b2 was its uniform, the choice
-                            // takes the draw after the Exp1 is settled
-                            x = exp1_df_cont(g, b1, b2, x, ex, xdf, xerr);
-                            bu = xo_next(g);
-                        }
-                        amb |= tot.h < 0x1p-90f || tot.h > 0x1p90f;
-                        const float r = rcp_approx(tot.h);
-                        const DF q = df_div(x, tot, r);
-                        const TF tn = tf_add(tc, q);
-                        // error bound, rounded up: previous bound, Exp1/total
-                        // against the reference's quotient, the reference's
-                        // rounding of its clock add, the low part's roundings
-                        float err_tn = __fadd_ru(err_t, __fmul_ru(c_q, q.h));
-                        err_tn = __fadd_ru(err_tn, __fmul_ru(__fmul_ru(xerr, r), 1.001f));
-                        err_tn = __fadd_ru(err_tn, __fmul_ru(0x1p-52f, tn.h));
-                        err_tn = __fadd_ru(err_tn, __fmul_ru(0x1p-23f, fabsf(tn.l)));
-                        // T - tn: the high difference is exact near T, the
-                        // rest is below 2^-46 max(T, tn) off
-                        const float d = __fadd_rn(__fsub_rn(Tc.h, tn.h),
-                                                  __fadd_rn(__fsub_rn(Tc.m, tn.m), __fsub_rn(Tc.l, tn.l)));
-                        const float mt = __fadd_ru(err_tn, __fmul_ru(0x1p-44f, fmaxf(Tc.h, tn.h)));
-                        const float dd = __fmul_rn(d, 1.0f - 0x1p-22f);
-                        fire = dd > mt;
-                        amb |= !(fire || dd < -mt) || !(err_tn < 1.0e30f) || q.h < 0x1p-100f;
-                        // choice #{r : cum_r < total * U} in float32: the high
-                        // parts are within 2^-23.9 of the exact sums, U and the
-                        // product add 2^-23 each; a comparison inside that
-                        // margin is redone exactly in binary64
-                        const float ch = __fmul_rn(tot.h, f23((uint32_t)(bu >> 41)) * 0x1p-23f);
-                        const float msel = c_sel * tot.h;
-                        bool close = false;
+                    if (slow && tot.h > 0.0f) {
+                        // wedge or tail: b2 was its uniform, the choice
+                        // takes the draw after the Exp1 is settled
+                        x = exp1_df_cont(g, b1, b2, x, ex, xdf, xerr);
+                        xerr *= 1.0f / kGamma;
+                        bu = xo_next(g);
+                    }
+                    bool amb = wild || !(tot.h >= 0x1p-90f && tot.h <= 0x1p90f);
+                    const float r = rcp_approx(tot.h);
+                    const DF q = df_div(x, tot, r);
+                    // time passed in this phase and interval, and what is left
+                    // after it: fires when that is above its error bound
+                    float an, e1;
+                    two_sum(ah, q.h, an, e1);
+                    const float ln = __fadd_rn(al, __fadd_rn(e1, q.l));
+                    const float d = __fadd_rn(__fsub_rn(rem.h, an), __fsub_rn(rem.m, ln));
+                    const float xn = __fmaf_ru(xerr, r, xsum);
+                    const float mt = __fmaf_ru(kGamma * 1.01f, xn, mrg);
+                    fire = d > mt;
+                    // choice #{r : cum_r < total * U} in float32: the high
+                    // parts are within 2^-23.9 of the exact sums, U and the
+                    // product add 2^-23 each; a comparison inside that
+                    // margin is redone exactly in binary64
+                    const float ch = __fmul_rn(tot.h, f23((uint32_t)(bu >> 41)) * 0x1p-23f);
+                    const float msel = c_sel * tot.h;
+                    bool close = false;
 #pragma unroll
-                        for (int rr = 0; rr < MAXR; ++rr) {
-                            if (rr < R) {
-                                const float dr = __fsub_rn(cum[rr], ch);
-                                idx += dr < 0.0f ? 1 : 0;
-                                close |= fabsf(dr) <= msel;
-                            }
+                    for (int rr = 0; rr < MAXR; ++rr) {
+                        if (rr < R) {
+                            const float dr = __fsub_rn(cum[rr], ch);
+                            idx += dr < 0.0f ? 1 : 0;
+                            close |= fabsf(dr) <= msel;
                         }
-                        if (!amb && fire && !close) {
-                            // the common step, decided in float32: commit the
-                            // clock and fire the reaction
-                            tc = tn;
-                            err_t = err_tn;
-                            ++ev;
-                            Ops::jump(c, a, ex, sp, NS, idx);
-                            continue;
-                        }
+                    }
+                    if (!amb && fire && !close) {
+                        // the common step, decided in float32: commit the
+                        // clock and fire the reaction
+                        ah = an;
+                        al = ln;
+                        xsum = xn;
+                        ++ev;
+                        Ops::jump(c, a, ex, sp, NS, idx);
+                        continue;
+                    }
+                    if (tot.h > 0.0f) {
+                        // past the sample: the bound's terms in the time
+                        // passed, which may be far above the time that was left
+                        amb |= !(fire || d < -__fmaf_ru(bd.c_rem * 1.01f, an, mt));
                         if (!amb) {
                             if (fire) {
                                 if (close) idx = Ops::exact_choice(a, ex, c, sp, NS, rl, RS, bu >> 11);
-                                tc = tn;
-                                err_t = err_tn;
+                                ah = an;
+                                al = ln;
+                                xsum = xn;
                             } else {
                                 // the sample records: the Exp1 draw alone was made
                                 xo_prev(g);
                             }
                         }
+                        replay = amb;
                     } else {
-                        // no reaction can fire: no draw is made
+                        // no reaction can fire: no draw is made (a count out of
+                        // range leaves the step undecided)
+                        fire = false;
+                        replay = wild;
                         xo_prev(g);
                         xo_prev(g);
                     }
-                    replay = amb;
                 }
                 if (replay) {
                     if (!exact_traj) atomicAdd(a.work + 3, 1ull);  // speculation undecided
-                    const unsigned long long ev0 = st[8 * NS];
-                    ev = Ops::replay(a, ex, sp, sps, gsv, rl, RS, NS, st[4 * NS], st[5 * NS], nat, ev0, t_start);
+                    const unsigned long long ev0 = st[7 * NS];
+                    const uint64_t si = st[8 * NS];
+                    const uint64_t t0 = si ? (uint64_t)__double_as_longlong(a.sample_t[si - 1]) : st[4 * NS];
+                    ev = Ops::replay(a, ex, sp, sps, gsv, rl, RS, NS, t0,
+                                     (uint64_t)__double_as_longlong(a.sample_t[si]), nat, ev0, t_start);
                     if (ev == ~0ull) {
                         ev = ev0;
                         abort_run = true;
                         break;
                     }
                     g = Xoshiro{gsv[0], gsv[NS], gsv[2 * NS], gsv[3 * NS]};
+                    for (int s = 0; s < S; ++s) sps[s * NS] = sp[s * NS];
                     exact_traj |= !Ops::load(c, a, sp, NS);
                     fire = false;
                 }
@@ -817,26 +848,26 @@ __device__ __forceinline__ void spec_body(const SsaArgs &a) {
                     ++ev;
                     Ops::jump(c, a, ex, sp, NS, idx);
                 } else {
-                    // record sample i at t = T
-                    if (!replay) Ops::store(c, a, sp, NS);
-                    const long long traj = (long long)st[6 * NS];
-                    const uint64_t i = st[9 * NS];
+                    // record sample i at t = T: the counts go to the copy that
+                    // a re-run of the next interval would start from
+                    if (!replay) Ops::save(c, a, sp, sps, NS);
+                    const long long traj = (long long)st[5 * NS];
+                    const uint64_t i = st[8 * NS];
                     int64_t *o = a.out + (size_t)i * a.n_save * a.n_traj + traj;
-                    for (int k = 0; k < a.n_save; ++k) o[(size_t)k * a.n_traj] = sp[ssave[k] * NS];
+                    for (int k = 0; k < a.n_save; ++k) o[(size_t)k * a.n_traj] = sps[ssave[k] * NS];
                     if (a.row_done) {
                         const uint32_t pw = spend[slot];
                         spend[slot] = (pw ? (pw & 0xFFFFu) : (uint32_t)i) | ((uint32_t)(i + 1) << 16);
                     }
                     if ((long long)i + 1 < a.n_samples) {
-                        st[9 * NS] = i + 1;
-                        st[4 * NS] = st[5 * NS];  // next interval starts at T
-                        tc = Tc;
-                        begin = true;
+                        st[8 * NS] = i + 1;
+                        begin_interval((long long)i + 1 < n_cache
+                                           ? sInt[i + 1]
+                                           : bd.interval(a.sample_t[i], a.sample_t[i + 1]));
                     } else {
-                        const uint64_t T = st[5 * NS];
                         if (a.fin_species)
-                            for (int s = 0; s < S; ++s) a.fin_species[traj * S + s] = sp[s * NS];
-                        if (a.fin_t) a.fin_t[traj] = __longlong_as_double((long long)T);
+                            for (int s = 0; s < S; ++s) a.fin_species[traj * S + s] = sps[s * NS];
+                        if (a.fin_t) a.fin_t[traj] = a.sample_t[i];
                         if (a.fin_rng) {
                             a.fin_rng[traj * 4 + 0] = g.s0;
                             a.fin_rng[traj * 4 + 1] = g.s1;
@@ -873,17 +904,20 @@ __device__ __forceinline__ void spec_body(const SsaArgs &a) {
                 st[1 * NS] = g.s1;
                 st[2 * NS] = g.s2;
                 st[3 * NS] = g.s3;
-                st[7 * NS] = ev;
-                stf[0 * NS + slot] = tc.h;
-                stf[1 * NS + slot] = tc.m;
-                stf[2 * NS + slot] = tc.l;
-                stf[3 * NS + slot] = err_t;
-                stf[4 * NS + slot] = Tc.h;
-                stf[5 * NS + slot] = Tc.m;
-                stf[6 * NS + slot] = Tc.l;
+                st[6 * NS] = ev;
+                // the time left, in three floats; the phase's part of the bound
+                // goes to the interval's
+                rem = tf_sub(rem, ah, al);
+                err0 = __fadd_ru(err0, __fmaf_ru(bd.c_rem, ah, __fmaf_ru(kGamma * 1.01f, xsum, bd.clock(T_h))));
+                stf[0 * NS + slot] = fmaxf(__fsub_rn(T_h, rem.h), 0.f);  // clock, for lag_select
+                stf[1 * NS + slot] = rem.h;
+                stf[2 * NS + slot] = rem.m;
+                stf[3 * NS + slot] = rem.l;
+                stf[4 * NS + slot] = err0;
+                stf[5 * NS + slot] = T_h;
             }
             stflag[slot] = (live ? kLive : 0u) | (have ? kHave : 0u) | (nat ? kNat : 0u) |
-                           (exact_traj ? kExactTraj : 0u) | (begin ? kBegin : 0u);
+                           (exact_traj ? kExactTraj : 0u);
             if (abort_run) ctr[1] = 1;
         }
         __syncwarp();
@@ -941,12 +975,13 @@ __device__ __forceinline__ void spec_body(const SsaArgs &a) {
             have = (fl & kHave) != 0;
             nat = (fl & kNat) != 0;
             exact_traj = (fl & kExactTraj) != 0;
-            begin = (fl & kBegin) != 0;
             g = Xoshiro{stw[0 * NS + slot], stw[1 * NS + slot], stw[2 * NS + slot], stw[3 * NS + slot]};
-            ev = stw[7 * NS + slot];
-            tc = TF{stf[0 * NS + slot], stf[1 * NS + slot], stf[2 * NS + slot]};
-            err_t = stf[3 * NS + slot];
-            Tc = TF{stf[4 * NS + slot], stf[5 * NS + slot], stf[6 * NS + slot]};
+            ev = stw[6 * NS + slot];
+            rem = TF{stf[1 * NS + slot], stf[2 * NS + slot], stf[3 * NS + slot]};
+            err0 = stf[4 * NS + slot];
+            T_h = stf[5 * NS + slot];
+            mrg = bd.margin(rem.h, rem.l, T_h, err0);
+            ah = al = xsum = 0.f;
             if (have && !exact_traj) Ops::load(c, a, spa + slot, NS);
         }
         __syncwarp();  // slot flags are rewritten by the next phase

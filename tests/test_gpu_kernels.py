@@ -174,3 +174,21 @@ def test_rate_expressions_on_a_generated_kernel(rb, O, monkeypatch, case, n):
     assert res.stats["mapping"] == 0 and ev.max() > 1
     np.testing.assert_array_equal(res.counts, ref)
     np.testing.assert_array_equal(res.events, ev)
+
+
+# the float-pair clock: no time at all, an interval too short for its parts, thousands of phases in
+# one interval, more intervals than the block keeps in shared memory
+@pytest.mark.parametrize("jit", ["0", "1"])
+@pytest.mark.parametrize("tmax,steps,scale", [(0.0, 3, 1.0), (2.0**-84, 4, 1.0), (2.0**-70, 2, 2.0**59), (4000.0, 1, 1.0),
+                                              (40.0, 700, 1.0)])
+def test_interval_clock(rb, O, monkeypatch, tmax, steps, scale, jit):
+    monkeypatch.setenv("RB_JIT", jit)
+    net, onet = rb.Network(2), O.OracleNet(2)
+    for k, e, d in [(20.0, [0, 0], [1, 0]), (0.5, [1, 0], [-1, 1]), (0.4, [0, 1], [0, -1])]:
+        net.add_reaction(rb.Rate.lma(k * scale, e), d)
+        onet.add_lma(k * scale, e, d)
+    seeds = _seeds(70, 5)
+    res = net.run_ensemble([3, 4], seeds, tmax, steps)
+    ref, ev, _, _ = onet.run_ensemble([3, 4], seeds, tmax, steps)
+    np.testing.assert_array_equal(res.counts, ref)
+    np.testing.assert_array_equal(res.events, ev)
