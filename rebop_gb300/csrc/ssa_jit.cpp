@@ -425,22 +425,25 @@ std::string jit_net_source(const Packed &p, int block) {
         o << "        return replay_interval<kMaxR, kMacro>(a, ex, sp, sps, gsv, rl, RS, NS, t0, T, nat, ev0, "
              "t_start);\n    }\n";
     }
-    // jump: per species, the sum of the deltas of the reaction that fired
-    o << "    __device__ static void jump(Counts &c, const SsaArgs &, const ExactTables &, int64_t *, int, int idx) "
-         "{\n";
-    for (int s = 0; s < S; s++) {
-        std::vector<std::pair<int, int64_t>> terms;
-        for (int r = 0; r < R; r++) {
-            int64_t d = 0;
-            for (int k = 0; k < p.Q; k++)
-                if (p.jmp_sp[(size_t)r * p.Q + k] == s) d += p.jmp_d[(size_t)r * p.Q + k];
-            if (d != 0) terms.push_back({r, d});
+    // jump: the row of the reaction that fired
+    bool moves = false;
+    for (size_t k = 0; k < (size_t)R * p.Q; k++) moves |= p.jmp_d[k] != 0;
+    o << "    static constexpr bool kJumpRows = " << (moves ? "true" : "false") << ";\n";
+    o << "    __device__ static void jump(Counts &c, const SsaArgs &, const ExactTables &, const float4 *jrow, int64_t *, "
+         "int,\n                                int idx) {\n";
+    const int words = (S + 3) / 4;
+    for (int w = 0; w < words && moves; w++) {
+        o << "        const float4 d" << w << " = jrow[idx * " << (words | 1) << " + " << w << "];\n";
+        for (int s = 4 * w; s < std::min(S, 4 * w + 4); s++) {
+            bool used = false;
+            for (int r = 0; r < R; r++) {
+                int64_t d = 0;
+                for (int k = 0; k < p.Q; k++)
+                    if (p.jmp_sp[(size_t)r * p.Q + k] == s) d += p.jmp_d[(size_t)r * p.Q + k];
+                used |= d != 0;
+            }
+            if (used) o << "        c.n[" << s << "] += d" << w << "." << "xyzw"[s & 3] << ";\n";
         }
-        if (terms.empty()) continue;
-        o << "        c.n[" << s << "] +=";
-        for (size_t k = 0; k < terms.size(); k++)
-            o << (k ? " +" : "") << " (idx == " << terms[k].first << " ? " << terms[k].second << ".0f : 0.0f)";
-        o << ";\n";
     }
     o << "    }\n};\n\n}  // namespace rbg\n\n";
     o << "extern \"C\" __global__ void __launch_bounds__(" << block << ", 1)\n"

@@ -505,7 +505,7 @@ __device__ __noinline__ unsigned long long thread_unit(const SsaArgs &it, const 
             tc = tn;
             err_t = err_tn;
             ++ev;
-            Ops::jump(c, it, ex, sp, NS, idx);
+            Ops::jump(c, it, ex, nullptr, sp, NS, idx);
         }
         if (replay) {
             // the interval again, exactly, from its saved start

@@ -192,3 +192,17 @@ def test_interval_clock(rb, O, monkeypatch, tmax, steps, scale, jit):
     ref, ev, _, _ = onet.run_ensemble([3, 4], seeds, tmax, steps)
     np.testing.assert_array_equal(res.counts, ref)
     np.testing.assert_array_equal(res.events, ev)
+
+
+# generated kernels: species at the edges of a row of four jumps, odd and even reaction counts
+@pytest.mark.parametrize("S,R,seed", [(1, 1, 41), (3, 2, 42), (4, 3, 43), (5, 7, 44), (8, 6, 45), (9, 16, 46), (13, 5, 47),
+                                      (16, 15, 48)])
+def test_generated_kernel_species_and_reactions(rb, O, monkeypatch, S, R, seed):
+    monkeypatch.setenv("RB_JIT", "1")
+    net, onet, x0 = _random(rb, O, seed, S, R)
+    seeds = _seeds(500, seed)
+    res = net.run_ensemble(x0, seeds, 2e-2, 7)
+    ref, ev, _, _ = onet.run_ensemble(x0, seeds, 2e-2, 7)
+    assert res.stats["mapping"] == 4
+    np.testing.assert_array_equal(res.counts, ref)
+    np.testing.assert_array_equal(res.events, ev)
