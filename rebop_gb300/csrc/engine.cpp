@@ -110,6 +110,9 @@ DeviceNet::~DeviceNet() {
     if (stream) cudaStreamDestroy(stream);
     if (copy_stream) cudaStreamDestroy(copy_stream);
     if (pin_rows) cudaFreeHost(pin_rows);
+    if (pin_stage) cudaFreeHost(pin_stage);
+    for (cudaStream_t s : stage_stream)
+        if (s) cudaStreamDestroy(s);
 }
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }

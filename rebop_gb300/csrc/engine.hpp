@@ -33,6 +33,11 @@ void zig_tables_host(double *x, double *f);
 // Acceptance thresholds K[256] and wedge differences d[256] of those tables.
 void zig_fast_tables_host(const double *x, const double *f, uint64_t *K, double *d);
 
+// Threads that bring a result into fresh pageable memory, and the bytes each
+// takes at a time (see StagedCopy in capi.cpp).
+constexpr int kStageThreads = 4;
+constexpr size_t kStageChunk = 2u << 20;
+
 // Device copy of one network's packed descriptor, its scratch words and the
 // staging buffers of host-pointer calls.
 struct DeviceNet {
@@ -52,6 +57,8 @@ struct DeviceNet {
     cudaStream_t copy_stream = nullptr; // result rows copied back while the kernel runs
     unsigned int *pin_rows = nullptr;   // page-locked copy of the row counters
     size_t pin_rows_n = 0;
+    unsigned char *pin_stage = nullptr; // page-locked slots of StagedCopy's threads, and their streams
+    cudaStream_t stage_stream[kStageThreads] = {};
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
     cudaStream_t last_stream = nullptr; // stream of the last device-pointer run
     int64_t runs = 0;                   // sampled launches of this network

@@ -206,3 +206,20 @@ def test_generated_kernel_species_and_reactions(rb, O, monkeypatch, S, R, seed):
     assert res.stats["mapping"] == 4
     np.testing.assert_array_equal(res.counts, ref)
     np.testing.assert_array_equal(res.events, ev)
+
+
+# results of 16 MB and more into fresh arrays go through page-locked slots of 2 MB: just above the
+# limit, a ragged last slot, rows of the kernels that count them and of one that does not
+@pytest.mark.parametrize("n,steps,kernel", [(2**19, 1, None), (30_011, 40, None), (70_001, 19, "generic")])
+def test_results_into_fresh_and_used_arrays(rb, monkeypatch, n, steps, kernel):
+    if kernel:
+        monkeypatch.setenv("RB_SSA_KERNEL", kernel)
+    net = rb.Network(2)
+    net.add_reaction(rb.Rate.lma(3.0, [0, 0]), [1, 0])
+    net.add_reaction(rb.Rate.lma(0.5, [1, 0]), [-1, 1])
+    seeds = _seeds(n, 71)
+    fresh = net.run_ensemble([2, 0], seeds, 1.0, steps)
+    used = np.full((steps + 1, 2, n), -1, dtype=np.int64)
+    net.run_ensemble([2, 0], seeds, 1.0, steps, out=used)
+    assert fresh.counts.nbytes >= 1 << 24 and fresh.counts[-1].sum() > 2 * n
+    np.testing.assert_array_equal(fresh.counts, used)
