@@ -1015,29 +1015,38 @@ __global__ void rre_kernel(const float *rates, const float *tq, int Q, int S, in
 // whose propensities have at most two factors each (mass action of order
 // <= 2): reaction r's factors are the slots (species, offset) in the generic
 // loop's order -- species ascending, offsets 0 then 1 -- so a = k * f1 * f2
-// with f = max(x[species] - offset, 0) (an unused slot multiplies by 1) is
-// the generic product, factor for factor; the changes are applied to every
-// species as there.  Same operations in the same order, same results.  A
-// network outside that form takes the generic loops.
+// with f = max(x[species] - offset, 0) is the generic product, factor for
+// factor; the changes are applied to every species as there.  Same operations
+// in the same order, same results.  A network outside that form takes the
+// generic loops.
+//
+// One query per lane and one warp per scheduler at 16 384 queries: the
+// instructions of a right-hand side bound it.  The slot's species is known at
+// run time only, so it is picked by all-ones masks, one three-input logic
+// operation per species, exact for any bits; a compare and a select per
+// species took twice that.  An unused slot has no mask and offset -1: it
+// multiplies by max(0 + 1, 0) = 1.  16 384 queries of 4 species and 5
+// reactions: 134 us with compares, 53 with masks.
 template <int S_>
-__device__ __forceinline__ float rre_pick(const float (&x)[S_], int s) {
-    float v = 1.0f;  // s == S_: the constant factor of an unused slot
+__device__ __forceinline__ float rre_pick(const float (&x)[S_], const uint32_t (&m)[S_]) {
+    uint32_t v = 0;
 #pragma unroll
-    for (int i = 0; i < S_; ++i) v = s == i ? x[i] : v;
-    return v;
+    for (int i = 0; i < S_; ++i) v |= __float_as_uint(x[i]) & m[i];
+    return __uint_as_float(v);
 }
 
 template <int S_, int R_>
-__device__ __forceinline__ void rre_rhs_fixed(const int (&s1)[R_], const float (&o1)[R_], const int (&s2)[R_],
-                                              const float (&o2)[R_], const float (&nn)[R_][S_], const float (&k)[R_],
-                                              const float (&x)[S_], float (&dx)[S_]) {
+__device__ __forceinline__ void rre_rhs_fixed(const uint32_t (&m1)[R_][S_], const float (&o1)[R_],
+                                              const uint32_t (&m2)[R_][S_], const float (&o2)[R_],
+                                              const float (&nn)[R_][S_], const float (&k)[R_], const float (&x)[S_],
+                                              float (&dx)[S_]) {
 #pragma unroll
     for (int s = 0; s < S_; ++s) dx[s] = 0.0f;
 #pragma unroll
     for (int r = 0; r < R_; ++r) {
         float a = k[r];
-        if (s1[r] < S_) a *= fmaxf(rre_pick<S_>(x, s1[r]) - o1[r], 0.0f);
-        if (s2[r] < S_) a *= fmaxf(rre_pick<S_>(x, s2[r]) - o2[r], 0.0f);
+        a *= fmaxf(rre_pick<S_>(x, m1[r]) - o1[r], 0.0f);
+        a *= fmaxf(rre_pick<S_>(x, m2[r]) - o2[r], 0.0f);
 #pragma unroll
         for (int s = 0; s < S_; ++s) dx[s] += nn[r][s] * a;
     }
@@ -1048,25 +1057,25 @@ __global__ void rre_fixed_kernel(const float *rates, const float *tq, int Q, con
                                  const float *x0, int n_steps, const int *out_idx, int n_out, float *out) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= Q) return;
-    int s1[R_], s2[R_];
+    uint32_t m1[R_][S_], m2[R_][S_];
     float o1[R_], o2[R_], nn[R_][S_], k[R_], x[S_], xt[S_], k1[S_], k2[S_], k3[S_], k4[S_];
     bool two = true;  // every reaction of order <= 2
 #pragma unroll
     for (int r = 0; r < R_; ++r) {
         k[r] = rates[(size_t)q * R_ + r];
-        s1[r] = s2[r] = S_;
-        o1[r] = o2[r] = 0.0f;
+        o1[r] = o2[r] = -1.0f;
         int n_f = 0;
 #pragma unroll
         for (int s = 0; s < S_; ++s) {
             nn[r][s] = N[r * S_ + s];
+            m1[r][s] = m2[r][s] = 0;
             const int e = E[r * S_ + s];
             for (int j = 0; j < e; ++j, ++n_f) {
                 if (n_f == 0) {
-                    s1[r] = s;
+                    m1[r][s] = ~0u;
                     o1[r] = (float)j;
                 } else if (n_f == 1) {
-                    s2[r] = s;
+                    m2[r][s] = ~0u;
                     o2[r] = (float)j;
                 }
             }
@@ -1097,16 +1106,16 @@ __global__ void rre_fixed_kernel(const float *rates, const float *tq, int Q, con
     const float h = tq[q] / (float)n_steps;
     const float h2 = 0.5f * h, h6 = h / 6.0f;  // the generic kernel's (0.5f * h) and (h / 6.0f)
     for (int n = 0; n < n_steps; ++n) {
-        rre_rhs_fixed<S_, R_>(s1, o1, s2, o2, nn, k, x, k1);
+        rre_rhs_fixed<S_, R_>(m1, o1, m2, o2, nn, k, x, k1);
 #pragma unroll
         for (int s = 0; s < S_; ++s) xt[s] = x[s] + h2 * k1[s];
-        rre_rhs_fixed<S_, R_>(s1, o1, s2, o2, nn, k, xt, k2);
+        rre_rhs_fixed<S_, R_>(m1, o1, m2, o2, nn, k, xt, k2);
 #pragma unroll
         for (int s = 0; s < S_; ++s) xt[s] = x[s] + h2 * k2[s];
-        rre_rhs_fixed<S_, R_>(s1, o1, s2, o2, nn, k, xt, k3);
+        rre_rhs_fixed<S_, R_>(m1, o1, m2, o2, nn, k, xt, k3);
 #pragma unroll
         for (int s = 0; s < S_; ++s) xt[s] = x[s] + h * k3[s];
-        rre_rhs_fixed<S_, R_>(s1, o1, s2, o2, nn, k, xt, k4);
+        rre_rhs_fixed<S_, R_>(m1, o1, m2, o2, nn, k, xt, k4);
 #pragma unroll
         for (int s = 0; s < S_; ++s)
             x[s] = fmaxf(x[s] + h6 * (k1[s] + 2.0f * k2[s] + 2.0f * k3[s] + k4[s]), 0.0f);
