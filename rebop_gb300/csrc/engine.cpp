@@ -369,7 +369,7 @@ bool launch_sampled(const Network &net, DeviceNet &dn, const RunDev &r, cudaStre
     // Networks with rate expressions run a generated kernel where it covers
     // them (float pairs as for mass action; mapping 0 all the same: the
     // program interpreter is what runs until it is compiled).  10 000
-    // trajectories of a 3-reaction enzyme network with a quotient (1.4e6
+    // trajectories of a 3-reaction enzyme network with a quotient (1.4e7
     // events): 6.6 ms in the interpreter, which the binary64 pipe bounds, and
     // 1.03 ms generated.  Counts beyond 2^23 throughout, where every interval
     // is run again in binary64: 2.04 and 2.56 ms (20 000 trajectories, 6.7e6

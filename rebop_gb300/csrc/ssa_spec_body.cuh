@@ -8,8 +8,9 @@
 // sample time the clock is reset to T exactly (gillespie.rs:328-330).
 //
 // So each step here evaluates propensities and their total in float pairs
-// (hi + lo, about 46 bits), the clock as a float triple, Exp1/total in float
-// pairs and the choice in float32, all on the FP32 and integer pipes,
+// (hi + lo, about 46 bits), the time left to the sample as a float triple and
+// the time passed in the phase beside it, Exp1/total in float pairs and the
+// choice in float32, all on the FP32 and integer pipes,
 // together with a bound on the distance of every quantity from the value
 // rebop's binary64 arithmetic produces.  A decision whose operands lie farther
 // apart than their bounds is the reference's decision:
