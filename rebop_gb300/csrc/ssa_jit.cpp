@@ -295,6 +295,12 @@ static void expr_pairs(const Packed &p, int r, std::ostringstream &o) {
     o << "            const DF acc = " << df(st.back()) << ";\n";
 }
 
+// Networks with more non-zero changes of a species than this add them by rows
+// (spec_jump_row); fewer are selected by the reaction's index.  Rows / selects
+// measured 22.1 / 22.3 ms on the dimer (6 changes), 0.825 / 0.816 ms on one SIR
+// trajectory (3) and 261 / 292 ms on Vilar oscillators (some 40).
+constexpr size_t kJitRowChanges = 8;
+
 std::string jit_net_source(const Packed &p, int block) {
     const int S = p.S, R = p.R;
     std::ostringstream o;
@@ -425,25 +431,33 @@ std::string jit_net_source(const Packed &p, int block) {
         o << "        return replay_interval<kMaxR, kMacro>(a, ex, sp, sps, gsv, rl, RS, NS, t0, T, nat, ev0, "
              "t_start);\n    }\n";
     }
-    // jump: the row of the reaction that fired
-    bool moves = false;
-    for (size_t k = 0; k < (size_t)R * p.Q; k++) moves |= p.jmp_d[k] != 0;
-    o << "    static constexpr bool kJumpRows = " << (moves ? "true" : "false") << ";\n";
+    // jump: the row of the reaction that fired (spec_jump_row), or with few
+    // changes per species the sum of the deltas of the reaction that fired
+    std::vector<std::vector<std::pair<int, int64_t>>> terms((size_t)S);
+    size_t changes = 0;
+    for (int s = 0; s < S; s++)
+        for (int r = 0; r < R; r++) {
+            int64_t d = 0;
+            for (int k = 0; k < p.Q; k++)
+                if (p.jmp_sp[(size_t)r * p.Q + k] == s) d += p.jmp_d[(size_t)r * p.Q + k];
+            if (d != 0) terms[(size_t)s].push_back({r, d});
+            changes += d != 0;
+        }
+    const bool rows = changes > kJitRowChanges;
+    o << "    static constexpr bool kJumpRows = " << (rows ? "true" : "false") << ";\n";
     o << "    __device__ static void jump(Counts &c, const SsaArgs &, const ExactTables &, const float4 *jrow, int64_t *, "
          "int,\n                                int idx) {\n";
     const int words = (S + 3) / 4;
-    for (int w = 0; w < words && moves; w++) {
-        o << "        const float4 d" << w << " = jrow[idx * " << (words | 1) << " + " << w << "];\n";
-        for (int s = 4 * w; s < std::min(S, 4 * w + 4); s++) {
-            bool used = false;
-            for (int r = 0; r < R; r++) {
-                int64_t d = 0;
-                for (int k = 0; k < p.Q; k++)
-                    if (p.jmp_sp[(size_t)r * p.Q + k] == s) d += p.jmp_d[(size_t)r * p.Q + k];
-                used |= d != 0;
-            }
-            if (used) o << "        c.n[" << s << "] += d" << w << "." << "xyzw"[s & 3] << ";\n";
-        }
+    for (int s = 0; s < S; s++) {
+        const auto &v = terms[(size_t)s];
+        if (rows && s % 4 == 0)
+            o << "        const float4 d" << s / 4 << " = jrow[idx * " << (words | 1) << " + " << s / 4 << "];\n";
+        if (v.empty()) continue;
+        o << "        c.n[" << s << "] +=";
+        if (rows) o << " d" << s / 4 << "." << "xyzw"[s & 3];
+        for (size_t k = 0; k < v.size() && !rows; k++)
+            o << (k ? " +" : "") << " (idx == " << v[k].first << " ? " << v[k].second << ".0f : 0.0f)";
+        o << ";\n";
     }
     o << "    }\n};\n\n}  // namespace rbg\n\n";
     o << "extern \"C\" __global__ void __launch_bounds__(" << block << ", 1)\n"

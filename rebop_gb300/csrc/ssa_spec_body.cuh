@@ -304,7 +304,7 @@ __host__ __device__ inline int spec_sample_cache(const SsaArgs &a) {
     return a.n_samples <= kSpecSampleCache ? (int)a.n_samples : 0;
 }
 
-// Generated kernels keep each reaction's changes of the species as a row of
+// Generated kernels of networks with many changes keep each reaction's changes of the species as a row of
 // floats (and a row of zeros for no reaction), an odd number of 16-byte words
 // so that rows spread over the banks.  Adding the row of the reaction that
 // fired takes S/4 loads and S adds; selecting every change by the reaction's
